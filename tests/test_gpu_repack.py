@@ -47,6 +47,21 @@ def test_gptq_marlin_repack(env, n_chunk, bits, act_order, mnk):
     assert np.array_equal(got.cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("bits,K,N", [(4, 16, 64), (8, 16, 64),            # one k-tile
+                                      (4, 12896, 128), (4, 12928, 128),    # last 32-column panel, first of 16
+                                      (8, 5808, 128), (8, 5824, 128),
+                                      (4, 25824, 64), (4, 25856, 64),      # last panel that fits, global gather
+                                      (8, 11616, 64), (8, 11632, 64)])
+def test_gptq_repack_act_order_panel_edges(env, bits, K, N):
+    torch, G, ops = env
+    rng = np.random.default_rng(K + bits)
+    packed = rng.integers(-2**31, 2**31 - 1, size=(K * bits // 32, N), dtype=np.int64).astype(np.int32)
+    perm = rng.permutation(K).astype(np.int32)
+    want = mo.gptq_marlin_repack(packed, perm, K, N, bits)
+    got = ops.gptq_marlin_repack(G.ti32(packed), G.ti32(perm), K, N, bits)
+    assert np.array_equal(got.cpu().numpy(), want)
+
+
 @pytest.mark.parametrize("n_chunk", [64, 256])
 @pytest.mark.parametrize("bits", [4, 8])
 @pytest.mark.parametrize("mnk", MNK_FACTORS)
