@@ -36,6 +36,11 @@ def _units():
         for bits in (4, 8):
             units.append(("gemm_stream_inst.cu", f"gemm_stream_{'bf16' if bf16 else 'f16'}_w{bits}.o",
                           [f"-DINST_BF16={bf16}", f"-DINST_BITS={bits}"]))
+    # tensor-core GEMM: two weight formats per unit (numbers: the Fmt enum of gemm_tc.cuh)
+    for bf16, pairs in ((0, ((0, 1), (2, 3), (4, 5), (7, 8))), (1, ((0, 1), (2, 3), (4, 5), (6, 6)))):
+        for f0, f1 in pairs:
+            units.append(("gemm_tc_inst.cu", f"gemm_tc_{'bf16' if bf16 else 'f16'}_{f0}{f1}.o",
+                          [f"-DINST_BF16={bf16}", f"-DINST_F0={f0}", f"-DINST_F1={f1}"]))
     for extra in ("gemm_tc.cu", "noalloc.cu", "allreduce.cu", "elementwise.cu"):
         units.append((extra, extra.replace(".cu", ".o"), []))
     return units

@@ -76,11 +76,13 @@ template <typename T, int BITS>
 int dispatch_stream(const StreamParams& p, bool has_zp, int gm, int mb, int ntw, int max_ctas,
                     cudaStream_t stream);
 
-bool tc_gemm_supported(int64_t size_m, int64_t size_n, int64_t size_k, int gm);
-int launch_tc_gemm(const void* a, int64_t lda, const uint32_t* b, const void* scales,
-                   const uint32_t* zeros, const void* bias, void* c, int a_dtype, int bits,
-                   int64_t size_m, int64_t size_n, int64_t size_k, int group_blocks,
-                   int channelwise, void* scratch, int64_t scratch_bytes, cudaStream_t stream);
+bool tc_gemm_supported(int64_t size_n, int64_t size_k, int gm);
+int launch_tc_gemm(const void* a, int64_t lda, const uint32_t* b, const void* scales, const uint32_t* zeros,
+                   const void* bias, const void* global_scale, void* c, int a_dtype, int fmt, int64_t size_m,
+                   int64_t size_n, int64_t size_k, int group_blocks, int channelwise, void* scratch,
+                   int64_t scratch_bytes, cudaStream_t stream);
+// weight formats of the tensor-core kernel (gemm_tc.cuh)
+enum { kTcU4B8, kTcU4Z, kTcU8B128, kTcU8Z, kTcF8, kTcNV4, kTcMX4, kTcU4ZF, kTcU8ZF };
 int64_t tc_gemm_scratch_bytes(int64_t size_m, int64_t size_n, int64_t size_k);
 int tc_error_flag(bool reset);
 int ar_error_flag(bool reset);
@@ -306,12 +308,17 @@ static int gemm_impl(const void* a, int64_t lda, const uint32_t* b_q_weight, con
     B200Q_REQUIRE(global_scale == nullptr && fp4_scales == 0, B200Q_EINVAL,
                   "global_scale can only be used for nvfp4 format.");
   }
-  // these run the reference-order kernel at every row count
+  // these run the tensor-core kernel at every row count (the reference-order one where it can not)
   const bool general_only = zp_float || w_fp8 || w_fp4;
-  // ---- prefill regime: tensor-core kernel ----------------------------------------------
-  if (!general_only && tc_path_enabled() && group_blocks >= 2 && tc_gemm_supported(size_m, size_n, size_k, gm)) {
-    int rc = launch_tc_gemm(a_used, lda_used, b_q_weight, b_scales, b_zeros, b_bias, c, a_dtype,
-                            bits, size_m, size_n, size_k, group_blocks, gm == kChannel, scratch,
+  // ---- tensor-core kernel: many rows, and the float formats at every row count ------------
+  if ((size_m >= 33 || general_only) && tc_path_enabled() && tc_gemm_supported(size_n, size_k, gm)) {
+    const int fmt = zp_float ? (bits == 4 ? kTcU4ZF : kTcU8ZF)
+                    : w_fp8 ? kTcF8
+                    : w_fp4 ? (fp4_scales == 1 ? kTcNV4 : kTcMX4)
+                    : bits == 4 ? (has_zp ? kTcU4Z : kTcU4B8)
+                                : (has_zp ? kTcU8Z : kTcU8B128);
+    int rc = launch_tc_gemm(a_used, lda_used, b_q_weight, b_scales, b_zeros, b_bias, global_scale, c, a_dtype, fmt,
+                            size_m, size_n, size_k, group_blocks, gm == kChannel, scratch,
                             (int64_t)((scratch_bytes - a_tmp_bytes) / 256 * 256), stream);
     if (rc != B200Q_OK || !link) return rc;
     return launch_all_reduce(*link, c, c, size_m * size_n, a_dtype, stream);

@@ -1,0 +1,882 @@
+// Mixed-precision GEMM on the 5th-generation tensor cores: C[M,N] = A[M,K] * dequant(B), tcgen05.mma
+// with TMEM accumulators.  The kernel computes C^T = B^T A^T: the weights are the 128-row (CTA pair:
+// 256-row) operand, the rows of A ("tokens") are the MMA's N dimension, so that a tile fits any token
+// count in steps of 16 (32), a lane of the accumulator is one output column (its channel scale and bias
+// are one register), and every CTA converts each weight of its tile once.
+//
+// One persistent CTA per SM, or (more than 128 tokens) one CTA pair per two SMs: with cta_group::2 a
+// 256 x 256 tile is computed by two CTAs that each convert 128 of the 256 weight columns and stage half
+// of the tokens; the tensor cores read the other half from the peer.  A single-CTA 256 x 256 tile needs
+// 96 B per clock of shared memory for the MMA operands alone, and 176 of the 128 there are together with
+// the conversion; the pair needs 64 for the operands and leaves room for two accumulators.
+//
+// Roles (23 warps), hand-offs through mbarriers; a step is 64 deep in k, two steps make a round:
+//   producer warp     packed weights, scales and zero-points of a round into a ring of kWD slots, one
+//                     2-D copy each (deep: this is what comes from HBM; with a copy per step and per scale
+//                     row the issuing thread was the bottleneck at 925 cycles a step)
+//   token warp        token rows of a round (TMA, 128B swizzle) into kRing slots
+//   16 dequant warps  a warp converts one 16 x 64 Marlin tile of the round: packed words -> exact 16-bit
+//                     codes -> scaled -> K-major swizzled operand in shared memory; the words of the next
+//                     round are fetched before the current ones are converted
+//   MMA warp          one elected lane issues eight 128 (256) x tn x 16 MMAs per round, commits the slot back
+//                     (a satisfied barrier wait costs about 200 cycles beside twenty busy warps, so token rows
+//                     and converted weights share one barrier, and it is waited for once per round)
+//   4 epilogue warps  TMEM -> registers -> scale, bias, rounding -> C, while the next tile is computed
+//
+// Work is cut into (tile, k-range) segments.  Whole waves of tiles run one tile per CTA (pair); what
+// would be a ragged last wave is cut into equal k-ranges instead ("shared" tiles): each contributor
+// leaves an fp32 partial tile in the scratch, the last to arrive (atomic counter, no waiting) adds all
+// of them in k order, so results are bitwise reproducible.  With fewer tiles than SMs every tile is
+// shared by several workers and nothing is left to hide that addition behind (four warps of one CTA in
+// three: 80 of 107 us at M = 256, 4096 x 4096): tc_reduce_kernel does it on the whole GPU instead.
+//
+// Every wait is bounded: after kSpinLimit polls a role records a code in *p.error, stops, and the
+// kernel drains (TMEM is freed), so a broken hand-off can not hang the GPU.
+#pragma once
+
+#include <cuda.h>
+
+#include <type_traits>
+
+#include "common.cuh"
+#include "gemm_params.cuh"
+
+namespace b200q {
+namespace tc {
+
+// weight formats
+enum Fmt : int {
+  kU4B8 = 0,   // uint4, built-in offset 8
+  kU4Z = 1,    // uint4 with packed zero-points
+  kU8B128 = 2,
+  kU8Z = 3,
+  kF8 = 4,     // float8_e4m3fn
+  kNV4 = 5,    // float4_e2m1f, fp8 (S0E5M3) scales per 16, global scale
+  kMX4 = 6,    // float4_e2m1f, e8m0 scales per 32
+  kU4ZF = 7,   // uint4 with 16-bit float zero-points (HQQ)
+  kU8ZF = 8,
+};
+template <int F>
+struct FmtInfo {
+  static constexpr int kBits = (F == kU8B128 || F == kU8Z || F == kF8 || F == kU8ZF) ? 8 : 4;
+  static constexpr bool kFp4 = F == kNV4 || F == kMX4;
+  static constexpr bool kZp = F == kU4Z || F == kU8Z;      // packed integer zero-points
+  static constexpr bool kZpF = F == kU4ZF || F == kU8ZF;   // float zero-points
+};
+
+constexpr int kBK = 64;            // k per step: one 128-byte swizzle row of 16-bit values
+constexpr int kRoundTiles = 8;     // k-tiles (16 rows) per round of two steps
+constexpr int kBN = 128;           // weight columns per CTA
+constexpr int kDequantWarps = 16;  // eight for each step of a round
+constexpr int kEpiWarp0 = kDequantWarps;  // 4 warps: TMEM lane quadrant = warp % 4
+constexpr int kProducerWarp = kEpiWarp0 + 4;
+constexpr int kTokenWarp = kProducerWarp + 1;
+constexpr int kMmaWarp = kTokenWarp + 1;
+constexpr int kThreads = 32 * (kMmaWarp + 1);
+constexpr uint32_t kSpinLimit = 1u << 24;
+
+struct TcParams {
+  int* error;                // device word: 0 = ok; else (role << 8) | barrier id of the first wait that timed out
+  const void* scales;        // [G, N] permuted (fp4: bytes, regrouped)
+  const void* bias;          // [N] permuted or null
+  const void* global_scale;  // NVFP4
+  void* c;                   // [M, N]
+  int m, n, k;
+  int group_blocks;          // k-tiles (16 rows) per scale group; K/16 when there is one group
+  int groups;                // scale groups of one expert
+  int group_rows;            // scale rows copied per round
+  int channelwise;           // one scale per column: applied to the fp32 sums
+  int tn;                    // tokens per tile (multiple of 16, of 32 for a CTA pair)
+  int box;                   // token rows a CTA stages per step
+  int tok_tiles;             // token tiles
+  int workers;               // CTAs, or CTA pairs, of the grid
+  int sk_tiles;              // the first tiles are shared out by k-range among all workers
+  int reduce_later;          // partial sums are added up by tc_reduce_kernel
+  float chan_factor;         // of the channel-wise scales (fp8: takes the exponent re-bias out)
+  float* partials;           // [worker][2][CG][tn][128] fp32
+  int32_t* counters;         // [worker][CG], zero between kernels; one byte per lane quadrant
+  // mixture of experts: tiles come from a list in device memory {expert, first row, rows}; the rows of A
+  // are in sorted order, output row = ids[row] (>= out_rows: padding), scaled by row_weights[id]
+  const int4* tile_list;
+  const int32_t* tile_count;
+  const int32_t* ids;
+  const float* row_weights;
+  int out_rows;
+  long long s_stride, bias_stride;  // per expert, elements
+};
+
+// A: rows of A; B: packed weights; S: scales; Z: zero-points (the last two only where the format has them)
+struct TcMaps {
+  CUtensorMap a, b, s, z;
+};
+
+// ---- PTX wrappers ------------------------------------------------------------------
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count));
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+// arrive on a barrier given by its cluster address (mapa).  (With .release.cluster the arrive took 1350
+// cycles; the operand data is ordered by the proxy fence in front of it.)
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes)
+               : "memory");
+}
+// Bounded wait on a phase parity.  Returns false (and records `what`) on time-out.  CLUSTER: the
+// barrier is also arrived on by the peer CTA (acquire at cluster scope).  SLEEP_NS: back off between
+// polls (roles with long waits leave the issue slots to the others).
+template <bool CLUSTER, int SLEEP_NS = 0>
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int what, volatile int* cta_abort,
+                                          int* error) {
+  for (uint32_t spin = 0; spin < kSpinLimit; ++spin) {
+    uint32_t done;
+    if (CLUSTER)
+      asm volatile(
+          "{\n\t.reg .pred p;\n\t"
+          "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+          "selp.u32 %0, 1, 0, p;\n\t}\n"
+          : "=r"(done)
+          : "r"(bar), "r"(parity)
+          : "memory");
+    else
+      asm volatile(
+          "{\n\t.reg .pred p;\n\t"
+          "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+          "selp.u32 %0, 1, 0, p;\n\t}\n"
+          : "=r"(done)
+          : "r"(bar), "r"(parity)
+          : "memory");
+    if (done) return true;
+    if (SLEEP_NS > 0) __nanosleep(SLEEP_NS);
+    // now and then: stop early if another role of this CTA has already given up
+    if ((spin & 1023u) == 1023u && *cta_abort != 0) return false;
+  }
+  *cta_abort = 1;
+  atomicCAS(error, 0, what);
+  return false;
+}
+__device__ __forceinline__ void fence_proxy_async_smem() {
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+}
+// CG == 2: the barrier may be the peer's (its cluster address is given)
+template <int CG>
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  if (CG == 2)
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
+        "[%0], [%1, {%2, %3}], [%4];\n" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar)
+        : "memory");
+  else
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+        "[%0], [%1, {%2, %3}], [%4];\n" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar)
+        : "memory");
+}
+template <int CG>
+__device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t cols) {
+  if (CG == 2) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_dst), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
+  } else {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_dst), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
+}
+template <int CG>
+__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
+  if (CG == 2)
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(cols) : "memory");
+  else
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(cols) : "memory");
+}
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
+// D[tmem] (+)= A[smem] * B[smem], 16-bit inputs, fp32 accumulate
+template <int CG>
+__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                         uint32_t accumulate) {
+  if (CG == 2)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// arrive on an mbarrier (CG == 2: the same one of both CTAs) when all MMAs issued so far have completed
+template <int CG>
+__device__ __forceinline__ void umma_commit(uint32_t bar) {
+  if (CG == 2)
+    asm volatile(
+        "{\n\t.reg .b16 mask;\n\tmov.u16 mask, 3;\n\t"
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], mask;\n\t}\n" ::
+            "r"(bar)
+        : "memory");
+  else
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
+}
+// 32 lanes x 32 consecutive fp32 columns of TMEM -> 32 registers per thread
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,"
+      "%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
+        "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
+        "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
+
+// true in one lane of a converged warp; unlike a lane test it keeps the operands of the tensor-core
+// instructions in uniform registers
+__device__ __forceinline__ bool elect_one() {
+  uint32_t pred;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(pred));
+  return pred != 0;
+}
+
+template <int OFF>
+__device__ __forceinline__ void sts32_off(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared.u32 [%0+%2], %1;\n" ::"r"(addr), "r"(v), "n"(OFF) : "memory");
+}
+
+// Shared-memory matrix descriptor: K-major tile, 128-byte swizzle, rows 128 B apart, 8-row atoms 1024 B
+// apart (version 1 = sm_100 format).
+__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
+  return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+}
+// instruction descriptor: fp32 accumulate, A and B K-major
+template <typename T>
+__device__ __forceinline__ uint32_t make_idesc(int m, int n) {
+  const uint32_t f = std::is_same<T, half>::value ? 0u : 1u;
+  return (1u << 4) | (f << 7) | (f << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+
+// Shared-memory plan.  TOK: token rows a CTA can stage per step (64 or 128).
+template <int F, int TOK>
+struct TcCfg {
+  using I = FmtInfo<F>;
+  static constexpr int kTileBytes = 16 * 64 * I::kBits / 8;    // one packed 16 x 64 weight tile
+  static constexpr int kWBytes = kRoundTiles * 2 * kTileBytes;  // 8 k-tiles x 2 column tiles
+  // rows of scales (fp4: of byte pairs) a round can touch
+  static constexpr int kSRow = 2 * kBN;
+  static constexpr int kSBytes = (F == kNV4 ? 4 : F == kMX4 ? 2 : kRoundTiles) * kSRow;
+  static constexpr int kZRow = I::kZpF ? 2 * kBN : I::kZp ? kBN * I::kBits / 8 : 0;
+  static constexpr int kWSlot = kWBytes + kSBytes + kRoundTiles * kZRow;  // a multiple of 128
+  // a slot: token rows of the two steps, converted weights of the two steps
+  static constexpr int kTokBytes = TOK * 128;
+  static constexpr int kABytes = kBN * 128;
+  static constexpr int kSlot = 2 * (kTokBytes + kABytes);
+  static constexpr int kRing = TOK == 64 ? 3 : 2;
+  static constexpr int kBarBytes = 1024;
+  static constexpr int kFit = (226 * 1024 - kBarBytes - 1024 - kRing * kSlot) / kWSlot;
+  static constexpr int kWD = kFit >= 8 ? 8 : kFit;
+  static constexpr int kSmemBytes = kRing * kSlot + kWD * kWSlot + kBarBytes + 1024;  // + alignment slack
+};
+
+// Position in a ring of N slots and the parity of the current pass over it.
+template <int N>
+struct Ring {
+  int i = 0;
+  uint32_t ph = 0;
+  __device__ __forceinline__ void next() {
+    if (++i == N) { i = 0; ph ^= 1; }
+  }
+};
+
+// ---- schedule ------------------------------------------------------------------------
+struct Segment {
+  int n_tile;        // tile along N, in units of CG * 128 columns
+  int tok0, rows;    // first token row, valid rows
+  int expert;
+  int r0, r1;        // rounds
+  bool shared;       // other workers hold the rest of the tile's k-range
+  int first, contributors, slot;  // shared: first contributing worker, how many, this segment's slot
+};
+
+// Which of `workers` equal shares of `units` holds `unit`.
+__device__ __forceinline__ int share_of(long long unit, int workers, long long units) {
+  return (int)(((unit + 1) * workers - 1) / units);
+}
+
+// All roles of a worker walk the same sequence of segments.
+struct Schedule {
+  const TcParams& p;
+  int worker, rounds;      // rounds per tile
+  long long u, u1, units;  // shared region: range of (tile, round) units
+  int tile, tiles;         // whole tiles
+  __device__ Schedule(const TcParams& p_, int worker_, int cols_per_tile)
+      : p(p_), worker(worker_), rounds((p_.k / kBK + 1) / 2) {
+    const int n_tiles = (p.n + cols_per_tile - 1) / cols_per_tile;
+    tiles = n_tiles * (p.tile_list ? *p.tile_count : p.tok_tiles);
+    units = (long long)p.sk_tiles * rounds;
+    u = units * worker / p.workers;
+    u1 = units * (worker + 1) / p.workers;
+    tile = p.sk_tiles + worker;
+  }
+  __device__ __forceinline__ void place(Segment& s, int t) const {
+    if (p.tile_list) {
+      const int count = *p.tile_count;
+      const int4 e = __ldg(p.tile_list + t % count);
+      s.n_tile = t / count;
+      s.expert = e.x; s.tok0 = e.y; s.rows = e.z;
+    } else {
+      s.n_tile = t / p.tok_tiles;
+      s.expert = 0;
+      s.tok0 = (t - s.n_tile * p.tok_tiles) * p.tn;
+      s.rows = min(p.tn, p.m - s.tok0);
+    }
+  }
+  __device__ __forceinline__ int owner(long long unit) const { return share_of(unit, p.workers, units); }
+  __device__ __forceinline__ bool next(Segment& s) {
+    if (u < u1) {
+      const int t = (int)(u / rounds);
+      s.r0 = (int)(u - (long long)t * rounds);
+      s.r1 = (int)min((long long)rounds, s.r0 + (u1 - u));
+      u += s.r1 - s.r0;
+      place(s, t);
+      s.shared = s.r0 > 0 || s.r1 < rounds;
+      if (s.shared) {
+        s.first = owner((long long)t * rounds);
+        s.contributors = owner((long long)t * rounds + rounds - 1) - s.first + 1;
+        s.slot = 2 * worker + (s.r0 > 0 ? 0 : 1);
+      }
+      return true;
+    }
+    if (tile < tiles) {
+      s.r0 = 0;
+      s.r1 = rounds;
+      s.shared = false;
+      place(s, tile);
+      tile += p.workers;
+      return true;
+    }
+    return false;
+  }
+  // tokens of the MMA for this segment
+  template <int CG>
+  __device__ __forceinline__ int mma_n(const Segment& s) const {
+    if (!p.tile_list) return p.tn;
+    constexpr int g = 16 * CG;
+    return (s.rows + g - 1) / g * g;
+  }
+};
+
+// ---- conversion ------------------------------------------------------------------------
+// Four 16-bit pairs of sub-tile `sub`: f[0], f[1] = column c8, k lo / hi; f[2], f[3] = column c8 + 8.
+template <typename T, int F>
+__device__ __forceinline__ void codes_to_16bit(const uint32_t* w, int sub, uint32_t (&f)[4]) {
+  using I = FmtInfo<F>;
+  constexpr bool kBiased = F == kU4B8 || F == kU8B128;
+  if constexpr (I::kFp4) {
+    // sign, two exponent bits, one mantissa bit into the fields of the 16-bit format; nibble i of the
+    // word sits where the uint4 codes do
+    constexpr int kShift = std::is_same<T, half>::value ? 3 : 6;
+    const uint32_t q = w[sub];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t x = q << (4 * (3 - i));
+      f[i] = (x & 0x80008000u) | ((x & 0x70007000u) >> kShift);
+    }
+    if constexpr (F == kMX4) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) f[i] = Pair<T>::mul(f[i], 0x7e807e80u);  // exact re-bias, 2^126
+    }
+  } else if constexpr (I::kBits == 4) {
+    dequant4<T, kBiased>(w[sub], f);
+  } else {
+    uint32_t t0[2], t1[2];
+    if constexpr (F == kF8) {
+      dequant_fp8<T>(w[2 * sub], t0);
+      dequant_fp8<T>(w[2 * sub + 1], t1);
+    } else {
+      dequant8<T, kBiased>(w[2 * sub], t0);
+      dequant8<T, kBiased>(w[2 * sub + 1], t1);
+    }
+    f[0] = t0[0]; f[1] = t0[1]; f[2] = t1[0]; f[3] = t1[1];
+  }
+}
+
+// fp4: one of a lane's scale bytes as a 16-bit pair
+template <typename T, int F>
+__device__ __forceinline__ uint32_t fp4_scale(uint32_t word, int byte) {
+  const uint32_t b = __byte_perm(word, 0, 0x4040 | byte | (byte << 8));  // the byte in both halves
+  if constexpr (F == kMX4 || std::is_same<T, half>::value) {
+    return b << 7;  // e8m0 -> bf16 exponent; S0E5M3 -> fp16 bits 14..7
+  } else {
+    const uint32_t t = b << 4;  // -> bf16: top exponent bit, then the seven lower bits
+    return (t & 0x07f007f0u) | ((t & 0x08000800u) << 3);
+  }
+}
+
+template <typename T, int F, int CG, int TOK>
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
+  using Cfg = TcCfg<F, TOK>;
+  using I = FmtInfo<F>;
+  constexpr int RING = Cfg::kRing, WD = Cfg::kWD, BITS = I::kBits;
+  constexpr bool kPair = CG == 2;
+  extern __shared__ unsigned char smem_raw[];
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t w_base = smem_base + RING * Cfg::kSlot;
+  const uint32_t bars = w_base + WD * Cfg::kWSlot;
+  auto tok_slot = [&](int i) { return smem_base + i * Cfg::kSlot; };
+  auto a_slot = [&](int i) { return smem_base + i * Cfg::kSlot + 2 * Cfg::kTokBytes; };
+  // barriers (8 bytes each).  full (token rows landed and weights converted) and tmem_empty of the
+  // leader CTA serve the pair.
+  auto full = [&](int i) { return bars + 8 * i; };
+  auto empty = [&](int i) { return bars + 8 * (RING + i); };
+  auto full_w = [&](int w) { return bars + 8 * (2 * RING + w); };
+  auto empty_w = [&](int w) { return bars + 8 * (2 * RING + WD + w); };
+  const uint32_t bars2 = bars + 8 * (2 * RING + 2 * WD);
+  auto tmem_full = [&](int b) { return bars2 + 8 * b; };
+  auto tmem_empty = [&](int b) { return bars2 + 16 + 8 * b; };
+  const uint32_t tmem_slot = bars2 + 32;
+
+  // the next kernel in the stream may be scheduled while this one runs (it waits for completion itself)
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  __shared__ int s_abort;
+  volatile int* cta_abort = &s_abort;
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const uint32_t rank = kPair ? (blockIdx.x & 1) : 0;
+  const int worker = kPair ? blockIdx.x >> 1 : blockIdx.x;
+  const int NT = p.n / 64;
+  const int gb = p.group_blocks;
+  const int steps = p.k / kBK;
+  constexpr uint32_t kTmemCols = 2 * CG * 128;
+
+  if (threadIdx.x == 0) {
+    s_abort = 0;
+    for (int i = 0; i < RING; ++i) {
+      mbar_init(full(i), 1 + kDequantWarps * CG);
+      mbar_init(empty(i), 1);
+    }
+    for (int w = 0; w < WD; ++w) {
+      mbar_init(full_w(w), 1);
+      mbar_init(empty_w(w), kDequantWarps);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(tmem_full(b), 1);
+      mbar_init(tmem_empty(b), 4 * CG);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  if (warp == kMmaWarp) tmem_alloc<CG>(tmem_slot, kTmemCols);
+  tc_fence_before();
+  __syncthreads();
+  if (kPair) {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  }
+  tc_fence_after();
+  uint32_t tmem_base;
+  asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(tmem_base) : "r"(tmem_slot));
+  // the tile list of a mixture-of-experts call is written by the kernel in front
+  if (p.tile_list) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  Schedule sched(p, worker, CG * kBN);
+  Segment sg;
+
+  if (warp == kProducerWarp) {
+    // ================= producer =========================================================
+    // Packed weights do not depend on the kernel in front: they run ahead from the start.
+    Ring<WD> wr;
+    bool ok = true;
+    const int kt_all = p.k / 16;
+    const bool scales = I::kFp4 || !p.channelwise;
+    const uint32_t bytes = Cfg::kWBytes + (scales ? (I::kFp4 ? Cfg::kSBytes : p.group_rows * Cfg::kSRow) : 0) +
+                           p.group_rows * Cfg::kZRow;
+    while (ok && sched.next(sg)) {
+      const int nt0 = (sg.n_tile * CG + (int)rank) * 2;
+      for (int r = sg.r0; r < sg.r1; ++r) {
+        if (!(ok = mbar_wait<false>(empty_w(wr.i), wr.ph ^ 1, (1 << 8) | 3, cta_abort, p.error))) break;
+        const uint32_t dst = w_base + wr.i * Cfg::kWSlot, bar = full_w(wr.i);
+        // first row of scales; everything past the end of a matrix is zero-filled and counted
+        const int g0 = sg.expert * p.groups + (r * kRoundTiles) / gb;
+        if (elect_one()) {
+          mbar_expect_tx(bar, bytes);
+          tma_load_2d<1>(dst, &maps.b, nt0 * (Cfg::kTileBytes / 8), sg.expert * kt_all + r * kRoundTiles, bar);
+          if (I::kFp4)
+            tma_load_2d<1>(dst + Cfg::kWBytes, &maps.s, nt0 * 16, r * (Cfg::kSBytes / Cfg::kSRow), bar);
+          else if (scales)
+            tma_load_2d<1>(dst + Cfg::kWBytes, &maps.s, nt0 * 64, g0, bar);
+          if (I::kZp || I::kZpF)
+            tma_load_2d<1>(dst + Cfg::kWBytes + Cfg::kSBytes, &maps.z, I::kZp ? nt0 * 2 * BITS : nt0 * 64, g0, bar);
+        }
+        __syncwarp();
+        wr.next();
+      }
+    }
+  } else if (warp == kTokenWarp) {
+    // ================= token rows =======================================================
+    Ring<RING> ring;
+    bool ok = true;
+    const uint32_t ft0 = kPair ? mapa(full(0), 0) : full(0);  // the leader's
+    // the rows of A come from the kernel in front (programmatic dependent launch)
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    while (ok && sched.next(sg)) {
+      const int row = sg.tok0 + (kPair ? (int)rank * (sched.template mma_n<CG>(sg) / 2) : 0);
+      for (int r = sg.r0; r < sg.r1; ++r) {
+        if (!(ok = mbar_wait<kPair>(empty(ring.i), ring.ph ^ 1, (1 << 8) | 4, cta_abort, p.error))) break;
+        const bool two = 2 * r + 1 < steps;  // a K of an odd number of steps ends with a round of one
+        if (elect_one()) {
+          if (rank == 0) mbar_expect_tx(full(ring.i), CG * p.box * (two ? 256 : 128));
+          tma_load_2d<CG>(tok_slot(ring.i), &maps.a, 2 * r * kBK, row, ft0 + 8 * ring.i);
+          if (two) tma_load_2d<CG>(tok_slot(ring.i) + Cfg::kTokBytes, &maps.a, (2 * r + 1) * kBK, row, ft0 + 8 * ring.i);
+        }
+        __syncwarp();
+        ring.next();
+      }
+    }
+  } else if (warp == kMmaWarp) {
+    // ================= MMA issuer (leader CTA) ==========================================
+    // the whole warp walks the loop, one elected lane issues
+    if (rank == 0) {
+      Ring<RING> ring;
+      int seg_i = 0;
+      bool ok = true;
+      while (ok && sched.next(sg)) {
+        const uint32_t idesc = make_idesc<T>(CG * 128, sched.template mma_n<CG>(sg));
+        const int buf = seg_i & 1;
+        if (!(ok = mbar_wait<kPair>(tmem_empty(buf), ((seg_i >> 1) & 1) ^ 1, (2 << 8) | 5, cta_abort, p.error))) break;
+        tc_fence_after();
+        const uint32_t d = tmem_base + buf * (CG * 128);
+        for (int r = sg.r0; r < sg.r1; ++r) {
+          if (!(ok = mbar_wait<kPair>(full(ring.i), ring.ph, (2 << 8) | 0, cta_abort, p.error))) break;
+          tc_fence_after();
+          const uint64_t da = smem_desc_sw128(a_slot(ring.i)), db = smem_desc_sw128(tok_slot(ring.i));
+          if (elect_one()) {
+#pragma unroll
+            for (int k16 = 0; k16 < 4; ++k16) umma_f16<CG>(d, da + 2 * k16, db + 2 * k16, idesc, r > sg.r0 || k16 > 0);
+            if (2 * r + 1 < steps) {
+#pragma unroll
+              for (int k16 = 0; k16 < 4; ++k16)
+                umma_f16<CG>(d, da + Cfg::kABytes / 16 + 2 * k16, db + Cfg::kTokBytes / 16 + 2 * k16, idesc, 1);
+            }
+            umma_commit<CG>(empty(ring.i));  // slot reusable once these MMAs have read it
+            if (r + 1 == sg.r1) umma_commit<CG>(tmem_full(buf));
+          }
+          __syncwarp();
+          ring.next();
+        }
+        ++seg_i;
+      }
+    }
+  } else if (warp < kDequantWarps) {
+    // ================= dequant warps ====================================================
+    const int c8 = lane >> 2, q = lane & 3;
+    const int step = warp >> 3;           // step of the round
+    const int kt = warp & 3, nt = (warp >> 2) & 1;
+    const int rkt = 4 * step + kt;        // k-tile within the round
+    // byte offsets of this lane's two k-positions (k = 16 kt + 2q, + 8) inside a 128 B row
+    const uint32_t a_rel = 2 * Cfg::kTokBytes + step * Cfg::kABytes;
+    const uint32_t b_lo_rel = a_rel + (nt * 64 + c8) * 128 + (((2 * kt) ^ c8) << 4) + 4 * q;
+    const uint32_t b_hi_rel = a_rel + (nt * 64 + c8) * 128 + (((2 * kt + 1) ^ c8) << 4) + 4 * q;
+    const uint32_t w_rel = rkt * (2 * Cfg::kTileBytes) + nt * Cfg::kTileBytes + lane * (BITS * 4);
+    const uint32_t fa0 = kPair ? mapa(full(0), 0) : full(0);
+    // scale row of this k-tile within the round's copy, where it is the same in every round
+    const bool fixed_row = (gb & 7) == 0 || (8 % gb) == 0;
+    const int row0 = (gb & 7) == 0 ? 0 : rkt / gb;
+    Ring<WD> wr;
+    Ring<RING> ring;
+    bool ok = true;
+    // packed words of the lane, [sub] (4-bit) or [2 sub + block] (8-bit), scales and zero-points: the next
+    // round's (n_) and the current one's
+    constexpr int NW = BITS == 4 ? 4 : 8;
+    uint32_t n_w[NW], n_sc[4], n_zr[4], w[NW], sc[4], zr[4];
+    auto fetch = [&](int r) {
+      const uint32_t wslot = w_base + wr.i * Cfg::kWSlot;
+#pragma unroll
+      for (int v = 0; v < BITS / 4; ++v) {
+        const uint4 w4 = lds128(wslot + w_rel + v * 16);
+        n_w[4 * v] = w4.x; n_w[4 * v + 1] = w4.y; n_w[4 * v + 2] = w4.z; n_w[4 * v + 3] = w4.w;
+      }
+      if constexpr (I::kFp4) {
+        // 16 bytes per (tile, c8) of a pair of groups; this k-tile's group is half of them
+        const uint32_t pair = F == kNV4 ? rkt >> 1 : rkt >> 2, half = F == kNV4 ? rkt & 1 : (rkt >> 1) & 1;
+        const uint32_t src = wslot + Cfg::kWBytes + pair * 256 + nt * 128 + c8 * 16 + half * 8;
+        n_sc[0] = lds32(src);
+        n_sc[1] = lds32(src + 4);
+      } else {
+        const int row = fixed_row ? row0 : (r * kRoundTiles + rkt) / gb - (r * kRoundTiles) / gb;
+        if (!p.channelwise) {
+          const uint4 s4 = lds128(wslot + Cfg::kWBytes + row * Cfg::kSRow + nt * 128 + c8 * 16);
+          n_sc[0] = s4.x; n_sc[1] = s4.y; n_sc[2] = s4.z; n_sc[3] = s4.w;
+        }
+        if constexpr (I::kZp) {
+          const uint32_t zsrc = wslot + Cfg::kWBytes + Cfg::kSBytes + row * Cfg::kZRow + nt * (8 * BITS) + c8 * BITS;
+          n_zr[0] = lds32(zsrc);
+          if (BITS == 8) n_zr[1] = lds32(zsrc + 4);
+        }
+        if constexpr (I::kZpF) {
+          const uint4 z4 = lds128(wslot + Cfg::kWBytes + Cfg::kSBytes + row * Cfg::kZRow + nt * 128 + c8 * 16);
+          n_zr[0] = z4.x; n_zr[1] = z4.y; n_zr[2] = z4.z; n_zr[3] = z4.w;
+        }
+      }
+    };
+    bool more = sched.next(sg);
+    int nr = sg.r0;  // the next round to fetch
+    if (more) {
+      if ((ok = mbar_wait<false>(full_w(wr.i), wr.ph, (3 << 8) | 1, cta_abort, p.error))) fetch(nr);
+    }
+    while (ok && more) {
+      const bool live = (sg.n_tile * CG + (int)rank) * 2 + nt < NT && 2 * nr + step < steps;
+#pragma unroll
+      for (int i = 0; i < NW; ++i) w[i] = n_w[i];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) { sc[i] = n_sc[i]; zr[i] = n_zr[i]; }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(empty_w(wr.i));
+      wr.next();
+      if (++nr == sg.r1) {
+        more = sched.next(sg);
+        nr = sg.r0;
+      }
+      if (more) {
+        if (!(ok = mbar_wait<false>(full_w(wr.i), wr.ph, (3 << 8) | 1, cta_abort, p.error))) break;
+        fetch(nr);
+      }
+      if (!(ok = mbar_wait<kPair>(empty(ring.i), ring.ph ^ 1, (3 << 8) | 4, cta_abort, p.error))) break;
+      {
+        if (live) {
+          const uint32_t b_lo = smem_base + ring.i * Cfg::kSlot + b_lo_rel, b_hi = smem_base + ring.i * Cfg::kSlot + b_hi_rel;
+          auto convert = [&](auto sub_c, auto scaled_c) {
+            constexpr int sub = decltype(sub_c)::value;
+            uint32_t f[4];
+            codes_to_16bit<T, F>(w, sub, f);
+            if constexpr (I::kZp) {
+              // zero-points of columns c8 + 16 sub (low half) and + 8 (high half), exact integers in T
+              uint32_t zpair;
+              if constexpr (BITS == 4) {
+                uint32_t z4[4];
+                dequant4<T, false>(zr[0] >> (4 * sub), z4);  // nibbles sub and sub + 4
+                zpair = z4[0];
+              } else {
+                uint32_t z8[2];
+                dequant8<T, false>((sub & 2) ? zr[1] : zr[0], z8);  // word sub / 2, bytes (0, 2) or (1, 3)
+                zpair = (sub & 1) ? z8[1] : z8[0];
+              }
+              const uint32_t z_lo = dup_lo(zpair), z_hi = dup_hi(zpair);
+              f[0] = Pair<T>::sub(f[0], z_lo);
+              f[1] = Pair<T>::sub(f[1], z_lo);
+              f[2] = Pair<T>::sub(f[2], z_hi);
+              f[3] = Pair<T>::sub(f[3], z_hi);
+            }
+            if constexpr (decltype(scaled_c)::value) {
+              uint32_t s_lo, s_hi;
+              if constexpr (I::kFp4) {
+                // byte 4 (sub / 2) + 2 h + sub % 2 of the lane's eight belongs to column c8 + 16 sub + 8 h
+                s_lo = fp4_scale<T, F>(sc[sub >> 1], sub & 1);
+                s_hi = fp4_scale<T, F>(sc[sub >> 1], 2 + (sub & 1));
+              } else {
+                s_lo = dup_lo(sc[sub]);
+                s_hi = dup_hi(sc[sub]);
+              }
+              if constexpr (I::kZpF) {
+                // q * s - zp * s with the product zp * s rounded, one fma per pair (as gemm_lookup.cuh)
+                const uint32_t z_lo = Pair<T>::mul(dup_lo(zr[sub]), s_lo) ^ 0x80008000u;
+                const uint32_t z_hi = Pair<T>::mul(dup_hi(zr[sub]), s_hi) ^ 0x80008000u;
+                f[0] = Pair<T>::fma(f[0], s_lo, z_lo);
+                f[1] = Pair<T>::fma(f[1], s_lo, z_lo);
+                f[2] = Pair<T>::fma(f[2], s_hi, z_hi);
+                f[3] = Pair<T>::fma(f[3], s_hi, z_hi);
+              } else {
+                f[0] = Pair<T>::mul(f[0], s_lo);
+                f[1] = Pair<T>::mul(f[1], s_lo);
+                f[2] = Pair<T>::mul(f[2], s_hi);
+                f[3] = Pair<T>::mul(f[3], s_hi);
+              }
+            } else if constexpr (F == kF8) {
+              // true magnitude before the MMA (exact); the epilogue takes the factor out of the scale
+#pragma unroll
+              for (int i = 0; i < 4; ++i) f[i] = Pair<T>::mul(f[i], Fp8Cvt<T>::kRebias);
+            }
+            sts32_off<sub * 2048>(b_lo, f[0]);
+            sts32_off<sub * 2048>(b_hi, f[1]);
+            sts32_off<sub * 2048 + 1024>(b_lo, f[2]);
+            sts32_off<sub * 2048 + 1024>(b_hi, f[3]);
+          };
+          auto convert_all = [&](auto scaled_c) {
+            convert(std::integral_constant<int, 0>{}, scaled_c);
+            convert(std::integral_constant<int, 1>{}, scaled_c);
+            convert(std::integral_constant<int, 2>{}, scaled_c);
+            convert(std::integral_constant<int, 3>{}, scaled_c);
+          };
+          if constexpr (I::kFp4 || I::kZpF) {
+            convert_all(std::true_type{});
+          } else {
+            if (p.channelwise) convert_all(std::false_type{});
+            else convert_all(std::true_type{});
+          }
+        }
+        fence_proxy_async_smem();  // generic-proxy stores -> visible to the tensor core
+        __syncwarp();
+        if (lane == 0) {
+          if (kPair) mbar_arrive_cluster(fa0 + 8 * ring.i);
+          else mbar_arrive(full(ring.i));
+        }
+        ring.next();
+      }
+    }
+  } else {
+    // ================= epilogue: TMEM -> registers -> C ==================================
+    const int quad = warp & 3;  // TMEM lanes 32 quad .. 32 quad + 31
+    const uint32_t te0 = kPair ? mapa(tmem_empty(0), 0) : tmem_empty(0);
+    uint16_t* C = static_cast<uint16_t*>(p.c);
+    int seg_i = 0;
+    bool ok = true;
+    // C, the partial sums and the counters may still be in use by the kernel in front
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    while (ok && sched.next(sg)) {
+      const int buf = seg_i & 1;
+      if (!(ok = mbar_wait<kPair, 100>(tmem_full(buf), (seg_i >> 1) & 1, (4 << 8) | 4, cta_abort, p.error))) break;
+      ++seg_i;
+      tc_fence_after();
+      const int n = (sg.n_tile * CG + (int)rank) * kBN + quad * 32 + lane;  // this lane's output column
+      const bool n_ok = n < p.n;                                            // uniform per warp: N % 64 == 0
+      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * (CG * 128);
+      float cs = 1.f, bs = 0.f;
+      if (n_ok) {
+        if (p.channelwise)
+          cs = Pair<T>::to_float(static_cast<const uint16_t*>(p.scales)[(size_t)sg.expert * p.s_stride + single_perm_pos(n)]) *
+               p.chan_factor;
+        if (F == kNV4) cs = Pair<T>::to_float(*static_cast<const uint16_t*>(p.global_scale));
+        if (p.bias)
+          bs = Pair<T>::to_float(static_cast<const uint16_t*>(p.bias)[(size_t)sg.expert * p.bias_stride + single_perm_pos(n)]);
+      }
+      // Scale, bias, rounding and store of 32 consecutive tokens of the warp's 32 columns.  Lanes pair
+      // up: of two neighbouring tokens the even lane stores the first for both lanes' columns, the odd
+      // lane the second, so that a store instruction writes 64 B of two rows.
+      auto store32 = [&](int t0, const float (&v)[32]) {
+        int my_id = 0;
+        float my_w = 1.f;
+        if (p.ids) {
+          my_id = t0 + lane < sg.rows ? p.ids[sg.tok0 + t0 + lane] : p.out_rows;
+          if (p.row_weights && my_id < p.out_rows) my_w = p.row_weights[my_id];
+        }
+        const bool odd = lane & 1;
+        uint16_t* col = C + (n & ~1);
+        uint32_t word[16];
+#pragma unroll
+        for (int t = 0; t < 32; t += 2) {
+          float a = v[t] * cs + bs, b = v[t + 1] * cs + bs;
+          if (p.ids) {
+            a *= __shfl_sync(~0u, my_w, t);
+            b *= __shfl_sync(~0u, my_w, t + 1);
+          }
+          const uint32_t mine = (uint32_t)Pair<T>::from_float(a) | ((uint32_t)Pair<T>::from_float(b) << 16);
+          const uint32_t theirs = __shfl_xor_sync(~0u, mine, 1);
+          word[t / 2] = odd ? __byte_perm(theirs, mine, 0x7632) : __byte_perm(mine, theirs, 0x5410);
+        }
+#pragma unroll
+        for (int t = 0; t < 32; t += 2) {
+          const int tt = t0 + t + (odd ? 1 : 0);
+          long long row = sg.tok0 + tt;
+          bool row_ok = tt < sg.rows;
+          if (p.ids) {
+            const int id = __shfl_sync(~0u, my_id, t + (odd ? 1 : 0));
+            row = id;
+            row_ok = row_ok && id < p.out_rows;
+          }
+          if (row_ok) *reinterpret_cast<uint32_t*>(col + (size_t)row * p.n) = word[t / 2];
+        }
+      };
+      auto release = [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (kPair) mbar_arrive_cluster(te0 + 8 * buf);
+          else mbar_arrive(tmem_empty(buf));
+        }
+      };
+      if (!sg.shared) {
+        for (int t0 = 0; t0 < sg.rows; t0 += 32) {
+          uint32_t r[32];
+          tmem_ld32(taddr + t0, r);
+          tmem_ld_wait();
+          if (n_ok) {
+            float v[32];
+#pragma unroll
+            for (int t = 0; t < 32; ++t) v[t] = __uint_as_float(r[t]);
+            store32(t0, v);
+          }
+        }
+        release();
+      } else {
+        // partial sums, token-major: a warp writes 128 B per token
+        const size_t slot_floats = (size_t)p.tn * kBN;
+        auto slot_ptr = [&](int slot) {
+          return p.partials + ((size_t)slot * CG + rank) * slot_floats + quad * 32 + lane;
+        };
+        float* mine = slot_ptr(sg.slot);
+        for (int t0 = 0; t0 < sg.rows; t0 += 32) {
+          uint32_t r[32];
+          tmem_ld32(taddr + t0, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int t = 0; t < 32; ++t)
+            if (t0 + t < sg.rows) __stcg(mine + (size_t)(t0 + t) * kBN, __uint_as_float(r[t]));
+        }
+        release();
+        if (p.reduce_later) continue;
+        __threadfence();
+        __syncwarp();
+        // one byte of the counter per quadrant: every warp hands over its own quarter of the tile
+        int32_t* counter = p.counters + sg.first * CG + rank;
+        uint32_t seen = 0;
+        if (lane == 0) seen = (uint32_t)atomicAdd(counter, 1 << (8 * quad)) >> (8 * quad) & 0xffu;
+        seen = __shfl_sync(~0u, seen, 0);
+        if ((int)seen == sg.contributors - 1) {
+          if (lane == 0) atomicSub(counter, sg.contributors << (8 * quad));
+          __threadfence();
+          for (int t0 = 0; t0 < sg.rows; t0 += 32) {
+            float v[32];
+#pragma unroll
+            for (int t = 0; t < 32; ++t) v[t] = 0.f;
+            for (int i = 0; i < sg.contributors; ++i) {
+              // the first contributor's piece begins the tile (slot 1 of its worker)
+              const float* src = slot_ptr(2 * (sg.first + i) + (i == 0 ? 1 : 0));
+#pragma unroll
+              for (int t = 0; t < 32; ++t)
+                if (t0 + t < sg.rows) v[t] += __ldcg(src + (size_t)(t0 + t) * kBN);
+            }
+            if (n_ok) store32(t0, v);
+          }
+        }
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  // no CTA of the pair may leave while the other may still arrive on its barriers or read its memory
+  if (kPair) {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  }
+  if (warp == kMmaWarp) {
+    tc_fence_after();
+    tmem_dealloc<CG>(tmem_base, kTmemCols);
+  }
+}
+
+}  // namespace tc
+}  // namespace b200q
