@@ -140,6 +140,10 @@ struct Pair<half> {
   static __device__ __forceinline__ uint16_t from_float(float f) {
     return __half_as_ushort(__float2half_rn(f));
   }
+  static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
+    half2 r = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<uint32_t*>(&r);
+  }
 };
 template <>
 struct Pair<__nv_bfloat16> {
@@ -164,6 +168,10 @@ struct Pair<__nv_bfloat16> {
   }
   static __device__ __forceinline__ uint16_t from_float(float f) {
     return __bfloat16_as_ushort(__float2bfloat16_rn(f));
+  }
+  static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
+    __nv_bfloat162 r = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<uint32_t*>(&r);
   }
 };
 

@@ -15,9 +15,10 @@
 //                     2-D copy each (deep: this is what comes from HBM; with a copy per step and per scale
 //                     row the issuing thread was the bottleneck at 925 cycles a step)
 //   token warp        token rows of a round (TMA, 128B swizzle) into kRing slots
-//   16 dequant warps  a warp converts one 16 x 64 Marlin tile of the round: packed words -> exact 16-bit
-//                     codes -> scaled -> K-major swizzled operand in shared memory; the words of the next
-//                     round are fetched before the current ones are converted
+//   16 dequant warps  packed words -> exact 16-bit codes -> scaled -> K-major swizzled operand in shared
+//                     memory.  Two groups of eight take alternate rounds, a warp two 16 x 64 Marlin tiles:
+//                     one group waits and fetches while the other converts (with all sixteen on every round
+//                     a round took 1450 cycles, half of them waits that all warps sat out together)
 //   MMA warp          one elected lane issues eight 128 (256) x tn x 16 MMAs per round, commits the slot back
 //                     (a satisfied barrier wait costs about 200 cycles beside twenty busy warps, so token rows
 //                     and converted weights share one barrier, and it is waited for once per round)
@@ -67,7 +68,7 @@ struct FmtInfo {
 constexpr int kBK = 64;            // k per step: one 128-byte swizzle row of 16-bit values
 constexpr int kRoundTiles = 8;     // k-tiles (16 rows) per round of two steps
 constexpr int kBN = 128;           // weight columns per CTA
-constexpr int kDequantWarps = 16;  // eight for each step of a round
+constexpr int kDequantWarps = 16;  // two groups of eight
 constexpr int kEpiWarp0 = kDequantWarps;  // 4 warps: TMEM lane quadrant = warp % 4
 constexpr int kProducerWarp = kEpiWarp0 + 4;
 constexpr int kTokenWarp = kProducerWarp + 1;
@@ -288,7 +289,7 @@ struct TcCfg {
   static constexpr int kRing = TOK == 64 ? 3 : 2;
   static constexpr int kBarBytes = 1024;
   static constexpr int kFit = (226 * 1024 - kBarBytes - 1024 - kRing * kSlot) / kWSlot;
-  static constexpr int kWD = kFit >= 8 ? 8 : kFit;
+  static constexpr int kWD = kFit >= 8 ? 8 : kFit / 2 * 2;  // even: a slot always belongs to the same group
   static constexpr int kSmemBytes = kRing * kSlot + kWD * kWSlot + kBarBytes + 1024;  // + alignment slack
 };
 
@@ -297,8 +298,9 @@ template <int N>
 struct Ring {
   int i = 0;
   uint32_t ph = 0;
-  __device__ __forceinline__ void next() {
-    if (++i == N) { i = 0; ph ^= 1; }
+  __device__ __forceinline__ void next(int by = 1) {
+    i += by;
+    if (i >= N) { i -= N; ph ^= 1; }
   }
 };
 
@@ -467,12 +469,12 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
   if (threadIdx.x == 0) {
     s_abort = 0;
     for (int i = 0; i < RING; ++i) {
-      mbar_init(full(i), 1 + kDequantWarps * CG);
+      mbar_init(full(i), 1 + kDequantWarps / 2 * CG);
       mbar_init(empty(i), 1);
     }
     for (int w = 0; w < WD; ++w) {
       mbar_init(full_w(w), 1);
-      mbar_init(empty_w(w), kDequantWarps);
+      mbar_init(empty_w(w), kDequantWarps / 2);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(tmem_full(b), 1);
@@ -583,81 +585,77 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
   } else if (warp < kDequantWarps) {
     // ================= dequant warps ====================================================
     const int c8 = lane >> 2, q = lane & 3;
-    const int step = warp >> 3;           // step of the round
-    const int kt = warp & 3, nt = (warp >> 2) & 1;
-    const int rkt = 4 * step + kt;        // k-tile within the round
+    const int group = warp >> 3;
+    const int kt = warp & 3, nt = (warp >> 2) & 1;  // k-tile of both steps of the round, column tile
     // byte offsets of this lane's two k-positions (k = 16 kt + 2q, + 8) inside a 128 B row
-    const uint32_t a_rel = 2 * Cfg::kTokBytes + step * Cfg::kABytes;
-    const uint32_t b_lo_rel = a_rel + (nt * 64 + c8) * 128 + (((2 * kt) ^ c8) << 4) + 4 * q;
-    const uint32_t b_hi_rel = a_rel + (nt * 64 + c8) * 128 + (((2 * kt + 1) ^ c8) << 4) + 4 * q;
-    const uint32_t w_rel = rkt * (2 * Cfg::kTileBytes) + nt * Cfg::kTileBytes + lane * (BITS * 4);
+    const uint32_t b_lo_rel = 2 * Cfg::kTokBytes + (nt * 64 + c8) * 128 + (((2 * kt) ^ c8) << 4) + 4 * q;
+    const uint32_t b_hi_rel = 2 * Cfg::kTokBytes + (nt * 64 + c8) * 128 + (((2 * kt + 1) ^ c8) << 4) + 4 * q;
+    const uint32_t w_rel = kt * (2 * Cfg::kTileBytes) + nt * Cfg::kTileBytes + lane * (BITS * 4);
     const uint32_t fa0 = kPair ? mapa(full(0), 0) : full(0);
-    // scale row of this k-tile within the round's copy, where it is the same in every round
+    // scale rows of this warp's two k-tiles within the round's copy, where they are the same in every round
     const bool fixed_row = (gb & 7) == 0 || (8 % gb) == 0;
-    const int row0 = (gb & 7) == 0 ? 0 : rkt / gb;
+    const int row0 = (gb & 7) == 0 ? 0 : kt / gb, row1 = (gb & 7) == 0 ? 0 : (kt + 4) / gb;
+    // (with three slots a group meets a slot every other pass; the MMAs retire in order and the group has
+    // waited for later ones in between, so the parity of the pass is never ambiguous)
     Ring<WD> wr;
     Ring<RING> ring;
+    wr.next(group);
+    ring.next(group);
+    int it = 0;  // rounds seen so far
     bool ok = true;
-    // packed words of the lane, [sub] (4-bit) or [2 sub + block] (8-bit), scales and zero-points: the next
-    // round's (n_) and the current one's
     constexpr int NW = BITS == 4 ? 4 : 8;
-    uint32_t n_w[NW], n_sc[4], n_zr[4], w[NW], sc[4], zr[4];
-    auto fetch = [&](int r) {
-      const uint32_t wslot = w_base + wr.i * Cfg::kWSlot;
-#pragma unroll
-      for (int v = 0; v < BITS / 4; ++v) {
-        const uint4 w4 = lds128(wslot + w_rel + v * 16);
-        n_w[4 * v] = w4.x; n_w[4 * v + 1] = w4.y; n_w[4 * v + 2] = w4.z; n_w[4 * v + 3] = w4.w;
-      }
-      if constexpr (I::kFp4) {
-        // 16 bytes per (tile, c8) of a pair of groups; this k-tile's group is half of them
-        const uint32_t pair = F == kNV4 ? rkt >> 1 : rkt >> 2, half = F == kNV4 ? rkt & 1 : (rkt >> 1) & 1;
-        const uint32_t src = wslot + Cfg::kWBytes + pair * 256 + nt * 128 + c8 * 16 + half * 8;
-        n_sc[0] = lds32(src);
-        n_sc[1] = lds32(src + 4);
-      } else {
-        const int row = fixed_row ? row0 : (r * kRoundTiles + rkt) / gb - (r * kRoundTiles) / gb;
-        if (!p.channelwise) {
-          const uint4 s4 = lds128(wslot + Cfg::kWBytes + row * Cfg::kSRow + nt * 128 + c8 * 16);
-          n_sc[0] = s4.x; n_sc[1] = s4.y; n_sc[2] = s4.z; n_sc[3] = s4.w;
-        }
-        if constexpr (I::kZp) {
-          const uint32_t zsrc = wslot + Cfg::kWBytes + Cfg::kSBytes + row * Cfg::kZRow + nt * (8 * BITS) + c8 * BITS;
-          n_zr[0] = lds32(zsrc);
-          if (BITS == 8) n_zr[1] = lds32(zsrc + 4);
-        }
-        if constexpr (I::kZpF) {
-          const uint4 z4 = lds128(wslot + Cfg::kWBytes + Cfg::kSBytes + row * Cfg::kZRow + nt * 128 + c8 * 16);
-          n_zr[0] = z4.x; n_zr[1] = z4.y; n_zr[2] = z4.z; n_zr[3] = z4.w;
-        }
-      }
-    };
-    bool more = sched.next(sg);
-    int nr = sg.r0;  // the next round to fetch
-    if (more) {
-      if ((ok = mbar_wait<false>(full_w(wr.i), wr.ph, (3 << 8) | 1, cta_abort, p.error))) fetch(nr);
-    }
-    while (ok && more) {
-      const bool live = (sg.n_tile * CG + (int)rank) * 2 + nt < NT && 2 * nr + step < steps;
-#pragma unroll
-      for (int i = 0; i < NW; ++i) w[i] = n_w[i];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) { sc[i] = n_sc[i]; zr[i] = n_zr[i]; }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(empty_w(wr.i));
-      wr.next();
-      if (++nr == sg.r1) {
-        more = sched.next(sg);
-        nr = sg.r0;
-      }
-      if (more) {
+    while (ok && sched.next(sg)) {
+      const bool live = (sg.n_tile * CG + (int)rank) * 2 + nt < NT;
+      for (int r = sg.r0 + ((it ^ group) & 1); r < sg.r1; r += 2) {
+        const uint32_t wslot = w_base + wr.i * Cfg::kWSlot;
         if (!(ok = mbar_wait<false>(full_w(wr.i), wr.ph, (3 << 8) | 1, cta_abort, p.error))) break;
-        fetch(nr);
-      }
-      if (!(ok = mbar_wait<kPair>(empty(ring.i), ring.ph ^ 1, (3 << 8) | 4, cta_abort, p.error))) break;
-      {
+        // packed words of the lane, [sub] (4-bit) or [2 sub + block] (8-bit), scales and zero-points of the
+        // two tiles
+        uint32_t w2[2][NW], sc2[2][4], zr2[2][4];
+#pragma unroll
+        for (int st = 0; st < 2; ++st) {
+#pragma unroll
+          for (int v = 0; v < BITS / 4; ++v) {
+            const uint4 w4 = lds128(wslot + w_rel + st * (8 * Cfg::kTileBytes) + v * 16);
+            w2[st][4 * v] = w4.x; w2[st][4 * v + 1] = w4.y; w2[st][4 * v + 2] = w4.z; w2[st][4 * v + 3] = w4.w;
+          }
+          const int rkt = 4 * st + kt;
+          if constexpr (I::kFp4) {
+            // 16 bytes per (tile, c8) of a pair of groups; this k-tile's group is half of them
+            const uint32_t pair = F == kNV4 ? rkt >> 1 : st, half = F == kNV4 ? rkt & 1 : (rkt >> 1) & 1;
+            const uint32_t src = wslot + Cfg::kWBytes + pair * 256 + nt * 128 + c8 * 16 + half * 8;
+            sc2[st][0] = lds32(src);
+            sc2[st][1] = lds32(src + 4);
+          } else {
+            const int row = fixed_row ? (st ? row1 : row0) : (r * kRoundTiles + rkt) / gb - (r * kRoundTiles) / gb;
+            if (!p.channelwise) {
+              const uint4 s4 = lds128(wslot + Cfg::kWBytes + row * Cfg::kSRow + nt * 128 + c8 * 16);
+              sc2[st][0] = s4.x; sc2[st][1] = s4.y; sc2[st][2] = s4.z; sc2[st][3] = s4.w;
+            }
+            if constexpr (I::kZp) {
+              const uint32_t zsrc = wslot + Cfg::kWBytes + Cfg::kSBytes + row * Cfg::kZRow + nt * (8 * BITS) + c8 * BITS;
+              zr2[st][0] = lds32(zsrc);
+              if (BITS == 8) zr2[st][1] = lds32(zsrc + 4);
+            }
+            if constexpr (I::kZpF) {
+              const uint4 z4 = lds128(wslot + Cfg::kWBytes + Cfg::kSBytes + row * Cfg::kZRow + nt * 128 + c8 * 16);
+              zr2[st][0] = z4.x; zr2[st][1] = z4.y; zr2[st][2] = z4.z; zr2[st][3] = z4.w;
+            }
+          }
+        }
+        if (!(ok = mbar_wait<kPair>(empty(ring.i), ring.ph ^ 1, (3 << 8) | 4, cta_abort, p.error))) break;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty_w(wr.i));
+        wr.next(2);
         if (live) {
-          const uint32_t b_lo = smem_base + ring.i * Cfg::kSlot + b_lo_rel, b_hi = smem_base + ring.i * Cfg::kSlot + b_hi_rel;
+          const uint32_t b_lo0 = smem_base + ring.i * Cfg::kSlot + b_lo_rel, b_hi0 = smem_base + ring.i * Cfg::kSlot + b_hi_rel;
+#pragma unroll
+          for (int st = 0; st < 2; ++st) {
+          if (2 * r + st >= steps) break;  // the last round of an odd number of steps
+          const uint32_t b_lo = b_lo0 + st * Cfg::kABytes, b_hi = b_hi0 + st * Cfg::kABytes;
+          const uint32_t (&w)[NW] = w2[st];
+          const uint32_t (&sc)[4] = sc2[st];
+          const uint32_t (&zr)[4] = zr2[st];
           auto convert = [&](auto sub_c, auto scaled_c) {
             constexpr int sub = decltype(sub_c)::value;
             uint32_t f[4];
@@ -726,6 +724,7 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
             if (p.channelwise) convert_all(std::false_type{});
             else convert_all(std::true_type{});
           }
+          }
         }
         fence_proxy_async_smem();  // generic-proxy stores -> visible to the tensor core
         __syncwarp();
@@ -733,8 +732,9 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
           if (kPair) mbar_arrive_cluster(fa0 + 8 * ring.i);
           else mbar_arrive(full(ring.i));
         }
-        ring.next();
+        ring.next(2);
       }
+      it += sg.r1 - sg.r0;
     }
   } else {
     // ================= epilogue: TMEM -> registers -> C ==================================
@@ -773,7 +773,6 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
           if (p.row_weights && my_id < p.out_rows) my_w = p.row_weights[my_id];
         }
         const bool odd = lane & 1;
-        uint16_t* col = C + (n & ~1);
         uint32_t word[16];
 #pragma unroll
         for (int t = 0; t < 32; t += 2) {
@@ -782,21 +781,29 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
             a *= __shfl_sync(~0u, my_w, t);
             b *= __shfl_sync(~0u, my_w, t + 1);
           }
-          const uint32_t mine = (uint32_t)Pair<T>::from_float(a) | ((uint32_t)Pair<T>::from_float(b) << 16);
+          const uint32_t mine = Pair<T>::pack(a, b);
           const uint32_t theirs = __shfl_xor_sync(~0u, mine, 1);
           word[t / 2] = odd ? __byte_perm(theirs, mine, 0x7632) : __byte_perm(mine, theirs, 0x5410);
         }
+        const int t1 = t0 + (odd ? 1 : 0);
+        if (!p.ids) {
+          uint16_t* dst = C + (size_t)(sg.tok0 + t1) * p.n + (n & ~1);
+          const size_t step2 = (size_t)2 * p.n;
+          if (t0 + 32 <= sg.rows) {
 #pragma unroll
-        for (int t = 0; t < 32; t += 2) {
-          const int tt = t0 + t + (odd ? 1 : 0);
-          long long row = sg.tok0 + tt;
-          bool row_ok = tt < sg.rows;
-          if (p.ids) {
-            const int id = __shfl_sync(~0u, my_id, t + (odd ? 1 : 0));
-            row = id;
-            row_ok = row_ok && id < p.out_rows;
+            for (int t = 0; t < 32; t += 2, dst += step2) *reinterpret_cast<uint32_t*>(dst) = word[t / 2];
+          } else {
+#pragma unroll
+            for (int t = 0; t < 32; t += 2, dst += step2)
+              if (t1 + t < sg.rows) *reinterpret_cast<uint32_t*>(dst) = word[t / 2];
           }
-          if (row_ok) *reinterpret_cast<uint32_t*>(col + (size_t)row * p.n) = word[t / 2];
+        } else {
+#pragma unroll
+          for (int t = 0; t < 32; t += 2) {
+            const int id = __shfl_sync(~0u, my_id, t + (odd ? 1 : 0));
+            if (t1 + t < sg.rows && id < p.out_rows)
+              *reinterpret_cast<uint32_t*>(C + (size_t)id * p.n + (n & ~1)) = word[t / 2];
+          }
         }
       };
       auto release = [&]() {
