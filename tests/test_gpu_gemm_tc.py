@@ -124,3 +124,41 @@ def test_tc_gemm_many_tiles_per_cta(env):
         for r0 in (0, 5000, 16384, 32768 - 16):
             small = f(a[r0:r0 + 16].contiguous()).float()
             assert (small - big[r0:r0 + 16]).abs().max().item() <= 2e-2 * scale, r0
+
+
+@pytest.mark.parametrize("M,K,N,qtype,group,dtype", [
+    (64, 192, 64, "uint4b8", 64, "float16"),        # an odd number of 64-deep steps, half a column tile
+    (97, 128, 192, "uint8b128", 16, "float16"),     # eight scale rows per round
+    (128, 576, 128, "uint4", 48, "bfloat16"),       # groups that straddle rounds
+    (129, 4096, 320, "uint4", -1, "float16"),       # CTA pairs, second CTA of a pair without columns, shared tiles
+    (192, 1088, 640, "uint4b8", 32, "bfloat16"),
+    (193, 2048, 256, "uint8b128", 128, "bfloat16"),
+    (257, 8192, 128, "uint4b8", 128, "float16"),    # more workers than tiles
+    (385, 640, 4736, "uint4b8", 128, "bfloat16"),
+])
+def test_tc_gemm_edges(env, M, K, N, qtype, group, dtype):
+    torch, G, ops, mu, lib = env
+    L = H.make_layer(K, N, qtype, group, False, dtype)
+    a = H.make_activations(M, K, dtype)
+    out = G.run_gemm(ops, mu, L, a)
+    assert lib.b200q_device_error(1) == 0
+    _check(out, mo.gemm_ref(a, L.w), f"{M} {K} {N} {qtype} g{group}")
+
+
+@pytest.mark.parametrize("M,qtype,group", [(100, "uint4b8", 128), (300, "uint8b128", -1), (700, "uint8b128", 128)])
+def test_tc_gemm_is_reproducible(env, M, qtype, group):
+    """The same call gives the same bits every time: a weight slot that is refilled before it was read
+    (the rings of these shapes are two slots deep) shows as a rare difference."""
+    torch, G, ops, mu, lib = env
+    from vllm_b200.scalar_type import ScalarType
+    K, N, bits = 3584, 4608, H.TYPE_BITS[qtype]
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    q = torch.randint(-2**31, 2**31 - 1, (K // 16, N * bits // 2), dtype=torch.int32, device="cuda", generator=gen)
+    s = (torch.rand((K // group if group > 0 else 1, N), device="cuda", generator=gen) * 0.018 + 0.002).half()
+    a = torch.randn((M, K), device="cuda", dtype=torch.float16, generator=gen)
+    ws, e = mu.marlin_make_workspace_new(torch.device("cuda")), torch.empty(0, dtype=torch.int32, device="cuda")
+    run = lambda: ops.gptq_marlin_gemm(a, None, q, None, s, None, e, e, e, ws, ScalarType.from_id(H.TYPE_IDS[qtype]),
+                                       M, N, K, True, False, True, False)
+    first = run()
+    assert all(torch.equal(first, run()) for _ in range(40))
+    assert lib.b200q_device_error(1) == 0

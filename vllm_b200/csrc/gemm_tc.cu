@@ -1,19 +1,10 @@
 // Host side of the tensor-core GEMM (gemm_tc.cuh): tensor maps, tile plan, dispatch by format.
 #include "gemm_tc.cuh"
 
-#include <mutex>
-#include <unordered_map>
-
 namespace b200q {
 namespace tc {
 
 __device__ int g_tc_error;
-
-// Arrival counters of shared tiles, zero between kernels.  One row per stream (calls on one stream are
-// ordered, calls on different streams may overlap); a process with more streams than rows runs its
-// further streams without shared tiles.
-constexpr int kCounterRows = 1024, kCounterLen = 256;
-__device__ int32_t g_tc_counters[kCounterRows][kCounterLen];
 
 // one definition per (type, format), in the gemm_tc_inst.cu units
 template <typename T, int F>
@@ -39,25 +30,16 @@ static EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
-// Device addresses of the error word and of the stream's counters (null when there are no rows left).
-static int device_words(cudaStream_t stream, int** error, int32_t** counters) {
-  static std::mutex mu;
-  static struct { int* error; int32_t* counters; std::unordered_map<cudaStream_t, int> rows; } per_device[64];
+static int error_word(int** out) {
+  static int* addr[64] = {};  // per device; benign race: the same value every time
   int dev = 0;
   B200Q_CUDA_OK(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lock(mu);
-  auto& d = per_device[dev & 63];
-  if (!d.error) {
-    void *e = nullptr, *c = nullptr;
-    B200Q_CUDA_OK(cudaGetSymbolAddress(&c, g_tc_counters));
-    B200Q_CUDA_OK(cudaGetSymbolAddress(&e, g_tc_error));
-    d.counters = static_cast<int32_t*>(c);
-    d.error = static_cast<int*>(e);
+  if (!addr[dev & 63]) {
+    void* a = nullptr;
+    B200Q_CUDA_OK(cudaGetSymbolAddress(&a, g_tc_error));
+    addr[dev & 63] = static_cast<int*>(a);
   }
-  *error = d.error;
-  auto it = d.rows.find(stream);
-  if (it == d.rows.end() && (int)d.rows.size() < kCounterRows) it = d.rows.emplace(stream, (int)d.rows.size()).first;
-  *counters = it == d.rows.end() ? nullptr : d.counters + (size_t)it->second * kCounterLen;
+  *out = addr[dev & 63];
   return B200Q_OK;
 }
 
@@ -117,21 +99,22 @@ static int make_a_map(CUtensorMap* map, const void* a, int64_t lda, int64_t m, i
   return B200Q_OK;
 }
 
-// Sums of tiles that are all shared: one thread per token and four columns, contributors in k order.
+// Sums of the shared tiles: blockIdx.y = tile, one thread per token and four columns, contributors in k
+// order.
 template <typename T>
 __global__ void __launch_bounds__(256) tc_reduce_kernel(const TcParams p, int cg) {
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-  const int n4 = p.n / 4;
-  const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
-  if (idx >= (long long)p.m * n4) return;
-  const int tok = (int)(idx / n4), n = (int)(idx - (long long)tok * n4) * 4;
+  const int cols4 = cg * kBN / 4;
+  const int idx = blockIdx.x * 256 + threadIdx.x, tile = blockIdx.y;
+  const int tt = idx / cols4, col = (idx - tt * cols4) * 4;  // inside the tile
+  const int n_tile = tile / p.tok_tiles, tok = (tile - n_tile * p.tok_tiles) * p.tn + tt;
+  const int n = n_tile * cg * kBN + col;
+  if (tt >= p.tn || tok >= p.m || n >= p.n) return;
   const int rounds = (p.k / kBK + 1) / 2;
-  const long long units = (long long)p.sk_tiles * rounds;
-  const int cols = cg * kBN, tok_tile = tok / p.tn;
-  const long long unit0 = ((long long)(n / cols) * p.tok_tiles + tok_tile) * rounds;
+  const long long units = (long long)p.sk_tiles * rounds, unit0 = (long long)tile * rounds;
   const int first = share_of(unit0, p.workers, units);
   const int count = share_of(unit0 + rounds - 1, p.workers, units) - first + 1;
-  const float* src = p.partials + ((size_t)((n / kBN) % cg) * p.tn + (tok - tok_tile * p.tn)) * kBN + n % kBN;
+  const float* src = p.partials + ((size_t)(col / kBN) * p.tn + tt) * kBN + col % kBN;
   const size_t slot_floats = (size_t)cg * p.tn * kBN;
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   float v[4] = {0.f, 0.f, 0.f, 0.f};
@@ -140,7 +123,7 @@ __global__ void __launch_bounds__(256) tc_reduce_kernel(const TcParams p, int cg
 #pragma unroll
     for (int i = 0; i < 4; ++i)
       if (i0 + i < count)
-        // the first contributor's piece begins the tile (slot 1 of its worker)
+        // a piece that begins the tile is in slot 1 of its worker, any other in slot 0
         x[i] = __ldcg(reinterpret_cast<const float4*>(src + (2 * (first + i0 + i) + (i0 + i == 0 ? 1 : 0)) * slot_floats));
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -161,9 +144,8 @@ __global__ void __launch_bounds__(256) tc_reduce_kernel(const TcParams p, int cg
 
 template <typename T>
 static int launch_reduce(const TcParams& p, int cg, cudaStream_t stream) {
-  const long long threads = (long long)p.m * (p.n / 4);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((threads + 255) / 256));
+  cfg.gridDim = dim3((unsigned)((p.tn * cg * kBN / 4 + 255) / 256), (unsigned)p.sk_tiles);
   cfg.blockDim = dim3(256);
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
@@ -177,60 +159,58 @@ static int launch_reduce(const TcParams& p, int cg, cudaStream_t stream) {
 }
 
 struct TcPlan {
-  int cg, tn, box, tok_tiles, workers, sk_tiles, reduce_later;
+  int cg, tn, box, tok_tiles, workers, sk_tiles;
   int64_t partial_bytes;
 };
 
-// Tile and work split by estimated time (microseconds; the constants are measured on B200).  Candidates:
-// single CTAs with token tiles of up to 128 rows, CTA pairs with up to 256; whole tiles only, the ragged
-// last wave shared by k-range, or, with fewer tiles than workers, all tiles shared and added up by the
-// reduce kernel.
+// Microseconds of a round (128 deep in k) of one tile, measured on B200 as the slope over K at one tile per
+// worker (4-bit: 0.45 at 48 tokens, 0.58 at 128; pairs 0.57 at 160, 0.78 at 256; other formats run 0 to 15 %
+// longer, which moves the choice little).
+static double round_us(int cg, int tn) {
+  if (cg == 1) return tn <= 64 ? 0.45 : 0.46 + 0.00096 * tn;
+  const double t = 0.22 + 0.00217 * tn;
+  return t < 0.5 ? 0.5 : t;
+}
+
+// Tile and work split by estimated time.  Candidates: single CTAs with token tiles of up to 128 rows, CTA
+// pairs with up to 256, a few tile widths each; whole tiles only, or the ragged last wave shared by
+// k-range (its partial sums are written and read once, and cost a launch).
 static TcPlan plan_tiles(int64_t m, int64_t n, int64_t k, int sms, int64_t scratch_bytes) {
   const int64_t rounds = (k / kBK + 1) / 2;
   TcPlan best = {};
   double best_cost = 1e300;
   for (int cg = 1; cg <= 2; ++cg) {
-    if (cg == 2 && m <= 128) break;
+    if (cg == 2 && m <= 64) break;
     const int64_t most = 128 * cg, grain = 16 * cg;
-    TcPlan pl = {};
-    pl.cg = cg;
     const int64_t want = (m + most - 1) / most;
-    pl.tn = (int)(((m + want - 1) / want + grain - 1) / grain * grain);
-    pl.tok_tiles = (int)((m + pl.tn - 1) / pl.tn);
-    pl.box = pl.tn / cg;
-    const int64_t cols = kBN * cg, most_workers = sms / cg;
-    const int64_t tiles = (n + cols - 1) / cols * pl.tok_tiles;
-    // a round: bound by the conversion, or by the MMAs of a full pair tile
-    const double round = cg == 2 ? 0.47 + 0.13 * pl.tn / 256 : 0.47 + 0.08 * pl.tn / 128;
-    const int64_t slot_bytes = (int64_t)cg * pl.tn * kBN * 4;
-    // whole tiles
-    {
+    int last_tn = 0;
+    for (int64_t more = 0; more < 4; ++more) {
+      TcPlan pl = {};
+      pl.cg = cg;
+      pl.tn = (int)(((m + want + more - 1) / (want + more) + grain - 1) / grain * grain);
+      if (pl.tn == last_tn) continue;
+      last_tn = pl.tn;
+      pl.tok_tiles = (int)((m + pl.tn - 1) / pl.tn);
+      pl.box = pl.tn / cg;
+      const int64_t cols = kBN * cg, most_workers = sms / cg;
+      const int64_t tiles = (n + cols - 1) / cols * pl.tok_tiles;
+      const double round = round_us(cg, pl.tn);
+      const int64_t waves = tiles / most_workers, rem = tiles % most_workers;
       pl.workers = (int)(tiles < most_workers ? tiles : most_workers);
-      const double cost = (double)((tiles + most_workers - 1) / most_workers * rounds) * round;
+      double cost = (double)((waves + (rem > 0)) * rounds) * round;
       if (cost < best_cost) { best_cost = cost; best = pl; }
-    }
-    const int64_t rem = tiles % most_workers;
-    if (rem == 0 || most_workers * cg > kCounterLen) continue;
-    if (tiles > most_workers) {
-      // the ragged wave together with one whole wave, so that no worker's share is a sliver; the additions
-      // hide behind a further whole wave where there is one
-      pl.workers = (int)most_workers;
-      pl.sk_tiles = (int)(rem + most_workers);
-      pl.partial_bytes = 2 * most_workers * slot_bytes;
-      const double cost = (double)(tiles * rounds) / (double)most_workers * round +
-                          (tiles >= 2 * most_workers ? 1.5 : 2.0 + 8.0 * pl.tn / (128 * cg));
-      if (pl.partial_bytes <= scratch_bytes && cost < best_cost) { best_cost = cost; best = pl; }
-    } else {
+      if (rem == 0) continue;
       // at least two rounds for every worker
-      int64_t workers = tiles * rounds / 2;
-      if (workers > most_workers) workers = most_workers;
-      if (workers <= tiles) continue;
+      const int64_t by_work = rem * rounds / 2;
+      int64_t workers = by_work < most_workers ? by_work : most_workers;
+      if (waves > 0) workers = most_workers;
+      if (workers <= rem) continue;
       pl.workers = (int)workers;
-      pl.sk_tiles = (int)tiles;
-      pl.reduce_later = 1;
+      pl.sk_tiles = (int)rem;
+      const int64_t slot_bytes = (int64_t)cg * pl.tn * kBN * 4;
       pl.partial_bytes = 2 * workers * slot_bytes;
-      const double cost = (double)((tiles * rounds + workers - 1) / workers) * round + 2.5 +
-                          2.0 * (double)((workers + tiles) * slot_bytes) / 4e6;
+      cost = (double)(waves * rounds + (rem * rounds + workers - 1) / workers) * round + 2.5 +
+             2.0 * (double)((workers + rem) * slot_bytes) / 4e6;
       if (pl.partial_bytes <= scratch_bytes && cost < best_cost) { best_cost = cost; best = pl; }
     }
   }
@@ -270,9 +250,9 @@ int launch_tc_gemm(const void* a, int64_t lda, const uint32_t* b, const void* sc
                    int64_t size_n, int64_t size_k, int group_blocks, int channelwise, void* scratch,
                    int64_t scratch_bytes, cudaStream_t stream) {
   tc::TcParams p = {};
-  int rc = tc::device_words(stream, &p.error, &p.counters);
+  int rc = tc::error_word(&p.error);
   if (rc != B200Q_OK) return rc;
-  const tc::TcPlan plan = tc::plan_tiles(size_m, size_n, size_k, device_sm_count(), p.counters ? scratch_bytes : 0);
+  const tc::TcPlan plan = tc::plan_tiles(size_m, size_n, size_k, device_sm_count(), scratch_bytes);
   tc::TcMaps maps = {};
   p.group_blocks = group_blocks; p.channelwise = channelwise;
   rc = tc::make_a_map(&maps.a, a, lda, size_m, size_k, plan.box, a_dtype);
@@ -281,7 +261,7 @@ int launch_tc_gemm(const void* a, int64_t lda, const uint32_t* b, const void* sc
   p.scales = scales; p.bias = bias; p.global_scale = global_scale; p.c = c;
   p.m = (int)size_m; p.n = (int)size_n; p.k = (int)size_k;
   p.tn = plan.tn; p.box = plan.box; p.tok_tiles = plan.tok_tiles; p.workers = plan.workers;
-  p.sk_tiles = plan.sk_tiles; p.reduce_later = plan.reduce_later;
+  p.sk_tiles = plan.sk_tiles;
   p.chan_factor = fmt != tc::kF8 ? 1.f : a_dtype == B200Q_F16 ? Fp8Cvt<half>::kRebiasInv : Fp8Cvt<__nv_bfloat16>::kRebiasInv;
   p.partials = static_cast<float*>(scratch);
   // early launch only where this kernel's fixed costs matter: with many rows the waiting CTAs would take
@@ -289,7 +269,7 @@ int launch_tc_gemm(const void* a, int64_t lda, const uint32_t* b, const void* sc
   const bool pdl = pdl_enabled() && size_m <= 128;
   rc = a_dtype == B200Q_F16 ? tc::launch_type<half>(maps, p, fmt, plan.cg, pdl, stream)
                             : tc::launch_type<__nv_bfloat16>(maps, p, fmt, plan.cg, pdl, stream);
-  if (rc != B200Q_OK || !plan.reduce_later) return rc;
+  if (rc != B200Q_OK || plan.sk_tiles == 0) return rc;
   return a_dtype == B200Q_F16 ? tc::launch_reduce<half>(p, plan.cg, stream)
                               : tc::launch_reduce<__nv_bfloat16>(p, plan.cg, stream);
 }
@@ -306,9 +286,6 @@ int tc_error_flag(bool reset) {
   if (reset && v != 0) {
     int zero = 0;
     cudaMemcpyToSymbol(tc::g_tc_error, &zero, sizeof(int));
-    // a kernel that gave up may have left arrivals behind
-    void* c = nullptr;
-    if (cudaGetSymbolAddress(&c, tc::g_tc_counters) == cudaSuccess) cudaMemset(c, 0, sizeof(tc::g_tc_counters));
   }
   return v;
 }

@@ -25,11 +25,10 @@
 //   4 epilogue warps  TMEM -> registers -> scale, bias, rounding -> C, while the next tile is computed
 //
 // Work is cut into (tile, k-range) segments.  Whole waves of tiles run one tile per CTA (pair); what
-// would be a ragged last wave is cut into equal k-ranges instead ("shared" tiles): each contributor
-// leaves an fp32 partial tile in the scratch, the last to arrive (atomic counter, no waiting) adds all
-// of them in k order, so results are bitwise reproducible.  With fewer tiles than SMs every tile is
-// shared by several workers and nothing is left to hide that addition behind (four warps of one CTA in
-// three: 80 of 107 us at M = 256, 4096 x 4096): tc_reduce_kernel does it on the whole GPU instead.
+// would be a ragged last wave (or the only one) is cut into equal k-ranges instead: the workers of such a
+// "shared" tile leave fp32 partial tiles in the scratch and tc_reduce_kernel adds them in k order on the
+// whole GPU.  (The last worker to arrive adding them in place was slower: four warps of one CTA in three
+// took 80 of 107 us at M = 256, 4096 x 4096.)
 //
 // Every wait is bounded: after kSpinLimit polls a role records a code in *p.error, stops, and the
 // kernel drains (TMEM is freed), so a broken hand-off can not hang the GPU.
@@ -92,10 +91,8 @@ struct TcParams {
   int tok_tiles;             // token tiles
   int workers;               // CTAs, or CTA pairs, of the grid
   int sk_tiles;              // the first tiles are shared out by k-range among all workers
-  int reduce_later;          // partial sums are added up by tc_reduce_kernel
   float chan_factor;         // of the channel-wise scales (fp8: takes the exponent re-bias out)
   float* partials;           // [worker][2][CG][tn][128] fp32
-  int32_t* counters;         // [worker][CG], zero between kernels; one byte per lane quadrant
   // mixture of experts: tiles come from a list in device memory {expert, first row, rows}; the rows of A
   // are in sorted order, output row = ids[row] (>= out_rows: padding), scaled by row_weights[id]
   const int4* tile_list;
@@ -104,6 +101,7 @@ struct TcParams {
   const float* row_weights;
   int out_rows;
   long long s_stride, bias_stride;  // per expert, elements
+  uint32_t zero;             // 0, for dependencies the compiler can not see through
 };
 
 // A: rows of A; B: packed weights; S: scales; Z: zero-points (the last two only where the format has them)
@@ -201,21 +199,24 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
-// D[tmem] (+)= A[smem] * B[smem], 16-bit inputs, fp32 accumulate
+// D[tmem] (+)= A[smem] * B[smem], 16-bit inputs, fp32 accumulate.  a / b: low words of the descriptors,
+// hi: their common high word.
 template <int CG>
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint32_t a, uint32_t b, uint32_t hi, uint32_t idesc,
                                          uint32_t accumulate) {
   if (CG == 2)
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %5, 0;\n\t"
+        "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, p;\n\t}\n" ::"r"(d_tmem),
+        "r"(a), "r"(b), "r"(hi), "r"(idesc), "r"(accumulate)
         : "memory");
   else
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %5, 0;\n\t"
+        "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}\n" ::"r"(d_tmem),
+        "r"(a), "r"(b), "r"(hi), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 // arrive on an mbarrier (CG == 2: the same one of both CTAs) when all MMAs issued so far have completed
@@ -260,10 +261,9 @@ __device__ __forceinline__ void sts32_off(uint32_t addr, uint32_t v) {
 }
 
 // Shared-memory matrix descriptor: K-major tile, 128-byte swizzle, rows 128 B apart, 8-row atoms 1024 B
-// apart (version 1 = sm_100 format).
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
-  return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
+// apart (version 1 = sm_100 format): low word (16-byte address, leading offset 1), high word.
+__device__ __forceinline__ uint32_t smem_desc_lo(uint32_t addr) { return ((addr & 0x3FFFFu) >> 4) | (1u << 16); }
+constexpr uint32_t kDescHi = 64u | (1u << 14) | (2u << 29);
 // instruction descriptor: fp32 accumulate, A and B K-major
 template <typename T>
 __device__ __forceinline__ uint32_t make_idesc(int m, int n) {
@@ -271,7 +271,7 @@ __device__ __forceinline__ uint32_t make_idesc(int m, int n) {
   return (1u << 4) | (f << 7) | (f << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-// Shared-memory plan.  TOK: token rows a CTA can stage per step (64 or 128).
+// Shared-memory plan.  TOK: token rows a CTA can stage per step.
 template <int F, int TOK>
 struct TcCfg {
   using I = FmtInfo<F>;
@@ -286,9 +286,12 @@ struct TcCfg {
   static constexpr int kTokBytes = TOK * 128;
   static constexpr int kABytes = kBN * 128;
   static constexpr int kSlot = 2 * (kTokBytes + kABytes);
-  static constexpr int kRing = TOK == 64 ? 3 : 2;
   static constexpr int kBarBytes = 1024;
-  static constexpr int kFit = (226 * 1024 - kBarBytes - 1024 - kRing * kSlot) / kWSlot;
+  static constexpr int kRoom = 226 * 1024 - kBarBytes - 1024;  // - alignment slack
+  // three slots where two slots of weights still fit: with two, the chain conversion -> MMAs -> next
+  // conversion of a slot (2540 cycles at 256 tokens) is longer than the MMAs of two rounds
+  static constexpr int kRing = 3 * kSlot + 2 * kWSlot <= kRoom ? 3 : 2;
+  static constexpr int kFit = (kRoom - kRing * kSlot) / kWSlot;
   static constexpr int kWD = kFit >= 8 ? 8 : kFit / 2 * 2;  // even: a slot always belongs to the same group
   static constexpr int kSmemBytes = kRing * kSlot + kWD * kWSlot + kBarBytes + 1024;  // + alignment slack
 };
@@ -310,8 +313,8 @@ struct Segment {
   int tok0, rows;    // first token row, valid rows
   int expert;
   int r0, r1;        // rounds
-  bool shared;       // other workers hold the rest of the tile's k-range
-  int first, contributors, slot;  // shared: first contributing worker, how many, this segment's slot
+  bool shared;       // a k-range of a shared tile
+  int slot;          // shared: where the partial sums go
 };
 
 // Which of `workers` equal shares of `units` holds `unit`.
@@ -347,7 +350,6 @@ struct Schedule {
       s.rows = min(p.tn, p.m - s.tok0);
     }
   }
-  __device__ __forceinline__ int owner(long long unit) const { return share_of(unit, p.workers, units); }
   __device__ __forceinline__ bool next(Segment& s) {
     if (u < u1) {
       const int t = (int)(u / rounds);
@@ -355,12 +357,8 @@ struct Schedule {
       s.r1 = (int)min((long long)rounds, s.r0 + (u1 - u));
       u += s.r1 - s.r0;
       place(s, t);
-      s.shared = s.r0 > 0 || s.r1 < rounds;
-      if (s.shared) {
-        s.first = owner((long long)t * rounds);
-        s.contributors = owner((long long)t * rounds + rounds - 1) - s.first + 1;
-        s.slot = 2 * worker + (s.r0 > 0 ? 0 : 1);
-      }
+      s.shared = true;
+      s.slot = 2 * worker + (s.r0 > 0 ? 0 : 1);
       return true;
     }
     if (tile < tiles) {
@@ -555,6 +553,8 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
       Ring<RING> ring;
       int seg_i = 0;
       bool ok = true;
+      // the ring stays below 256 KB: slot offsets add up in the address field of the descriptors
+      const uint32_t da0 = smem_desc_lo(a_slot(0)), db0 = smem_desc_lo(tok_slot(0));
       while (ok && sched.next(sg)) {
         const uint32_t idesc = make_idesc<T>(CG * 128, sched.template mma_n<CG>(sg));
         const int buf = seg_i & 1;
@@ -564,14 +564,14 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         for (int r = sg.r0; r < sg.r1; ++r) {
           if (!(ok = mbar_wait<kPair>(full(ring.i), ring.ph, (2 << 8) | 0, cta_abort, p.error))) break;
           tc_fence_after();
-          const uint64_t da = smem_desc_sw128(a_slot(ring.i)), db = smem_desc_sw128(tok_slot(ring.i));
+          const uint32_t da = da0 + ring.i * (Cfg::kSlot / 16), db = db0 + ring.i * (Cfg::kSlot / 16);
           if (elect_one()) {
 #pragma unroll
-            for (int k16 = 0; k16 < 4; ++k16) umma_f16<CG>(d, da + 2 * k16, db + 2 * k16, idesc, r > sg.r0 || k16 > 0);
+            for (int k16 = 0; k16 < 4; ++k16) umma_f16<CG>(d, da + 2 * k16, db + 2 * k16, kDescHi, idesc, k16 > 0 || r > sg.r0);
             if (2 * r + 1 < steps) {
 #pragma unroll
               for (int k16 = 0; k16 < 4; ++k16)
-                umma_f16<CG>(d, da + Cfg::kABytes / 16 + 2 * k16, db + Cfg::kTokBytes / 16 + 2 * k16, idesc, 1);
+                umma_f16<CG>(d, da + Cfg::kABytes / 16 + 2 * k16, db + Cfg::kTokBytes / 16 + 2 * k16, kDescHi, idesc, 1);
             }
             umma_commit<CG>(empty(ring.i));  // slot reusable once these MMAs have read it
             if (r + 1 == sg.r1) umma_commit<CG>(tmem_full(buf));
@@ -611,7 +611,7 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         if (!(ok = mbar_wait<false>(full_w(wr.i), wr.ph, (3 << 8) | 1, cta_abort, p.error))) break;
         // packed words of the lane, [sub] (4-bit) or [2 sub + block] (8-bit), scales and zero-points of the
         // two tiles
-        uint32_t w2[2][NW], sc2[2][4], zr2[2][4];
+        uint32_t w2[2][NW], sc2[2][4] = {}, zr2[2][4] = {};
 #pragma unroll
         for (int st = 0; st < 2; ++st) {
 #pragma unroll
@@ -644,86 +644,96 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
           }
         }
         if (!(ok = mbar_wait<kPair>(empty(ring.i), ring.ph ^ 1, (3 << 8) | 4, cta_abort, p.error))) break;
+        // The slot goes back as soon as its words are in registers.  A release does not wait for loads still
+        // in flight (seen: a slot refilled before it was read), so the arrival is made to depend on them.
+        uint32_t got = 0;
+#pragma unroll
+        for (int st = 0; st < 2; ++st) {
+#pragma unroll
+          for (int i = 0; i < NW; ++i) got |= w2[st][i];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) got |= sc2[st][i] | zr2[st][i];
+        }
         __syncwarp();
-        if (lane == 0) mbar_arrive(empty_w(wr.i));
+        if (lane == 0) mbar_arrive(empty_w(wr.i) + (got & p.zero));
         wr.next(2);
         if (live) {
           const uint32_t b_lo0 = smem_base + ring.i * Cfg::kSlot + b_lo_rel, b_hi0 = smem_base + ring.i * Cfg::kSlot + b_hi_rel;
 #pragma unroll
           for (int st = 0; st < 2; ++st) {
-          if (2 * r + st >= steps) break;  // the last round of an odd number of steps
-          const uint32_t b_lo = b_lo0 + st * Cfg::kABytes, b_hi = b_hi0 + st * Cfg::kABytes;
-          const uint32_t (&w)[NW] = w2[st];
-          const uint32_t (&sc)[4] = sc2[st];
-          const uint32_t (&zr)[4] = zr2[st];
-          auto convert = [&](auto sub_c, auto scaled_c) {
-            constexpr int sub = decltype(sub_c)::value;
-            uint32_t f[4];
-            codes_to_16bit<T, F>(w, sub, f);
-            if constexpr (I::kZp) {
-              // zero-points of columns c8 + 16 sub (low half) and + 8 (high half), exact integers in T
-              uint32_t zpair;
-              if constexpr (BITS == 4) {
-                uint32_t z4[4];
-                dequant4<T, false>(zr[0] >> (4 * sub), z4);  // nibbles sub and sub + 4
-                zpair = z4[0];
-              } else {
-                uint32_t z8[2];
-                dequant8<T, false>((sub & 2) ? zr[1] : zr[0], z8);  // word sub / 2, bytes (0, 2) or (1, 3)
-                zpair = (sub & 1) ? z8[1] : z8[0];
+            if (2 * r + st >= steps) break;  // the last round of an odd number of steps
+            const uint32_t b_lo = b_lo0 + st * Cfg::kABytes, b_hi = b_hi0 + st * Cfg::kABytes;
+            const uint32_t (&w)[NW] = w2[st];
+            const uint32_t (&sc)[4] = sc2[st];
+            const uint32_t (&zr)[4] = zr2[st];
+            auto convert = [&](auto sub_c, auto scaled_c) {
+              constexpr int sub = decltype(sub_c)::value;
+              uint32_t f[4];
+              codes_to_16bit<T, F>(w, sub, f);
+              if constexpr (I::kZp) {
+                // zero-points of columns c8 + 16 sub (low half) and + 8 (high half), exact integers in T
+                uint32_t zpair;
+                if constexpr (BITS == 4) {
+                  uint32_t z4[4];
+                  dequant4<T, false>(zr[0] >> (4 * sub), z4);  // nibbles sub and sub + 4
+                  zpair = z4[0];
+                } else {
+                  uint32_t z8[2];
+                  dequant8<T, false>((sub & 2) ? zr[1] : zr[0], z8);  // word sub / 2, bytes (0, 2) or (1, 3)
+                  zpair = (sub & 1) ? z8[1] : z8[0];
+                }
+                const uint32_t z_lo = dup_lo(zpair), z_hi = dup_hi(zpair);
+                f[0] = Pair<T>::sub(f[0], z_lo);
+                f[1] = Pair<T>::sub(f[1], z_lo);
+                f[2] = Pair<T>::sub(f[2], z_hi);
+                f[3] = Pair<T>::sub(f[3], z_hi);
               }
-              const uint32_t z_lo = dup_lo(zpair), z_hi = dup_hi(zpair);
-              f[0] = Pair<T>::sub(f[0], z_lo);
-              f[1] = Pair<T>::sub(f[1], z_lo);
-              f[2] = Pair<T>::sub(f[2], z_hi);
-              f[3] = Pair<T>::sub(f[3], z_hi);
-            }
-            if constexpr (decltype(scaled_c)::value) {
-              uint32_t s_lo, s_hi;
-              if constexpr (I::kFp4) {
-                // byte 4 (sub / 2) + 2 h + sub % 2 of the lane's eight belongs to column c8 + 16 sub + 8 h
-                s_lo = fp4_scale<T, F>(sc[sub >> 1], sub & 1);
-                s_hi = fp4_scale<T, F>(sc[sub >> 1], 2 + (sub & 1));
-              } else {
-                s_lo = dup_lo(sc[sub]);
-                s_hi = dup_hi(sc[sub]);
-              }
-              if constexpr (I::kZpF) {
-                // q * s - zp * s with the product zp * s rounded, one fma per pair (as gemm_lookup.cuh)
-                const uint32_t z_lo = Pair<T>::mul(dup_lo(zr[sub]), s_lo) ^ 0x80008000u;
-                const uint32_t z_hi = Pair<T>::mul(dup_hi(zr[sub]), s_hi) ^ 0x80008000u;
-                f[0] = Pair<T>::fma(f[0], s_lo, z_lo);
-                f[1] = Pair<T>::fma(f[1], s_lo, z_lo);
-                f[2] = Pair<T>::fma(f[2], s_hi, z_hi);
-                f[3] = Pair<T>::fma(f[3], s_hi, z_hi);
-              } else {
-                f[0] = Pair<T>::mul(f[0], s_lo);
-                f[1] = Pair<T>::mul(f[1], s_lo);
-                f[2] = Pair<T>::mul(f[2], s_hi);
-                f[3] = Pair<T>::mul(f[3], s_hi);
-              }
-            } else if constexpr (F == kF8) {
-              // true magnitude before the MMA (exact); the epilogue takes the factor out of the scale
+              if constexpr (decltype(scaled_c)::value) {
+                uint32_t s_lo, s_hi;
+                if constexpr (I::kFp4) {
+                  // byte 4 (sub / 2) + 2 h + sub % 2 of the lane's eight belongs to column c8 + 16 sub + 8 h
+                  s_lo = fp4_scale<T, F>(sc[sub >> 1], sub & 1);
+                  s_hi = fp4_scale<T, F>(sc[sub >> 1], 2 + (sub & 1));
+                } else {
+                  s_lo = dup_lo(sc[sub]);
+                  s_hi = dup_hi(sc[sub]);
+                }
+                if constexpr (I::kZpF) {
+                  // q * s - zp * s with the product zp * s rounded, one fma per pair (as gemm_lookup.cuh)
+                  const uint32_t z_lo = Pair<T>::mul(dup_lo(zr[sub]), s_lo) ^ 0x80008000u;
+                  const uint32_t z_hi = Pair<T>::mul(dup_hi(zr[sub]), s_hi) ^ 0x80008000u;
+                  f[0] = Pair<T>::fma(f[0], s_lo, z_lo);
+                  f[1] = Pair<T>::fma(f[1], s_lo, z_lo);
+                  f[2] = Pair<T>::fma(f[2], s_hi, z_hi);
+                  f[3] = Pair<T>::fma(f[3], s_hi, z_hi);
+                } else {
+                  f[0] = Pair<T>::mul(f[0], s_lo);
+                  f[1] = Pair<T>::mul(f[1], s_lo);
+                  f[2] = Pair<T>::mul(f[2], s_hi);
+                  f[3] = Pair<T>::mul(f[3], s_hi);
+                }
+              } else if constexpr (F == kF8) {
+                // true magnitude before the MMA (exact); the epilogue takes the factor out of the scale
 #pragma unroll
-              for (int i = 0; i < 4; ++i) f[i] = Pair<T>::mul(f[i], Fp8Cvt<T>::kRebias);
+                for (int i = 0; i < 4; ++i) f[i] = Pair<T>::mul(f[i], Fp8Cvt<T>::kRebias);
+              }
+              sts32_off<sub * 2048>(b_lo, f[0]);
+              sts32_off<sub * 2048>(b_hi, f[1]);
+              sts32_off<sub * 2048 + 1024>(b_lo, f[2]);
+              sts32_off<sub * 2048 + 1024>(b_hi, f[3]);
+            };
+            auto convert_all = [&](auto scaled_c) {
+              convert(std::integral_constant<int, 0>{}, scaled_c);
+              convert(std::integral_constant<int, 1>{}, scaled_c);
+              convert(std::integral_constant<int, 2>{}, scaled_c);
+              convert(std::integral_constant<int, 3>{}, scaled_c);
+            };
+            if constexpr (I::kFp4 || I::kZpF) {
+              convert_all(std::true_type{});
+            } else {
+              if (p.channelwise) convert_all(std::false_type{});
+              else convert_all(std::true_type{});
             }
-            sts32_off<sub * 2048>(b_lo, f[0]);
-            sts32_off<sub * 2048>(b_hi, f[1]);
-            sts32_off<sub * 2048 + 1024>(b_lo, f[2]);
-            sts32_off<sub * 2048 + 1024>(b_hi, f[3]);
-          };
-          auto convert_all = [&](auto scaled_c) {
-            convert(std::integral_constant<int, 0>{}, scaled_c);
-            convert(std::integral_constant<int, 1>{}, scaled_c);
-            convert(std::integral_constant<int, 2>{}, scaled_c);
-            convert(std::integral_constant<int, 3>{}, scaled_c);
-          };
-          if constexpr (I::kFp4 || I::kZpF) {
-            convert_all(std::true_type{});
-          } else {
-            if (p.channelwise) convert_all(std::false_type{});
-            else convert_all(std::true_type{});
-          }
           }
         }
         fence_proxy_async_smem();  // generic-proxy stores -> visible to the tensor core
@@ -830,10 +840,7 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
       } else {
         // partial sums, token-major: a warp writes 128 B per token
         const size_t slot_floats = (size_t)p.tn * kBN;
-        auto slot_ptr = [&](int slot) {
-          return p.partials + ((size_t)slot * CG + rank) * slot_floats + quad * 32 + lane;
-        };
-        float* mine = slot_ptr(sg.slot);
+        float* mine = p.partials + ((size_t)sg.slot * CG + rank) * slot_floats + quad * 32 + lane;
         for (int t0 = 0; t0 < sg.rows; t0 += 32) {
           uint32_t r[32];
           tmem_ld32(taddr + t0, r);
@@ -843,31 +850,6 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
             if (t0 + t < sg.rows) __stcg(mine + (size_t)(t0 + t) * kBN, __uint_as_float(r[t]));
         }
         release();
-        if (p.reduce_later) continue;
-        __threadfence();
-        __syncwarp();
-        // one byte of the counter per quadrant: every warp hands over its own quarter of the tile
-        int32_t* counter = p.counters + sg.first * CG + rank;
-        uint32_t seen = 0;
-        if (lane == 0) seen = (uint32_t)atomicAdd(counter, 1 << (8 * quad)) >> (8 * quad) & 0xffu;
-        seen = __shfl_sync(~0u, seen, 0);
-        if ((int)seen == sg.contributors - 1) {
-          if (lane == 0) atomicSub(counter, sg.contributors << (8 * quad));
-          __threadfence();
-          for (int t0 = 0; t0 < sg.rows; t0 += 32) {
-            float v[32];
-#pragma unroll
-            for (int t = 0; t < 32; ++t) v[t] = 0.f;
-            for (int i = 0; i < sg.contributors; ++i) {
-              // the first contributor's piece begins the tile (slot 1 of its worker)
-              const float* src = slot_ptr(2 * (sg.first + i) + (i == 0 ? 1 : 0));
-#pragma unroll
-              for (int t = 0; t < 32; ++t)
-                if (t0 + t < sg.rows) v[t] += __ldcg(src + (size_t)(t0 + t) * kBN);
-            }
-            if (n_ok) store32(t0, v);
-          }
-        }
       }
     }
   }

@@ -59,7 +59,9 @@ int launch_format(const TcMaps& maps, const TcParams& p, int cg, bool pdl, cudaS
 #define B200Q_TC_FORMAT(F)                                                                                  \
   template <>                                                                                               \
   int launch_format<InstT, F>(const TcMaps& maps, const TcParams& p, int cg, bool pdl, cudaStream_t stream) { \
-    if (cg == 2) return launch_one<InstT, F, 2, 128>(maps, p, pdl, stream);                                 \
+    if (cg == 2)                                                                                            \
+      return p.box <= 96 ? launch_one<InstT, F, 2, 96>(maps, p, pdl, stream)                                \
+                         : launch_one<InstT, F, 2, 128>(maps, p, pdl, stream);                              \
     return p.box <= 64 ? launch_one<InstT, F, 1, 64>(maps, p, pdl, stream)                                  \
                        : launch_one<InstT, F, 1, 128>(maps, p, pdl, stream);                                \
   }
