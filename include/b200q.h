@@ -229,6 +229,43 @@ int b200q_moe_wna16_marlin_gemm(
     int64_t size_k, int64_t num_groups, b200q_stream_t stream);
 
 /*
+ * Sorting step of the mixture-of-experts form (fused_moe/moe_align_block_size.py:13-86): the numel ids of
+ * topk_ids (int32, or int64 with ids64) grouped by expert, stable, every expert's run padded to a multiple
+ * of block_size.  sorted_token_ids [sorted_len >= numel + num_experts * (block_size - 1)], padded with
+ * numel; expert_ids [num_blocks >= sorted_len / block_size rounded up], mapped through expert_map
+ * [num_experts] (null: identity), blocks past the end those of expert 0; num_tokens_post_padded: one value.
+ */
+int b200q_moe_align_block_size(const void* topk_ids, int ids64, const int32_t* expert_map,
+                               int64_t numel, int64_t block_size, int64_t num_experts,
+                               int32_t* sorted_token_ids, int64_t sorted_len, int32_t* expert_ids,
+                               int64_t num_blocks, int32_t* num_tokens_post_padded,
+                               b200q_stream_t stream);
+
+/*
+ * One mixture-of-experts layer (fused_marlin_moe.py:186-340): sort, gate_up GEMM, silu(gate) * up, down
+ * GEMM, sum over a token's experts.
+ *   hidden        [size_m, size_k] 16-bit, row stride lda; out [size_m, size_k]
+ *   w1, w2        [num_experts] of Marlin layout: size_k -> 2 size_n and size_n -> size_k; scales, zeros and
+ *                 biases as for b200q_moe_wna16_marlin_gemm, groups1 / groups2 scale groups
+ *   topk_weights  fp32 [size_m, top_k]; topk_ids int32 / int64 [size_m, top_k], global expert numbers
+ *   expert_map    [global_experts] -> expert of this rank or -1 (those slots add nothing), or null
+ *   weight_on_input  the router weight scales the first GEMM's output instead of the second's
+ *   scratch       b200q_fused_marlin_moe_scratch_bytes(), aligned to 256 bytes
+ * size_k % 64 == 0, size_n % 32 == 0; integer weight types.
+ */
+size_t b200q_fused_marlin_moe_scratch_bytes(int64_t size_m, int64_t top_k, int64_t num_experts,
+                                            int64_t global_experts, int64_t size_k, int64_t size_n,
+                                            int bits);
+int b200q_fused_marlin_moe(
+    const void* hidden, int64_t lda, const uint32_t* w1, const uint32_t* w2, const void* w1_scale,
+    const void* w2_scale, const uint32_t* w1_zeros, const uint32_t* w2_zeros, const void* bias1,
+    const void* bias2, const float* topk_weights, const void* topk_ids, int ids64,
+    const int32_t* expert_map, void* out, void* scratch, size_t scratch_bytes, int64_t b_q_type_id,
+    int a_dtype, int64_t size_m, int64_t top_k, int64_t size_k, int64_t size_n, int64_t num_experts,
+    int64_t global_experts, int64_t groups1, int64_t groups2, int weight_on_input,
+    b200q_stream_t stream);
+
+/*
  * b200q_marlin_gemm followed by the SUM all-reduce of C over the same peer link, as
  * RowParallelLinear does (vllm/model_executor/layers/linear.py:1386-1411: the
  * quantized matmul of the K shard, then tensor_model_parallel_all_reduce).  Where one

@@ -154,3 +154,65 @@ def test_moe_error_messages():
     with pytest.raises(RuntimeError, match="actual_size_n"):
         ops.moe_wna16_marlin_gemm(a, None, q, None, s, None, None, None, None, ws, ids, ex, num, tw, 16, 1,
                                   False, False, scalar_types.uint4b8, M, 2 * N, K)
+
+
+@pytest.mark.parametrize("numel,E,block,idtype", [(1, 1, 8, "int32"), (32, 8, 8, "int32"), (1000, 8, 32, "int64"),
+                                                  (33, 64, 16, "int32"), (5000, 257, 64, "int32"), (65536, 16, 48, "int64")])
+@pytest.mark.parametrize("mapped", [False, True])
+def test_moe_align_kernel(numel, E, block, idtype, mapped):
+    """The kernel gives what the torch formulation (run on the CPU copy) gives, order included."""
+    import torch
+    from vllm_b200 import fused_moe
+    gen = torch.Generator().manual_seed(numel)
+    ids = torch.randint(0, E, (numel, 1), generator=gen).to(getattr(torch, idtype))
+    emap = torch.where(torch.arange(E) % 3 == 1, -1, torch.arange(E) // 2).to(torch.int32) if mapped else None
+    want = fused_moe.moe_align_block_size(ids, block, E, emap)
+    got = fused_moe.moe_align_block_size(ids.cuda(), block, E, None if emap is None else emap.cuda())
+    n = int(want[2])
+    assert int(got[2]) == n
+    assert torch.equal(got[0].cpu()[:n], want[0][:n]) and torch.equal(got[1].cpu(), want[1])
+
+
+@pytest.mark.parametrize("M,E,topk,qtype,dtype,expert_parallel,on_input", [
+    (1, 8, 2, "uint8b128", "bfloat16", False, False),      # tensor-core kernel, one row per expert
+    (70, 2, 2, "uint4", "float16", False, False),          # runs longer than a tile of single CTAs
+    (150, 3, 2, "uint4b8", "bfloat16", True, False),       # CTA pairs, experts of another rank
+    (513, 2, 1, "uint8", "float16", False, True),          # runs split over several tiles, weight on the input
+    (3, 16, 4, "uint4b8", "bfloat16", True, True),         # decode kernel
+])
+def test_fused_marlin_moe_kernels(M, E, topk, qtype, dtype, expert_parallel, on_input):
+    import torch
+    from vllm_b200 import _lib, fused_moe
+    from vllm_b200.scalar_type import scalar_types
+    K, N = 320, 192
+    rng = np.random.default_rng(M + E)
+    local = [e for e in range(E) if not expert_parallel or e % 2 == 0]
+    w1 = _experts(len(local), K, 2 * N, qtype, 64, dtype, with_bias=True, seed=1)
+    w2 = _experts(len(local), N, K, qtype, -1, dtype, seed=2)
+    a = 0.1 * H.make_activations(M, K, dtype)
+    a = mo.round_to_dtype(a, dtype)
+    topk_ids = np.stack([rng.permutation(E)[:topk] for _ in range(M)]).astype(np.int64)
+    tw = rng.uniform(0.1, 1.0, size=(M, topk)).astype(np.float32)
+    dev = torch.device("cuda")
+    q1, s1, z1, b1 = _stack(torch, w1, dtype)
+    q2, s2, z2, _ = _stack(torch, w2, dtype)
+    emap = np.full(E, -1, dtype=np.int32)
+    emap[local] = np.arange(len(local))
+    out = fused_moe.fused_marlin_moe(
+        G.t16(a, dtype), q1, q2, s1, s2, torch.from_numpy(tw).to(dev), torch.from_numpy(topk_ids).to(dev),
+        getattr(scalar_types, qtype), bias1=b1, w1_zeros=z1, w2_zeros=z2, global_num_experts=E,
+        expert_map=torch.from_numpy(emap).to(dev) if expert_parallel else None, apply_router_weight_on_input=on_input)
+    torch.cuda.synchronize()
+    assert _lib.load().b200q_device_error(1) == 0
+    ref = np.zeros((M, K), dtype=np.float32)
+    for t in range(M):
+        for j in range(topk):
+            e = int(emap[topk_ids[t, j]])
+            if e < 0:
+                continue
+            h = a[t].astype(np.float32) @ w1[e].w.astype(np.float32) + w1[e].bias
+            h = mo.round_to_dtype(h * (tw[t, j] if on_input else 1), dtype)
+            act = mo.round_to_dtype(h[:N] / (1.0 + np.exp(-h[:N])) * h[N:], dtype)
+            ref[t] += mo.round_to_dtype((act @ w2[e].w.astype(np.float32)) * (1 if on_input else tw[t, j]), dtype)
+    mf, mr = H.gemm_errors(G.n16(out), ref)
+    assert mf <= 3e-2 and mr <= 1.5e-2, (mf, mr)

@@ -160,6 +160,20 @@ def _moe_wna16_marlin_gemm_fake(a, c_or_none, b_q_weight, b_bias_or_none, b_scal
     return torch.empty((size_m * top_k, size_n), dtype=a.dtype, device=a.device)
 
 
+@torch.library.register_fake(f"{_MOE_NS}::b200q_moe_align_block_size")
+def _moe_align_block_size_fake(topk_ids, block_size, num_experts, expert_map):
+    padded = topk_ids.numel() + num_experts * (block_size - 1)
+    new = lambda n: torch.empty((n,), dtype=torch.int32, device=topk_ids.device)
+    return new(padded), new((padded + block_size - 1) // block_size), new(1)
+
+
+@torch.library.register_fake(f"{_MOE_NS}::b200q_fused_marlin_moe")
+def _fused_marlin_moe_fake(hidden_states, w1, w2, w1_scale, w2_scale, topk_weights, topk_ids, bias1, bias2,
+                           w1_zeros, w2_zeros, b_q_type_id, global_num_experts, expert_map,
+                           apply_router_weight_on_input):
+    return torch.empty(hidden_states.shape, dtype=hidden_states.dtype, device=hidden_states.device)
+
+
 _ops = getattr(torch.ops, _NS)
 _moe_ops = getattr(torch.ops, _MOE_NS)
 
@@ -240,6 +254,21 @@ def moe_wna16_marlin_gemm(input: torch.Tensor, output: torch.Tensor | None, b_qw
         sorted_token_ids, expert_ids, num_tokens_past_padded, topk_weights, moe_block_size, top_k,
         mul_topk_weights, is_ep, b_q_type.id, size_m, size_n, size_k, is_k_full, use_atomic_add,
         use_fp32_reduce, is_zp_float)
+
+
+def moe_align_block_size(topk_ids: torch.Tensor, block_size: int, num_experts: int,
+                         expert_map: torch.Tensor | None):
+    return _moe_ops.b200q_moe_align_block_size(topk_ids, block_size, num_experts, expert_map)
+
+
+def fused_marlin_moe(hidden_states: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, w1_scale: torch.Tensor,
+                     w2_scale: torch.Tensor, topk_weights: torch.Tensor, topk_ids: torch.Tensor,
+                     bias1: torch.Tensor | None, bias2: torch.Tensor | None, w1_zeros: torch.Tensor | None,
+                     w2_zeros: torch.Tensor | None, quant_type: ScalarType, global_num_experts: int,
+                     expert_map: torch.Tensor | None, apply_router_weight_on_input: bool) -> torch.Tensor:
+    return _moe_ops.b200q_fused_marlin_moe(hidden_states, w1, w2, w1_scale, w2_scale, topk_weights, topk_ids,
+                                           bias1, bias2, w1_zeros, w2_zeros, quant_type.id, global_num_experts,
+                                           expert_map, apply_router_weight_on_input)
 
 
 def _dtype_code(t: torch.Tensor) -> int:

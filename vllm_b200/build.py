@@ -41,7 +41,7 @@ def _units():
         for f0, f1 in pairs:
             units.append(("gemm_tc_inst.cu", f"gemm_tc_{'bf16' if bf16 else 'f16'}_{f0}{f1}.o",
                           [f"-DINST_BF16={bf16}", f"-DINST_F0={f0}", f"-DINST_F1={f1}"]))
-    for extra in ("gemm_tc.cu", "noalloc.cu", "allreduce.cu", "elementwise.cu"):
+    for extra in ("gemm_tc.cu", "moe.cu", "noalloc.cu", "allreduce.cu", "elementwise.cu"):
         units.append((extra, extra.replace(".cu", ".o"), []))
     return units
 

@@ -274,6 +274,34 @@ int launch_tc_gemm(const void* a, int64_t lda, const uint32_t* b, const void* sc
                               : tc::launch_reduce<__nv_bfloat16>(p, plan.cg, stream);
 }
 
+// Mixture of experts: rows of A in sorted order, tiles {expert, first row, rows} in device memory, written by
+// a kernel in front.  `box`: token rows a CTA stages; a tile has at most that many rows (pairs: twice).
+int launch_tc_moe(const void* a, int64_t rows, const uint32_t* b, const void* scales, const uint32_t* zeros,
+                  const void* bias, void* c, int a_dtype, int fmt, int64_t experts, int64_t size_n, int64_t size_k,
+                  int64_t num_groups, int pairs, int box, const int4* tile_list, const int32_t* tile_count,
+                  const int32_t* ids, int scatter, const float* row_weights, cudaStream_t stream) {
+  tc::TcParams p = {};
+  int rc = tc::error_word(&p.error);
+  if (rc != B200Q_OK) return rc;
+  B200Q_REQUIRE(size_k % num_groups == 0 && (size_k / num_groups) % 16 == 0, B200Q_EINVAL,
+                "size_k = %lld does not split into %lld groups", (long long)size_k, (long long)num_groups);
+  tc::TcMaps maps = {};
+  p.group_blocks = (int)(size_k / num_groups / 16); p.channelwise = num_groups == 1;
+  rc = tc::make_a_map(&maps.a, a, size_k, rows, size_k, box, a_dtype);
+  if (rc == B200Q_OK) rc = tc::make_weight_maps(&maps, &p, b, scales, zeros, fmt, size_n, size_k, experts);
+  if (rc != B200Q_OK) return rc;
+  const int cg = pairs ? 2 : 1;
+  p.scales = scales; p.bias = bias; p.c = c; p.chan_factor = 1.f;
+  p.m = (int)rows; p.n = (int)size_n; p.k = (int)size_k;
+  p.tn = box * cg; p.box = box; p.tok_tiles = 1; p.workers = device_sm_count() / cg;
+  p.tile_list = tile_list; p.tile_count = tile_count;
+  p.ids = row_weights || scatter ? ids : nullptr; p.scatter = scatter; p.row_weights = row_weights; p.out_rows = (int)rows;
+  p.s_stride = num_groups * size_n; p.bias_stride = size_n;
+  const bool pdl = pdl_enabled();
+  return a_dtype == B200Q_F16 ? tc::launch_type<half>(maps, p, fmt, cg, pdl, stream)
+                              : tc::launch_type<__nv_bfloat16>(maps, p, fmt, cg, pdl, stream);
+}
+
 // Scratch the tensor-core kernel would like for this problem (fp32 partials of shared tiles).
 int64_t tc_gemm_scratch_bytes(int64_t size_m, int64_t size_n, int64_t size_k) {
   if (size_k % tc::kBK != 0 || size_n % 64 != 0) return 0;

@@ -94,10 +94,11 @@ struct TcParams {
   float chan_factor;         // of the channel-wise scales (fp8: takes the exponent re-bias out)
   float* partials;           // [worker][2][CG][tn][128] fp32
   // mixture of experts: tiles come from a list in device memory {expert, first row, rows}; the rows of A
-  // are in sorted order, output row = ids[row] (>= out_rows: padding), scaled by row_weights[id]
+  // are in sorted order, output row = ids[row] (scatter) or row, scaled by row_weights[ids[row]]
   const int4* tile_list;
   const int32_t* tile_count;
   const int32_t* ids;
+  int scatter;               // 0: output rows stay in sorted order
   const float* row_weights;
   int out_rows;
   long long s_stride, bias_stride;  // per expert, elements
@@ -796,7 +797,7 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
           word[t / 2] = odd ? __byte_perm(theirs, mine, 0x7632) : __byte_perm(mine, theirs, 0x5410);
         }
         const int t1 = t0 + (odd ? 1 : 0);
-        if (!p.ids) {
+        if (!p.scatter) {
           uint16_t* dst = C + (size_t)(sg.tok0 + t1) * p.n + (n & ~1);
           const size_t step2 = (size_t)2 * p.n;
           if (t0 + 32 <= sg.rows) {

@@ -491,6 +491,101 @@ at::Tensor moe_wna16_marlin_gemm(
   return c;
 }
 
+// fused_moe/moe_align_block_size.py:13-86
+std::tuple<at::Tensor, at::Tensor, at::Tensor> moe_align_block_size(const at::Tensor& topk_ids, int64_t block_size,
+                                                                    int64_t num_experts,
+                                                                    const std::optional<at::Tensor>& expert_map) {
+  TORCH_CHECK(topk_ids.is_cuda() && topk_ids.is_contiguous() &&
+                  (topk_ids.scalar_type() == at::kInt || topk_ids.scalar_type() == at::kLong),
+              "topk_ids must be a contiguous int32 / int64 CUDA tensor");
+  if (expert_map.has_value())
+    TORCH_CHECK(expert_map->is_cuda() && expert_map->is_contiguous() && expert_map->scalar_type() == at::kInt &&
+                    expert_map->numel() >= num_experts,
+                "expert_map must be a contiguous int32 CUDA tensor with an entry per expert");
+  const c10::cuda::OptionalCUDAGuard guard(device_of(topk_ids));
+  const int64_t numel = topk_ids.numel(), len = numel + num_experts * (block_size - 1);
+  const int64_t blocks = (len + block_size - 1) / block_size;
+  const auto opts = topk_ids.options().dtype(at::kInt);
+  at::Tensor sorted = at::empty({len}, opts), experts = at::empty({blocks}, opts), total = at::empty({1}, opts);
+  B200Q_TORCH_OK(b200q_moe_align_block_size(topk_ids.data_ptr(), topk_ids.scalar_type() == at::kLong,
+                                            expert_map.has_value() ? expert_map->data_ptr<int32_t>() : nullptr, numel,
+                                            block_size, num_experts, sorted.data_ptr<int32_t>(), len,
+                                            experts.data_ptr<int32_t>(), blocks, total.data_ptr<int32_t>(),
+                                            at::cuda::getCurrentCUDAStream(topk_ids.get_device())),
+                 "moe_align_block_size");
+  return {sorted, experts, total};
+}
+
+// fused_moe/fused_marlin_moe.py:186-340: all steps of the layer in one call
+at::Tensor fused_marlin_moe(const at::Tensor& hidden, const at::Tensor& w1, const at::Tensor& w2,
+                            const at::Tensor& w1_scale, const at::Tensor& w2_scale, const at::Tensor& topk_weights,
+                            const at::Tensor& topk_ids, const std::optional<at::Tensor>& bias1,
+                            const std::optional<at::Tensor>& bias2, const std::optional<at::Tensor>& w1_zeros,
+                            const std::optional<at::Tensor>& w2_zeros, int64_t b_q_type_id,
+                            int64_t global_num_experts, const std::optional<at::Tensor>& expert_map,
+                            bool apply_router_weight_on_input) {
+  TypeInfo qt;
+  TORCH_CHECK(decode_type(b_q_type_id, &qt) && !qt.is_float,
+              "moe_wna16_marlin_gemm: b_q_type must be uint4b8, uint8b128, uint4 or uint8; id ", b_q_type_id,
+              " is not supported");
+  const int64_t pf = 32 / qt.bits;
+  TORCH_CHECK(hidden.is_cuda() && hidden.dim() == 2 && hidden.stride(1) == 1 && hidden.stride(0) % 8 == 0 &&
+                  (hidden.scalar_type() == at::kHalf || hidden.scalar_type() == at::kBFloat16),
+              "hidden_states must be a 16-bit CUDA matrix with unit inner stride and a row stride divisible by 8");
+  const int64_t m = hidden.size(0), k = hidden.size(1);
+  TORCH_CHECK(w1.dim() == 3 && w2.dim() == 3 && w1.size(0) == w2.size(0), "w1 and w2 must hold the same experts");
+  const int64_t e = w1.size(0), n = w2.size(1) * 16, top_k = topk_ids.size(-1);
+  TORCH_CHECK(w1.size(1) * 16 == k && w1.size(2) / 16 * pf == 2 * n && w2.size(2) / 16 * pf == k,
+              "Shape mismatch: w1 = ", w1.sizes(), ", w2 = ", w2.sizes(), ", hidden = ", hidden.sizes());
+  TORCH_CHECK(topk_weights.is_cuda() && topk_weights.is_contiguous() && topk_weights.scalar_type() == at::kFloat &&
+                  topk_weights.numel() == m * top_k && topk_ids.numel() == m * top_k && topk_ids.is_cuda() &&
+                  topk_ids.is_contiguous() && (topk_ids.scalar_type() == at::kInt || topk_ids.scalar_type() == at::kLong),
+              "topk_weights (float32) and topk_ids (int32 / int64) must be contiguous [tokens, top_k] CUDA tensors");
+  struct { const void* scales; const uint32_t* zeros; const void* bias; int64_t groups; } mat[2];
+  for (int i = 0; i < 2; ++i) {
+    const at::Tensor &w = i ? w2 : w1, &s = i ? w2_scale : w1_scale;
+    const std::optional<at::Tensor>&z = i ? w2_zeros : w1_zeros, &b = i ? bias2 : bias1;
+    const int64_t cols = i ? k : 2 * n;
+    TORCH_CHECK(w.is_cuda() && w.is_contiguous() && w.scalar_type() == at::kInt, "expert weights must be contiguous int32");
+    TORCH_CHECK(s.is_cuda() && s.is_contiguous() && s.dim() == 3 && s.size(0) == e && s.size(2) == cols &&
+                    s.scalar_type() == hidden.scalar_type(),
+                "expert scales must be [experts, groups, columns] of the dtype of the activations");
+    mat[i] = {s.data_ptr(), nullptr, nullptr, s.size(1)};
+    if (z.has_value() && z->size(-1) > 0) {
+      TORCH_CHECK(z->is_cuda() && z->is_contiguous() && z->scalar_type() == at::kInt &&
+                      z->numel() == e * s.size(1) * cols / pf,
+                  "expert zero-points must be int32 [experts, groups, columns / pack_factor]");
+      mat[i].zeros = static_cast<const uint32_t*>(z->data_ptr());
+    }
+    if (b.has_value()) {
+      TORCH_CHECK(b->is_cuda() && b->is_contiguous() && b->numel() == e * cols && b->scalar_type() == hidden.scalar_type(),
+                  "expert biases must be [experts, columns] of the dtype of the activations");
+      mat[i].bias = b->data_ptr();
+    }
+  }
+  if (expert_map.has_value())
+    TORCH_CHECK(expert_map->is_cuda() && expert_map->is_contiguous() && expert_map->scalar_type() == at::kInt &&
+                    expert_map->numel() >= global_num_experts,
+                "expert_map must be a contiguous int32 CUDA tensor with an entry per expert");
+  const c10::cuda::OptionalCUDAGuard guard(device_of(hidden));
+  at::Tensor out = at::empty({m, k}, hidden.options());
+  if (m == 0) return out;
+  const size_t bytes = b200q_fused_marlin_moe_scratch_bytes(m, top_k, e, global_num_experts, k, n, qt.bits);
+  at::Tensor scratch = at::empty({(int64_t)bytes}, hidden.options().dtype(at::kByte));
+  B200Q_TORCH_OK(
+      b200q_fused_marlin_moe(
+          hidden.data_ptr(), hidden.stride(0), static_cast<const uint32_t*>(w1.data_ptr()),
+          static_cast<const uint32_t*>(w2.data_ptr()), mat[0].scales, mat[1].scales, mat[0].zeros, mat[1].zeros,
+          mat[0].bias, mat[1].bias, topk_weights.data_ptr<float>(), topk_ids.data_ptr(),
+          topk_ids.scalar_type() == at::kLong, expert_map.has_value() ? expert_map->data_ptr<int32_t>() : nullptr,
+          out.data_ptr(), scratch.data_ptr(), bytes, b_q_type_id,
+          hidden.scalar_type() == at::kBFloat16 ? B200Q_BF16 : B200Q_F16, m, top_k, k, n, e, global_num_experts,
+          mat[0].groups, mat[1].groups, apply_router_weight_on_input ? 1 : 0,
+          at::cuda::getCurrentCUDAStream(hidden.get_device())),
+      "fused_marlin_moe");
+  return out;
+}
+
 std::unique_ptr<torch::Library> g_moe_defs, g_moe_impls;
 
 extern "C" int b200q_torch_register(const char* ns) {
@@ -559,9 +654,19 @@ extern "C" int b200q_torch_register_moe(const char* ns) {
         "int size_m, int size_n, int size_k,"
         "bool is_full_k, bool use_atomic_add,"
         "bool use_fp32_reduce, bool is_zp_float) -> Tensor");
+    // no counterparts in the reference's extension (its Python does these steps one by one)
+    g_moe_defs->def(
+        "b200q_moe_align_block_size(Tensor topk_ids, int block_size, int num_experts, Tensor? expert_map) -> "
+        "(Tensor, Tensor, Tensor)");
+    g_moe_defs->def(
+        "b200q_fused_marlin_moe(Tensor hidden_states, Tensor w1, Tensor w2, Tensor w1_scale, Tensor w2_scale, "
+        "Tensor topk_weights, Tensor topk_ids, Tensor? bias1, Tensor? bias2, Tensor? w1_zeros, Tensor? w2_zeros, "
+        "int b_q_type_id, int global_num_experts, Tensor? expert_map, bool apply_router_weight_on_input) -> Tensor");
     g_moe_impls = std::make_unique<torch::Library>(torch::Library::IMPL, name,
                                                    c10::DispatchKey::CUDA, __FILE__, __LINE__);
     g_moe_impls->impl("moe_wna16_marlin_gemm", &moe_wna16_marlin_gemm);
+    g_moe_impls->impl("b200q_moe_align_block_size", &moe_align_block_size);
+    g_moe_impls->impl("b200q_fused_marlin_moe", &fused_marlin_moe);
   } catch (const std::exception&) {
     g_moe_impls.reset();
     g_moe_defs.reset();

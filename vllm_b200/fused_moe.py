@@ -1,23 +1,28 @@
 """Mixture-of-experts layer over the Marlin GEMM, mirroring
 vllm/model_executor/layers/fused_moe/fused_marlin_moe.py and moe_align_block_size.py: tokens are
-sorted by expert into blocks, two grouped GEMMs (gate_up, then down with the router weights) run
-over the blocks, and the top-k outputs of a token are summed."""
+sorted by expert, two grouped GEMMs (gate_up, then down with the router weights) run over the
+sorted rows, and the top-k outputs of a token are summed; all steps are one native call."""
 from __future__ import annotations
 
 import torch
 
 from . import _custom_ops as ops
-from .marlin_utils import marlin_make_workspace_new
 from .scalar_type import ScalarType, scalar_types
+
+
+def _int32(expert_map: torch.Tensor | None) -> torch.Tensor | None:
+    return None if expert_map is None else expert_map.to(torch.int32).contiguous()
 
 
 def moe_align_block_size(topk_ids: torch.Tensor, block_size: int, num_experts: int,
                          expert_map: torch.Tensor | None = None):
     """Sort the (token, slot) pairs by expert and pad every expert's run to a multiple of
-    block_size (fused_moe/moe_align_block_size.py:13-86; the reference does this in a CUDA op,
-    here it is a handful of torch ops on the device: no host synchronisation).
+    block_size (fused_moe/moe_align_block_size.py:13-86): one kernel on the GPU, torch ops on a CPU tensor.
     Returns (sorted_token_ids [numel + E (block_size - 1)] padded with numel, expert_ids per block,
     num_tokens_post_padded [1])."""
+    if topk_ids.is_cuda:
+        ids = topk_ids if topk_ids.dtype in (torch.int32, torch.int64) else topk_ids.to(torch.int64)
+        return ops.moe_align_block_size(ids.contiguous(), block_size, num_experts, _int32(expert_map))
     numel = topk_ids.numel()
     dev = topk_ids.device
     max_padded = numel + num_experts * (block_size - 1)
@@ -60,29 +65,9 @@ def fused_marlin_moe(hidden_states: torch.Tensor, w1: torch.Tensor, w2: torch.Te
     N = w2.size(1) * 16
     assert w1.size(2) // 16 * pf == 2 * N and w2.size(2) // 16 * pf == K
     assert topk_weights.dtype == torch.float32
-    # the reference walks 8, 16, 32, 48, 64 (fused_marlin_moe.py:286-288); here blocks of up to 32
-    # ids run the decode kernel, which is faster than the 48 / 64 path even when an expert's
-    # weights are then read twice
-    for block_size_m in (8, 16, 32):
-        if M * topk / E / block_size_m < 0.9:
-            break
     if global_num_experts == -1:
         global_num_experts = E
-    sorted_ids, expert_ids, num_post_padded = moe_align_block_size(topk_ids, block_size_m,
-                                                                   global_num_experts, expert_map)
-    if workspace is None:
-        workspace = marlin_make_workspace_new(hidden_states.device)
-    tw = topk_weights.reshape(-1).contiguous()
-    cache1 = ops.moe_wna16_marlin_gemm(
-        hidden_states, None, w1, bias1, w1_scale, None, w1_zeros, None, None, workspace, sorted_ids,
-        expert_ids, num_post_padded, tw, block_size_m, topk, apply_router_weight_on_input,
-        expert_map is not None, quant_type, M, 2 * N, K)
-    cache2 = torch.empty((M * topk, N), dtype=hidden_states.dtype, device=hidden_states.device)
-    ops.silu_and_mul(cache2, cache1)
-    out = torch.zeros((M * topk, K), dtype=hidden_states.dtype, device=hidden_states.device) \
-        if expert_map is not None else None
-    out = ops.moe_wna16_marlin_gemm(
-        cache2, out, w2, bias2, w2_scale, None, w2_zeros, None, None, workspace, sorted_ids,
-        expert_ids, num_post_padded, tw, block_size_m, 1, not apply_router_weight_on_input,
-        expert_map is not None, quant_type, M * topk, K, N)
-    return out.view(M, topk, K).sum(dim=1)
+    ids = topk_ids if topk_ids.dtype in (torch.int32, torch.int64) else topk_ids.to(torch.int64)
+    return ops.fused_marlin_moe(hidden_states, w1, w2, w1_scale, w2_scale, topk_weights.contiguous(), ids.contiguous(),
+                                bias1, bias2, w1_zeros, w2_zeros, quant_type, global_num_experts, _int32(expert_map),
+                                apply_router_weight_on_input)
