@@ -54,7 +54,7 @@ def _pick_moe_namespace() -> str:
 _MOE_NS = _pick_moe_namespace()
 
 
-def _load_torch_extension(ns: str) -> None:
+def _load_torch_extension(ns: str):
     path = os.path.join(os.path.dirname(_lib.LIB_PATH), "b200q_torch.so")
     if not os.path.exists(path):
         raise _lib.B200QError(
@@ -72,9 +72,16 @@ def _load_torch_extension(ns: str) -> None:
                               "set VLLM_B200_OPS_NAMESPACE to a free namespace")
     if ext.b200q_torch_register_moe(_MOE_NS.encode()) != 0:
         raise _lib.B200QError(f"torch.ops.{_MOE_NS}.moe_wna16_marlin_gemm is taken by another extension")
+    make = ctypes.PyDLL(path).b200q_torch_python_module
+    make.restype = ctypes.py_object
+    return make()
 
 
-_load_torch_extension(_NS)
+# the GEMM operator callable without the dispatcher (see py_linear in csrc/torch_bindings.cpp)
+_direct = _load_torch_extension(_NS)
+_linear = _direct.linear
+_is_compiling = torch.compiler.is_compiling
+K_FULL, ZP_FLOAT = 1, 2     # flags of linear()
 
 
 def ops_namespace() -> str:
@@ -231,9 +238,31 @@ def gptq_marlin_gemm(a: torch.Tensor, c: torch.Tensor | None, b_q_weight: torch.
             b_q_type.id, size_m, size_n, size_k, is_k_full, use_atomic_add, use_fp32_reduce,
             is_zp_float, reduce_link.peer_ptrs, reduce_link.state, reduce_link.rank,
             reduce_link.world_size, reduce_link.max_size)
+    if c is None and not _is_compiling():
+        out = _linear(a, b_q_weight, b_bias, b_scales, global_scale, b_zeros, g_idx, perm, workspace, b_q_type.id,
+                      size_m, size_n, size_k, (K_FULL if is_k_full else 0) | (ZP_FLOAT if is_zp_float else 0))
+        if out is not None:
+            return out
     return _ops.gptq_marlin_gemm(a, c, b_q_weight, b_bias, b_scales, global_scale, b_zeros, g_idx,
                                  perm, workspace, b_q_type.id, size_m, size_n, size_k, is_k_full,
                                  use_atomic_add, use_fp32_reduce, is_zp_float)
+
+
+def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None, scales: torch.Tensor,
+           global_scale: torch.Tensor | None, zeros: torch.Tensor | None, g_idx: torch.Tensor | None,
+           perm: torch.Tensor | None, workspace: torch.Tensor, type_id: int, size_n: int, size_k: int,
+           flags: int = K_FULL) -> torch.Tensor:
+    """gptq_marlin_gemm on x [..., size_k] -> [..., size_n]: straight into the native code in eager mode, through
+    the operator where something traces or intercepts operators."""
+    if not _is_compiling():
+        out = _linear(x, weight, bias, scales, global_scale, zeros, g_idx, perm, workspace, type_id, -1, size_n, size_k,
+                      flags)
+        if out is not None:
+            return out
+    a = x.reshape(-1, x.shape[-1])
+    out = _ops.gptq_marlin_gemm(a, None, weight, bias, scales, global_scale, zeros, g_idx, perm, workspace, type_id,
+                                a.shape[0], size_n, size_k, bool(flags & K_FULL), False, True, bool(flags & ZP_FLOAT))
+    return out.reshape(x.shape[:-1] + (size_n,))
 
 
 def moe_wna16_marlin_gemm(input: torch.Tensor, output: torch.Tensor | None, b_qweight: torch.Tensor,

@@ -102,6 +102,21 @@ bool tc_path_enabled() {
   return on;
 }
 
+// Integer weights up to 32 rows: decode kernel or tensor-core kernel.  The decode kernel starts faster and
+// spends less per weight up to 16 rows of 4-bit codes; the tensor-core kernel streams at a rate that does
+// not depend on the rows.  The lines are where the two meet on B200 (us, decode / tensor cores; 4-bit g128:
+// 24 rows 4096 x 4096 10.0 / 10.3, 4096 x 6144 13.9 / 12.0, 4096 x 28672 51 / 31, 4096 x 1024, where the
+// decode kernel has too few slices, 10.2 / 6.7; 8-bit channel-wise, one row: 2048 x 2048 5.0 / 5.9,
+// 4096 x 4096 11.4 / 9.3, 4096 x 28672 43 / 30).
+bool few_rows_on_tc(int64_t m, int64_t n, int64_t k, int bits, int gm) {
+  const int64_t weights = n * k;
+  const int64_t M = 1 << 20;
+  if (bits == 8) return m > 16 ? weights >= 2 * M : weights >= (gm == kChannel ? 16 * M : 20 * M);
+  if (m <= 16) return false;
+  if (gm == kChannel) return weights >= 100 * M || (n <= 2048 && k >= 2048);
+  return weights >= 20 * M || n < 2048;
+}
+
 inline int64_t align_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
 
 // partial-sum scratch: (grid + slices) slots of (rows x slice width) floats
@@ -311,7 +326,7 @@ static int gemm_impl(const void* a, int64_t lda, const uint32_t* b_q_weight, con
   // these run the tensor-core kernel at every row count (the reference-order one where it can not)
   const bool general_only = zp_float || w_fp8 || w_fp4;
   // ---- tensor-core kernel: many rows, and the float formats at every row count ------------
-  if ((size_m >= 33 || general_only) && tc_path_enabled() && tc_gemm_supported(size_n, size_k, gm)) {
+  if ((size_m >= 33 || general_only || (!link && few_rows_on_tc(size_m, size_n, size_k, bits, gm))) && tc_path_enabled() && tc_gemm_supported(size_n, size_k, gm)) {
     const int fmt = zp_float ? (bits == 4 ? kTcU4ZF : kTcU8ZF)
                     : w_fp8 ? kTcF8
                     : w_fp4 ? (fp4_scales == 1 ? kTcNV4 : kTcMX4)

@@ -17,8 +17,14 @@
 //
 // Compiled with the host compiler only (no device code here); links libb200q.so.
 #include <ATen/ATen.h>
+#include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <ATen/record_function.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
 #include <torch/library.h>
 
 #include <memory>
@@ -133,7 +139,9 @@ at::Tensor check_gemm(const at::Tensor& a, const std::optional<at::Tensor>& c_or
     TORCH_CHECK(c.size(1) == size_n, "Shape mismatch: c.size(1) = ", c.size(1), ", size_n = ", size_n);
     TORCH_CHECK(c.scalar_type() == a.scalar_type(), "c must have the dtype of a");
   } else {
-    c = at::empty({size_m, size_n}, a.options());
+    // (not at::empty: one trip through the dispatcher less)
+    const int64_t shape[2] = {size_m, size_n};
+    c = at::detail::empty_cuda(shape, a.scalar_type(), a.device(), std::nullopt);
   }
   g->act_order = false;
   if (size_m == 0) return c;
@@ -585,6 +593,62 @@ at::Tensor fused_marlin_moe(const at::Tensor& hidden, const at::Tensor& w1, cons
       "fused_marlin_moe");
   return out;
 }
+
+// ---- direct call from Python -------------------------------------------------------------------
+// The operator without the dispatcher: linear(a, weight, bias, scales, global_scale, zeros, g_idx, perm,
+// workspace, type_id, size_m, size_n, size_k, flags) -> output, or None when something wants to see
+// the call go through the dispatcher (a dispatch or torch-function mode, functorch, a profiler, tensor
+// subclasses, autograd), in which case the caller issues the operator.  a: [..., size_k]; size_m = -1 takes
+// the rows of a as they are.  An eager decode step issues a few hundred such calls; operator parsing,
+// boxing and reshapes in Python cost 8 us of a call's 15.
+bool plain_tensor(PyObject* o) { return THPVariable_CheckExact(o); }
+bool optional_tensor(PyObject* o, std::optional<at::Tensor>* t) {
+  if (o == Py_None) return true;
+  if (!plain_tensor(o)) return false;
+  *t = THPVariable_Unpack(o);
+  return true;
+}
+
+PyObject* py_linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(nargs == 14, "linear takes 14 arguments");
+  if (c10::impl::TorchDispatchModeTLS::any_modes_set() || at::impl::PythonTorchFunctionTLS::stack_len() > 0 ||
+      at::hasCallbacks() || c10::impl::tls_local_dispatch_key_set().included_ != c10::default_included_set)
+    Py_RETURN_NONE;
+  if (!plain_tensor(args[0]) || !plain_tensor(args[1]) || !plain_tensor(args[3]) || !plain_tensor(args[8]))
+    Py_RETURN_NONE;
+  std::optional<at::Tensor> bias, global_scale, zeros, g_idx, perm;
+  if (!optional_tensor(args[2], &bias) || !optional_tensor(args[4], &global_scale) || !optional_tensor(args[5], &zeros) ||
+      !optional_tensor(args[6], &g_idx) || !optional_tensor(args[7], &perm))
+    Py_RETURN_NONE;
+  const at::Tensor& x = THPVariable_Unpack(args[0]);
+  if (!x.is_cuda() || x.dim() < 1 || (x.requires_grad() && c10::GradMode::is_enabled())) Py_RETURN_NONE;
+  const int64_t type_id = PyLong_AsLongLong(args[9]), size_m = PyLong_AsLongLong(args[10]),
+                size_n = PyLong_AsLongLong(args[11]), size_k = PyLong_AsLongLong(args[12]);
+  const long flags = PyLong_AsLong(args[13]);  // 1: is_k_full, 2: is_zp_float
+  if (PyErr_Occurred()) return nullptr;
+  at::Tensor a = x.dim() == 2 ? x : x.reshape({-1, x.size(-1)});
+  const int64_t rows = size_m < 0 ? a.size(0) : size_m;
+  at::Tensor w = THPVariable_Unpack(args[1]), s = THPVariable_Unpack(args[3]), ws = THPVariable_Unpack(args[8]);
+  at::Tensor c = gptq_marlin_gemm(a, std::nullopt, w, bias, s, global_scale, zeros, g_idx, perm, ws, type_id, rows, size_n,
+                                  size_k, flags & 1, false, true, (flags & 2) != 0);
+  if (x.dim() != 2) {
+    c10::SmallVector<int64_t, 6> shape(x.sizes().begin(), x.sizes().end());
+    shape.back() = size_n;
+    c = c.view(shape);
+  }
+  return THPVariable_Wrap(std::move(c));
+  END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef g_methods[] = {
+    {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_linear)), METH_FASTCALL,
+     "gptq_marlin_gemm without the dispatcher; None when the call has to go through it"},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "b200q_direct", nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};
+
+// New reference to a module with the functions above (called through ctypes.PyDLL).
+extern "C" PyObject* b200q_torch_python_module() { return PyModule_Create(&g_module); }
 
 std::unique_ptr<torch::Library> g_moe_defs, g_moe_impls;
 

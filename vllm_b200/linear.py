@@ -106,7 +106,7 @@ class ColumnParallelLinear(LinearBase):
                                         self.tp_size)
 
     def forward(self, input_: torch.Tensor) -> torch.Tensor:
-        out = self.quant_method.apply(self, input_, self.bias)
+        out = self.quant_method.apply(self, input_, self._parameters.get("bias"))
         if self.gather_output and self.tp_size > 1:
             out = tensor_model_parallel_all_gather(out)
         return out
@@ -171,7 +171,7 @@ class RowParallelLinear(LinearBase):
         with what follows, e.g. residual add + RMSNorm)."""
         if not self.input_is_parallel and self.tp_size > 1:
             input_ = input_.chunk(self.tp_size, dim=-1)[self.tp_rank].contiguous()
-        bias = self.bias if (self.tp_rank == 0 or self.tp_size == 1) else None
+        bias = self._parameters.get("bias") if (self.tp_rank == 0 or self.tp_size == 1) else None
         if not (reduce and self.reduce_results and self.tp_size > 1):
             return self.quant_method.apply(self, input_, bias)
         if all_reduce is not tensor_model_parallel_all_reduce:

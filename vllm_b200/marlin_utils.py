@@ -238,6 +238,9 @@ def apply_gptq_marlin_linear(input: torch.Tensor, weight: torch.Tensor,
                              reduce_link=None) -> torch.Tensor:
     """reduce_link (not in the reference): a peer-memory link; the output is then all-reduced
     over it by the same op (row-parallel layers)."""
+    if reduce_link is None:
+        return ops.linear(input, weight, bias, weight_scale, None, weight_zp, g_idx, g_idx_sort_indices, workspace,
+                          wtype.id, output_size_per_partition, input_size_per_partition, ops.K_FULL if is_k_full else 0)
     reshaped_x = input.reshape(-1, input.shape[-1])
     out_shape = input.shape[:-1] + (output_size_per_partition,)
     use_atomic_add = should_use_atomic_add_reduce(
@@ -260,6 +263,9 @@ def apply_awq_marlin_linear(input: torch.Tensor, weight: torch.Tensor,
                             bias: torch.Tensor | None = None,
                             use_fp32_reduce: bool = USE_FP32_REDUCE_DEFAULT,
                             reduce_link=None) -> torch.Tensor:
+    if reduce_link is None:
+        return ops.linear(input, weight, bias, weight_scale, None, weight_zp, g_idx, g_idx_sort_indices, workspace,
+                          quant_type.id, output_size_per_partition, input_size_per_partition, ops.K_FULL)
     reshaped_x = input.reshape(-1, input.shape[-1])
     out_shape = input.shape[:-1] + (output_size_per_partition,)
     use_atomic_add = should_use_atomic_add_reduce(

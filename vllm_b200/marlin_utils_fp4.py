@@ -8,7 +8,7 @@ import torch
 
 from . import _custom_ops as ops
 from .marlin_utils import (USE_FP32_REDUCE_DEFAULT, marlin_make_workspace_new, marlin_permute_bias,
-                           marlin_permute_scales, should_use_atomic_add_reduce)
+                           marlin_permute_scales)
 from .scalar_type import scalar_types
 
 FP4_MARLIN_SUPPORTED_GROUP_SIZES = [16]
@@ -66,13 +66,8 @@ def apply_fp4_marlin_linear(input: torch.Tensor, weight: torch.Tensor, weight_sc
                             size_n: int, size_k: int, bias: torch.Tensor | None = None,
                             use_fp32_reduce: bool = USE_FP32_REDUCE_DEFAULT) -> torch.Tensor:
     """marlin_utils_fp4.py:93-133."""
-    x = input.reshape(-1, input.shape[-1])
-    use_atomic_add = should_use_atomic_add_reduce(m=x.size(0), n=size_n, k=size_k,
-                                                  device=input.device, dtype=input.dtype)
-    out = ops.gptq_marlin_gemm(x, None, weight, bias, weight_scale, weight_scale_2, None, None, None,
-                               workspace, scalar_types.float4_e2m1f, x.size(0), size_n, size_k,
-                               use_atomic_add=use_atomic_add, use_fp32_reduce=use_fp32_reduce)
-    return out.reshape(input.shape[:-1] + (size_n,))
+    return ops.linear(input, weight, bias, weight_scale, weight_scale_2, None, None, None, workspace,
+                      scalar_types.float4_e2m1f.id, size_n, size_k)
 
 
 def _fp4_codes_to_dtype(codes: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:

@@ -8,7 +8,7 @@ import torch
 
 from . import _custom_ops as ops
 from .marlin_utils import (USE_FP32_REDUCE_DEFAULT, marlin_make_workspace_new,
-                           marlin_permute_scales, should_use_atomic_add_reduce)
+                           marlin_permute_scales)
 from .scalar_type import scalar_types
 
 
@@ -83,12 +83,5 @@ def apply_fp8_marlin_linear(input: torch.Tensor, weight: torch.Tensor, weight_sc
                             bias: torch.Tensor | None,
                             use_fp32_reduce: bool = USE_FP32_REDUCE_DEFAULT) -> torch.Tensor:
     """marlin_utils_fp8.py:40-79."""
-    reshaped_x = input.reshape(-1, input.shape[-1])
-    out_shape = input.shape[:-1] + (size_n,)
-    use_atomic_add = should_use_atomic_add_reduce(m=reshaped_x.size(0), n=size_n, k=size_k,
-                                                  device=input.device, dtype=input.dtype)
-    output = ops.gptq_marlin_gemm(
-        reshaped_x, None, weight, bias, weight_scale, None, None, None, None, workspace,
-        scalar_types.float8_e4m3fn, size_m=reshaped_x.size(0), size_n=size_n, size_k=size_k,
-        use_atomic_add=use_atomic_add, use_fp32_reduce=use_fp32_reduce)
-    return output.reshape(out_shape)
+    return ops.linear(input, weight, bias, weight_scale, None, None, None, None, workspace,
+                      scalar_types.float8_e4m3fn.id, size_n, size_k)
