@@ -298,6 +298,10 @@ int b200q_fused_add_rms_norm(void* input, int64_t ld_input, void* residual, cons
                              float epsilon, int64_t num_tokens, int64_t hidden_size, int dtype,
                              b200q_stream_t stream);
 
+/* out = rms_norm(input) * weight, out contiguous (may be the input); row stride of input ld_input elements */
+int b200q_rms_norm(void* out, const void* input, int64_t ld_input, const void* weight, float epsilon,
+                   int64_t num_tokens, int64_t hidden_size, int dtype, b200q_stream_t stream);
+
 /*
  * The same with the SUM all-reduce of `input` over the peer link in front, in one
  * kernel: what follows RowParallelLinear in a decoder layer (all-reduce, residual

@@ -325,11 +325,14 @@ def rms_norm(out: torch.Tensor, input: torch.Tensor, weight: torch.Tensor, epsil
     """out = rms_norm(input) * weight (vllm/_custom_ops.py:328-333)."""
     _check(out.is_contiguous() and out.shape == input.shape and out.dtype == input.dtype,
            "out must be contiguous with the shape and dtype of input")
-    out.copy_(input)
     n = out.size(-1)
+    if not (input.dtype == out.dtype and input.device == out.device and input.stride(-1) == 1 and n % 8 == 0
+            and input.data_ptr() % 16 == 0 and (input.is_contiguous() or (input.dim() == 2 and input.stride(0) % 8 == 0))):
+        out.copy_(input)          # whatever copy_ can bring into the shape of the output
+        input = out
     with _on_device(out.device):
-        rc = _L.b200q_fused_add_rms_norm(_ptr(out), n, None, _ptr(weight), float(epsilon),
-                                         out.numel() // n, n, _dtype_code(out), _stream(out.device))
+        rc = _L.b200q_rms_norm(_ptr(out), _ptr(input), n if input.is_contiguous() else input.stride(0), _ptr(weight),
+                               float(epsilon), out.numel() // n, n, _dtype_code(out), _stream(out.device))
     _lib.check(rc, "rms_norm")
 
 

@@ -106,6 +106,8 @@ def load() -> ctypes.CDLL:
     lib.b200q_all_reduce.restype = i32
     lib.b200q_fused_add_rms_norm.restype = i32
     lib.b200q_fused_add_rms_norm.argtypes = [vp, i64, vp, vp, c.c_float, i64, i64, i32, vp]
+    lib.b200q_rms_norm.restype = i32
+    lib.b200q_rms_norm.argtypes = [vp, vp, i64, vp, c.c_float, i64, i64, i32, vp]
     lib.b200q_all_reduce_fused_add_rms_norm.restype = i32
     lib.b200q_all_reduce_fused_add_rms_norm.argtypes = [vp, vp, i32, i32, i64, vp, vp, vp, c.c_float,
                                                         i64, i64, i32, vp]

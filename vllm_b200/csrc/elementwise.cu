@@ -24,7 +24,9 @@ namespace ew {
 constexpr int kNormThreads = 512;
 
 struct NormParams {
-  void* x;            // [M, N] in: (partial) input, out: normalised; row stride ldx elements
+  void* x;            // [M, N] out: normalised; in (when src is null): (partial) input; row stride ldx elements
+  const void* src;    // [M, N] input of a plain out-of-place rms_norm, row stride ldsrc; or null
+  int64_t ldsrc;
   int64_t ldx;
   void* residual;     // [M, N] contiguous, in/out; may be null (plain rms_norm of x)
   const void* weight; // [N]
@@ -42,15 +44,28 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
   return (uint32_t)Pair<T>::from_float(a) | ((uint32_t)Pair<T>::from_float(b) << 16);
 }
 
-// One block per row; a thread handles 16-byte vectors v = tid, tid + blockDim, ...
+// One block per row; a thread handles 16-byte vectors v = tid, tid + blockDim, ...  Latency-bound at
+// decode sizes (a few rows): the weight is fetched and the next kernel in the stream (a GEMM, which starts
+// fetching its own weights) is let go before this one waits for its input, and up to kKeep vectors per
+// thread stay in registers between the sum of squares and the scaling.
+constexpr int kKeep = 4;
 template <typename T>
 __global__ void __launch_bounds__(kNormThreads, 1) fused_add_rms_norm_kernel(const NormParams p) {
   __shared__ float s_part[kNormThreads / 32];
   __shared__ float s_rstd;
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   const int row = blockIdx.x;
   const int vecs = p.n / 8;
+  const uint4* wrow = static_cast<const uint4*>(p.weight);
+  uint4 keep[kKeep], gain[kKeep];
+#pragma unroll
+  for (int i = 0; i < kKeep; ++i) {
+    const int v = threadIdx.x + i * blockDim.x;
+    if (v < vecs) gain[i] = wrow[v];
+  }
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  const uint4* srow = p.src ? reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.src) + (size_t)row * p.ldsrc)
+                            : nullptr;
   uint4* xrow = reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.x) + (size_t)row * p.ldx);
   uint4* rrow = p.residual
                     ? reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.residual) + (size_t)row * p.n)
@@ -77,14 +92,15 @@ __global__ void __launch_bounds__(kNormThreads, 1) fused_add_rms_norm_kernel(con
   const char* mybuf = l.world ? static_cast<const char*>(l.bufs[l.rank]) + parity_off : nullptr;
   float ss = 0.f;
   bool ok = true;
-  for (int v = threadIdx.x; v < vecs && ok; v += blockDim.x) {
-    uint4 x = xrow[v];
+  // input, all-reduce and residual of vector v; adds to the sum of squares
+  auto take = [&](int v) {
+    uint4 x = srow ? srow[v] : xrow[v];
     if (l.world) {
       // all-reduce: fp32 sum in rank order, one rounding (what the separate kernel stores)
       uint32_t d[kArMaxWorld][4];
       if (!ar_collect<4>(l, mybuf, ((size_t)row * vecs + v) * 32, flag, d)) {
         ok = false;
-        break;
+        return x;
       }
       float acc[8];
 #pragma unroll
@@ -109,8 +125,6 @@ __global__ void __launch_bounds__(kNormThreads, 1) fused_add_rms_norm_kernel(con
       x.z = pack2<T>(lo_f<T>(x.z) + lo_f<T>(r.z), hi_f<T>(x.z) + hi_f<T>(r.z));
       x.w = pack2<T>(lo_f<T>(x.w) + lo_f<T>(r.w), hi_f<T>(x.w) + hi_f<T>(r.w));
       rrow[v] = x;
-    } else {
-      xrow[v] = x;  // the reduced row, normalised in place below
     }
     const uint32_t w[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
@@ -118,6 +132,17 @@ __global__ void __launch_bounds__(kNormThreads, 1) fused_add_rms_norm_kernel(con
       const float a = lo_f<T>(w[e]), b = hi_f<T>(w[e]);
       ss += a * a + b * b;
     }
+    return x;
+  };
+#pragma unroll
+  for (int i = 0; i < kKeep; ++i) {
+    const int v = threadIdx.x + i * blockDim.x;
+    if (v < vecs && ok) keep[i] = take(v);
+  }
+  // longer rows: the rest waits in the residual, or in x where there is none
+  for (int v = threadIdx.x + kKeep * blockDim.x; v < vecs && ok; v += blockDim.x) {
+    const uint4 x = take(v);
+    if (!rrow) xrow[v] = x;
   }
   // block sum of squares
 #pragma unroll
@@ -131,11 +156,8 @@ __global__ void __launch_bounds__(kNormThreads, 1) fused_add_rms_norm_kernel(con
   }
   __syncthreads();
   const float rstd = s_rstd;
-  const uint4* wrow = static_cast<const uint4*>(p.weight);
   const uint4* zrow = rrow ? rrow : xrow;
-  for (int v = threadIdx.x; v < vecs; v += blockDim.x) {
-    const uint4 z = zrow[v];
-    const uint4 g = wrow[v];
+  auto finish = [&](int v, const uint4& z, const uint4& g) {
     const uint32_t zw[4] = {z.x, z.y, z.z, z.w}, gw[4] = {g.x, g.y, g.z, g.w};
     uint32_t o[4];
 #pragma unroll
@@ -146,7 +168,13 @@ __global__ void __launch_bounds__(kNormThreads, 1) fused_add_rms_norm_kernel(con
       o[e] = pack2<T>(a * lo_f<T>(gw[e]), b * hi_f<T>(gw[e]));
     }
     xrow[v] = make_uint4(o[0], o[1], o[2], o[3]);
+  };
+#pragma unroll
+  for (int i = 0; i < kKeep; ++i) {
+    const int v = threadIdx.x + i * blockDim.x;
+    if (v < vecs && ok) finish(v, keep[i], gain[i]);
   }
+  for (int v = threadIdx.x + kKeep * blockDim.x; v < vecs && ok; v += blockDim.x) finish(v, zrow[v], wrow[v]);
   if (l.world) {
     __syncthreads();
     if (threadIdx.x == 0) ar_arrive(l, call, gridDim.x);
@@ -157,8 +185,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) silu_and_mul_kernel(const uint16_t* __restrict__ in,
                                                            uint16_t* __restrict__ out, int64_t m,
                                                            int d) {
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
   const int vecs = d / 8;
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= m * vecs) return;
@@ -201,8 +229,9 @@ int launch_norm(NormParams p, int dtype, cudaStream_t stream) {
   B200Q_REQUIRE(p.x && p.weight, B200Q_EINVAL, "null pointer");
   B200Q_REQUIRE(p.ldx >= p.n && p.ldx % 8 == 0, B200Q_EINVAL, "row stride must be a multiple of 8");
   B200Q_REQUIRE(((reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.weight) |
-                  reinterpret_cast<uintptr_t>(p.residual)) & 15) == 0,
+                  reinterpret_cast<uintptr_t>(p.residual) | reinterpret_cast<uintptr_t>(p.src)) & 15) == 0,
                 B200Q_EINVAL, "tensors must be aligned to 16 bytes");
+  B200Q_REQUIRE(!p.src || (p.ldsrc >= p.n && p.ldsrc % 8 == 0), B200Q_EINVAL, "row stride must be a multiple of 8");
   if (p.m == 0) return B200Q_OK;
   int threads = (p.n / 8 + 31) / 32 * 32;
   if (threads > kNormThreads) threads = kNormThreads;
@@ -225,6 +254,23 @@ extern "C" int b200q_fused_add_rms_norm(void* input, int64_t ld_input, void* res
   p.x = input;
   p.ldx = ld_input;
   p.residual = residual;
+  p.weight = weight;
+  p.eps = epsilon;
+  p.m = (int)num_tokens;
+  p.n = (int)hidden_size;
+  return ew::launch_norm(p, dtype, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int b200q_rms_norm(void* out, const void* input, int64_t ld_input, const void* weight, float epsilon,
+                              int64_t num_tokens, int64_t hidden_size, int dtype, b200q_stream_t stream) {
+  B200Q_REQUIRE(num_tokens >= 0 && num_tokens < (1ll << 31) && hidden_size < (1ll << 31),
+                B200Q_EINVAL, "size out of range");
+  B200Q_REQUIRE(input, B200Q_EINVAL, "null pointer");
+  ew::NormParams p = {};
+  p.x = out;
+  p.ldx = hidden_size;
+  p.src = input;
+  p.ldsrc = ld_input;
   p.weight = weight;
   p.eps = epsilon;
   p.m = (int)num_tokens;

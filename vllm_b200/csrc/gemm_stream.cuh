@@ -206,6 +206,8 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
   const uint16_t* __restrict__ Bias = static_cast<const uint16_t*>(p.bias);
   const int32_t* moe_ids = nullptr;   // this block's sorted ids
   if constexpr (MOE) {
+    // the ids may come from the kernel in front; without them the weights are not known
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
     // (uniform over the cluster: its CTAs share blockIdx.y)
     if ((int)blockIdx.y * p.m >= *p.moe_num_padded) return;
     const int expert = p.moe_expert_ids[blockIdx.y];

@@ -104,7 +104,7 @@ class AWQMarlinLinearMethod:
         layer.g_idx = marlin_make_empty_g_idx(device)
         layer.g_idx_sort_indices = marlin_make_empty_g_idx(device)
         if getattr(layer, "bias", None) is not None:
-            layer.bias.data = marlin_permute_bias(layer.bias)
+            replace("bias", marlin_permute_bias(layer.bias.data))
 
     def apply(self, layer: torch.nn.Module, x: torch.Tensor,
               bias: torch.Tensor | None = None, reduce_link=None) -> torch.Tensor:

@@ -122,7 +122,7 @@ class GPTQMarlinLinearMethod:
                                                 group_size=qc.group_size))
         replace("qzeros", marlin_make_empty_g_idx(device))
         if getattr(layer, "bias", None) is not None:
-            layer.bias.data = marlin_permute_bias(layer.bias)
+            replace("bias", marlin_permute_bias(layer.bias.data))
 
     def apply(self, layer: torch.nn.Module, x: torch.Tensor,
               bias: torch.Tensor | None = None, reduce_link=None) -> torch.Tensor:
