@@ -43,6 +43,7 @@ struct StreamParams {
   long long moe_b_stride, moe_s_stride, moe_z_stride, moe_bias_stride;  // per expert: words / elements
   // weight-embedding constants of the streaming kernel (filled by its launcher)
   uint32_t c_ex, c_mask_lo, c_mask_hi;
+  uint32_t c_zero;  // 0, for values the compiler is not to treat as uniform
   // when ar.world > 0 the streaming kernel all-reduces its output over the link
   ArLink ar;
 };

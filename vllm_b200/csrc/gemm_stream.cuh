@@ -200,7 +200,15 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
   const int KT = p.kt_total;
   const int NT = p.n / 64;
   const uint16_t* __restrict__ S = static_cast<const uint16_t*>(p.scales);
-  const uint32_t ex = p.c_ex, mlo = p.c_mask_lo, mhi = p.c_mask_hi;
+  // Made to look different per thread: values known to be uniform live in uniform registers, which cost
+  // copies in front of every LOP3 and MMA that uses them (4096 -> 28672 at one row 19.2 -> 18.9 us).  Not where
+  // the registers are full already: with zero-points the loop became 7 % slower, with blocks of experts 2 %.
+  const uint32_t vary = HAS_ZP || MOE ? 0u : threadIdx.x & p.c_zero;
+  const uint32_t ex = p.c_ex ^ vary, mlo = p.c_mask_lo ^ vary, mhi = p.c_mask_hi ^ vary;
+  const uint32_t off_lo = (kBiased ? E::kOffLoBiased : E::kOffLoRaw) ^ vary;
+  const uint32_t off_hi = (kBiased ? E::kOffHiBiased : E::kOffHiRaw) ^ vary;
+  const uint32_t off[4] = {off_lo, off_lo, off_hi, off_hi};
+  const uint32_t one[4] = {E::kOneLo ^ vary, E::kOneLo ^ vary, E::kOneHi ^ vary, E::kOneHi ^ vary};
   const unsigned char* __restrict__ Bw = reinterpret_cast<const unsigned char*>(p.b);
   const uint32_t* __restrict__ Zp = p.zeros;
   const uint16_t* __restrict__ Bias = static_cast<const uint16_t*>(p.bias);
@@ -488,17 +496,8 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
 #pragma unroll
       for (int i = 0; i < MT; ++i) {
         if (E::kPrescale) act[i][1] = Pair<T>::mul(act[i][1], E::kAScaleHi);
-        if (E::kEmbed) {
-          const uint32_t off[4] = {kBiased ? E::kOffLoBiased : E::kOffLoRaw,
-                                   kBiased ? E::kOffLoBiased : E::kOffLoRaw,
-                                   kBiased ? E::kOffHiBiased : E::kOffHiRaw,
-                                   kBiased ? E::kOffHiBiased : E::kOffHiRaw};
-          mma16816<T>(corr[i], off, act[i][0], act[i][1]);
-        }
-        if (HAS_ZP) {
-          const uint32_t one[4] = {E::kOneLo, E::kOneLo, E::kOneHi, E::kOneHi};
-          mma16816<T>(rsum[i], one, act[i][0], act[i][1]);
-        }
+        if (E::kEmbed) mma16816<T>(corr[i], off, act[i][0], act[i][1]);
+        if (HAS_ZP) mma16816<T>(rsum[i], one, act[i][0], act[i][1]);
       }
 
 #pragma unroll
