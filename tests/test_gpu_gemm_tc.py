@@ -145,6 +145,34 @@ def test_tc_gemm_edges(env, M, K, N, qtype, group, dtype):
     _check(out, mo.gemm_ref(a, L.w), f"{M} {K} {N} {qtype} g{group}")
 
 
+def test_captured_call_keeps_its_scratch(env):
+    """A graph's calls do not use the scratch that later, larger calls replace."""
+    torch, G, ops, mu, lib = env
+    from vllm_b200.scalar_type import scalar_types
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    ws, e = mu.marlin_make_workspace_new(torch.device("cuda")), torch.empty(0, dtype=torch.int32, device="cuda")
+
+    def problem(M, K, N):
+        q = torch.randint(-2**31, 2**31 - 1, (K // 16, N * 2), dtype=torch.int32, device="cuda", generator=gen)
+        s = (torch.rand((K // 128, N), device="cuda", generator=gen) * 0.018 + 0.002).half()
+        a = torch.randn((M, K), device="cuda", dtype=torch.float16, generator=gen)
+        return lambda: ops.gptq_marlin_gemm(a, None, q, None, s, None, e, e, e, ws, scalar_types.uint4b8, M, N, K, True,
+                                            False, True, False)
+
+    calls = [problem(40, 2048, 1024), problem(48, 4096, 4096), problem(200, 4096, 14336)]
+    want = [c() for c in calls]
+    graphs, outs = [], []
+    for c in calls:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            outs.append(c())
+        graphs.append(g)
+    for g in graphs + graphs[::-1]:
+        g.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, w) for o, w in zip(outs, want))
+
+
 @pytest.mark.parametrize("M,qtype,group", [(100, "uint4b8", 128), (300, "uint8b128", -1), (700, "uint8b128", 128)])
 def test_tc_gemm_is_reproducible(env, M, qtype, group):
     """The same call gives the same bits every time: a weight slot that is refilled before it was read

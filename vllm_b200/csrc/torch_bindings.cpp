@@ -56,15 +56,20 @@ bool decode_type(int64_t id, TypeInfo* t) {
 
 // Scratch of the GEMM: fp32 partial sums, and the gathered activations of act-order
 // layers.  One grow-only buffer per (device, stream): calls on one stream are ordered,
-// so they can share it; calls on different streams must not.
-at::Tensor& scratch_for(const at::Device& dev, cudaStream_t stream, size_t bytes) {
+// so they can share it; calls on different streams must not.  A call that is being captured
+// gets memory of its own from the graph's pool (`own`): the shared buffer may be replaced by a larger
+// one, and released, while the graph is still in use.
+at::Tensor& scratch_for(const at::Device& dev, cudaStream_t stream, size_t bytes, at::Tensor& own) {
   static std::mutex mu;
   static std::unordered_map<uint64_t, at::Tensor> cache;
+  const auto make = [&] { return at::empty({(int64_t)bytes}, at::TensorOptions().dtype(at::kByte).device(dev)); };
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) cudaGetLastError();
+  if (status != cudaStreamCaptureStatusNone) return own = make();
   const uint64_t key = ((uint64_t)(uintptr_t)stream << 8) ^ (uint64_t)(dev.index() & 0xff);
   std::lock_guard<std::mutex> lock(mu);
   at::Tensor& t = cache[key];
-  if (!t.defined() || (size_t)t.numel() < bytes)
-    t = at::empty({(int64_t)bytes}, at::TensorOptions().dtype(at::kByte).device(dev));
+  if (!t.defined() || (size_t)t.numel() < bytes) t = make();
   return t;
 }
 
@@ -261,7 +266,8 @@ at::Tensor gptq_marlin_gemm(at::Tensor& a, std::optional<at::Tensor> c_or_none,
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream(a.get_device());
   const size_t nbytes =
       b200q_marlin_gemm_preferred_scratch_bytes(size_m, size_n, size_k, g.act_order ? 1 : 0);
-  at::Tensor& scratch = scratch_for(a.device(), stream, nbytes);
+  at::Tensor own;
+  at::Tensor& scratch = scratch_for(a.device(), stream, nbytes, own);
   int rc;
   if (g.fp4_scales != 0) {
     TORCH_CHECK(g.zeros == nullptr && !g.act_order,
@@ -310,7 +316,8 @@ at::Tensor gptq_marlin_gemm_all_reduce(
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream(a.get_device());
   const size_t nbytes =
       b200q_marlin_gemm_preferred_scratch_bytes(size_m, size_n, size_k, g.act_order ? 1 : 0);
-  at::Tensor& scratch = scratch_for(a.device(), stream, nbytes);
+  at::Tensor own;
+  at::Tensor& scratch = scratch_for(a.device(), stream, nbytes, own);
   const int rc = b200q_marlin_gemm_all_reduce(
       g.a, g.lda, g.b, g.scales, g.zeros, g.g_idx, g.perm, g.bias, c.data_ptr(), scratch.data_ptr(),
       (size_t)scratch.numel(), workspace.data_ptr<int32_t>(), workspace.numel(), b_q_type, g.dtype,
