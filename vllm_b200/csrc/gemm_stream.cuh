@@ -37,6 +37,7 @@
 // spinning, and the result is bitwise reproducible.
 #pragma once
 
+#include <atomic>
 #include <cstdlib>
 
 #include "gemm_params.cuh"
@@ -202,8 +203,9 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
   const uint16_t* __restrict__ S = static_cast<const uint16_t*>(p.scales);
   // Made to look different per thread: values known to be uniform live in uniform registers, which cost
   // copies in front of every LOP3 and MMA that uses them (4096 -> 28672 at one row 19.2 -> 18.9 us).  Not where
-  // the registers are full already: with zero-points the loop became 7 % slower, with blocks of experts 2 %.
-  const uint32_t vary = HAS_ZP || MOE ? 0u : threadIdx.x & p.c_zero;
+  // the registers are full already: with zero-points the loop became 7 % slower, with
+  // 16 rows and one tile per slice 8 %, with blocks of experts 2 %.
+  const uint32_t vary = HAS_ZP || MOE || (MT == 2 && NTW == 1) ? 0u : threadIdx.x & p.c_zero;
   const uint32_t ex = p.c_ex ^ vary, mlo = p.c_mask_lo ^ vary, mhi = p.c_mask_hi ^ vary;
   const uint32_t off_lo = (kBiased ? E::kOffLoBiased : E::kOffLoRaw) ^ vary;
   const uint32_t off_hi = (kBiased ? E::kOffHiBiased : E::kOffHiRaw) ^ vary;
@@ -776,6 +778,30 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
   }
 }
 
+// Clusters of `size` CTAs that run at once on the current device (per kernel; asked once per device and size).
+template <typename K>
+int max_clusters(K kernel, int smem, int size, std::atomic<int>& known) {
+  int n = known.load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(size * 1024);
+  cfg.blockDim = dim3(kStreamThreads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = size;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
+    cudaGetLastError();
+    n = device_sm_count() / size;
+  }
+  known.store(n, std::memory_order_relaxed);
+  return n;
+}
+
 // Host launcher for one (type, bits, zp, group mode, MT, NTW) variant.
 template <typename T, int BITS, bool HAS_ZP, int GM, int MT, int NTW, bool MOE = false>
 int launch_stream(StreamParams p, int max_ctas, cudaStream_t stream) {
@@ -801,7 +827,20 @@ int launch_stream(StreamParams p, int max_ctas, cudaStream_t stream) {
   const int target = device_sm_count() * kMinBlocks;
   int ksplit = 1;
   const int blocks = MOE ? p.moe_blocks : 1;
-  while (ksplit < 8 && p.slices * blocks * ksplit * 2 <= target && p.kt_total / (ksplit * 2) >= 8) ksplit *= 2;
+  // (and no more than run at once: a cluster has to fit into one GPC, so of the 16 clusters of 8 that 148 SMs
+  // seem to hold one waits for a second round; 2048 x 2048 at 9 rows took 9.3 us with them, 5.7 with clusters
+  // of 4)
+  static std::atomic<int> fit[64][4];
+  for (int s = 1; ksplit < 8 && s < 4; ++s) {
+    const int more = 1 << s;
+    if (p.slices * blocks * more > target || p.kt_total / more < 8) break;
+    if (p.slices * blocks > max_clusters(kernel, Cfg::kSmemBytes, more, fit[dev & 63][s])) break;
+    // two CTAs on an SM instead of one: only with enough k to pay for the wider exchange of sums (4-bit,
+    // 1024 x 4096 at one row 6.1 us in eight parts, 4.3 in four; 4096 x 4096 6.0 against 7.2)
+    const int least = more == 8 ? 24 : BITS == 4 ? 17 : 12;
+    if (p.slices * blocks * more > device_sm_count() && p.kt_total / more < least) break;
+    ksplit = more;
+  }
   (void)max_ctas;
   const int grid = p.slices * ksplit;
   // programmatic dependent launch: the kernel may start while its predecessor in
