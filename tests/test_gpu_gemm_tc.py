@@ -145,6 +145,27 @@ def test_tc_gemm_edges(env, M, K, N, qtype, group, dtype):
     _check(out, mo.gemm_ref(a, L.w), f"{M} {K} {N} {qtype} g{group}")
 
 
+@pytest.mark.parametrize("M,K,N,qtype,group,dtype", [
+    (9, 1024, 2048, "uint4b8", 128, "float16"),     # sixteen clusters of eight would not run at once
+    (16, 2048, 2048, "uint8b128", 128, "bfloat16"),
+    (20, 1024, 2048, "uint4b8", -1, "bfloat16"),
+    (1, 1024, 4096, "uint4b8", 128, "bfloat16"),    # too little k for eight parts
+    (8, 3072, 4096, "uint4", 128, "float16"),       # eight parts, two CTAs on an SM
+    (4, 1024, 6144, "uint8b128", -1, "float16"),
+    (12, 5504, 2560, "uint4b8", 128, "float16"),    # either side of the line to the tensor-core kernel
+    (8, 2304, 9024, "uint8b128", 128, "float16"),
+    (16, 1152, 19392, "uint8b128", -1, "bfloat16"),  # fewer rounds in the last wave than workers
+    (32, 2048, 4096, "uint4", 64, "bfloat16"),
+])
+def test_few_rows_split_edges(env, M, K, N, qtype, group, dtype):
+    torch, G, ops, mu, lib = env
+    L = H.make_layer(K, N, qtype, group, False, dtype)
+    a = H.make_activations(M, K, dtype)
+    out = G.run_gemm(ops, mu, L, a)
+    assert lib.b200q_device_error(1) == 0
+    _check(out, mo.gemm_ref(a, L.w), f"{M} {K} {N} {qtype} g{group}")
+
+
 def test_captured_call_keeps_its_scratch(env):
     """A graph's calls do not use the scratch that later, larger calls replace."""
     torch, G, ops, mu, lib = env

@@ -84,6 +84,7 @@ int launch_tc_gemm(const void* a, int64_t lda, const uint32_t* b, const void* sc
 // weight formats of the tensor-core kernel (gemm_tc.cuh)
 enum { kTcU4B8, kTcU4Z, kTcU8B128, kTcU8Z, kTcF8, kTcNV4, kTcMX4, kTcU4ZF, kTcU8ZF };
 int64_t tc_gemm_scratch_bytes(int64_t size_m, int64_t size_n, int64_t size_k);
+double tc_gemm_estimate_us(int64_t size_m, int64_t size_n, int64_t size_k, double factor);
 int tc_error_flag(bool reset);
 int ar_error_flag(bool reset);
 
@@ -102,19 +103,54 @@ bool tc_path_enabled() {
   return on;
 }
 
-// Integer weights up to 32 rows: decode kernel or tensor-core kernel.  The decode kernel starts faster and
-// spends less per weight up to 16 rows of 4-bit codes; the tensor-core kernel streams at a rate that does
-// not depend on the rows.  The lines are where the two meet on B200 (us, decode / tensor cores; 4-bit g128:
-// 24 rows 4096 x 4096 10.0 / 10.3, 4096 x 6144 13.9 / 12.0, 4096 x 28672 51 / 31, 4096 x 1024, where the
-// decode kernel has too few slices, 10.2 / 6.7; 8-bit channel-wise, one row: 2048 x 2048 5.0 / 5.9,
-// 4096 x 4096 11.4 / 9.3, 4096 x 28672 43 / 30).
-bool few_rows_on_tc(int64_t m, int64_t n, int64_t k, int bits, int gm) {
-  const int64_t weights = n * k;
-  const int64_t M = 1 << 20;
-  if (bits == 8) return m > 16 ? weights >= 2 * M : weights >= (gm == kChannel ? 16 * M : 20 * M);
-  if (m <= 16) return false;
-  if (gm == kChannel) return weights >= 100 * M || (n <= 2048 && k >= 2048);
-  return weights >= 20 * M || n < 2048;
+// Work split of the decode kernel as launch_stream makes it, with the clusters that fit taken as three fewer
+// than the SMs would hold (true of 4 and 8 CTAs on 148 SMs).
+struct DecodeSplit {
+  int64_t ctas, parts, tiles;  // CTAs; CTAs per column slice; k-tiles (16 x 64) that the busiest SM reads
+  bool one_tile;               // slices of one 64-column tile
+};
+DecodeSplit decode_split(int64_t m, int64_t n, int64_t k, int bits, int gm) {
+  const int64_t nt = n / 64, kt = k / 16, sms = device_sm_count();
+  const int mt = m <= 8 ? 1 : m <= 16 ? 2 : 4;
+  const int ntw = nt % 2 == 0 && (gm == kChannel || mt <= 2) ? 2 : 1;
+  const int per_sm = mt * ntw * (gm == kGrouped ? 2 : 1) <= 4 && mt <= 2 ? 2 : 1;
+  const int64_t slices = nt / ntw;
+  int64_t parts = 1;
+  for (int64_t more = 2; more <= 8; more *= 2) {
+    if (slices * more > sms * per_sm || kt / more < 8 || (more > 2 && slices > sms * per_sm / more - 3)) break;
+    if (slices * more > sms && kt / more < (more == 8 ? 24 : bits == 4 ? 17 : 12)) break;
+    parts = more;
+  }
+  return {slices * parts, parts, (slices * parts + sms - 1) / sms * ntw * ((kt + parts - 1) / parts), ntw == 1};
+}
+
+// Integer weights up to 32 rows: decode kernel or tensor-core kernel, by estimated time.  The decode kernel
+// takes a time per k-tile of its busiest SM that grows with the rows (its instructions), and how its whole
+// column slices divide among the SMs decides the rest; the tensor-core kernel divides the weights evenly and
+// its conversion does not depend on the rows.  The constants are fits to B200 times over 18 shapes from
+// 1024 x 1024 to 9472 x 18624.  (8-bit g128 fp16, 8 rows, us, decode / tensor cores: 7168 x 9024, 141 slices on
+// 148 SMs, 22.4 / 20.1; 3456 x 9024 13.0 / 13.1; 11008 x 5120, 160 half slices, 28.0 / 18.6.)
+bool few_rows_on_tc(int64_t m, int64_t n, int64_t k, int bits, int gm, bool has_zp, bool bf16) {
+  if (m > 32 || (bits == 4 && m <= 8)) return false;
+  const bool grouped = gm == kGrouped;
+  const DecodeSplit d = decode_split(m, n, k, bits, gm);
+  const bool alone = d.ctas <= device_sm_count();  // one CTA on an SM where two would fit
+  double base = 3.0, tile, factor;  // us: fixed and per tile of the decode kernel; conversion cost, 1 = 4-bit
+  if (bits == 8) {
+    factor = bf16 ? (grouped ? 1.22 : 1.15) : (grouped ? 1.08 : 1.03);
+    if (m <= 8) tile = alone ? 0.048 : bf16 && d.one_tile ? 0.045 : 0.041;
+    else if (m <= 16) tile = alone && !grouped ? 0.070 : d.one_tile ? 0.052 : 0.045;
+    else tile = grouped ? 0.056 : bf16 && d.one_tile ? 0.090 : 0.047;
+    if (m > 16) base = grouped ? 2.6 + 0.4 * (double)d.parts : 5.0;
+  } else {
+    factor = has_zp ? 1.17 : 1.0;
+    if (m <= 16) tile = (grouped ? 0.0245 : 0.020) * (has_zp ? 1.06 : 1.0);
+    else tile = (grouped ? 0.046 : 0.0295) * (has_zp ? 1.2 : 1.0);
+    if (m > 16) base = grouped ? 2.6 + 0.4 * (double)d.parts : 5.0;
+  }
+  // clusters of eight that nearly fill the GPU start in turns
+  if (d.parts == 8 && 2 * d.ctas > 3 * device_sm_count()) base += 2.0;
+  return tc_gemm_estimate_us(m, n, k, factor) < 0.98 * (base + tile * (double)d.tiles);
 }
 
 inline int64_t align_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
@@ -326,7 +362,7 @@ static int gemm_impl(const void* a, int64_t lda, const uint32_t* b_q_weight, con
   // these run the tensor-core kernel at every row count (the reference-order one where it can not)
   const bool general_only = zp_float || w_fp8 || w_fp4;
   // ---- tensor-core kernel: many rows, and the float formats at every row count ------------
-  if ((size_m >= 33 || general_only || (!link && few_rows_on_tc(size_m, size_n, size_k, bits, gm))) && tc_path_enabled() && tc_gemm_supported(size_n, size_k, gm)) {
+  if ((size_m >= 33 || general_only || (!link && few_rows_on_tc(size_m, size_n, size_k, bits, gm, has_zp, a_dtype == B200Q_BF16))) && tc_path_enabled() && tc_gemm_supported(size_n, size_k, gm)) {
     const int fmt = zp_float ? (bits == 4 ? kTcU4ZF : kTcU8ZF)
                     : w_fp8 ? kTcF8
                     : w_fp4 ? (fp4_scales == 1 ? kTcNV4 : kTcMX4)

@@ -161,6 +161,8 @@ static int launch_reduce(const TcParams& p, int cg, cudaStream_t stream) {
 struct TcPlan {
   int cg, tn, box, tok_tiles, workers, sk_tiles;
   int64_t partial_bytes;
+  double us;         // estimate that the plans are compared by
+  double rounds_us;  // the part of it that is rounds
 };
 
 // Microseconds of a round (128 deep in k) of one tile, measured on B200 as the slope over K at one tile per
@@ -178,7 +180,7 @@ static double round_us(int cg, int tn) {
 static TcPlan plan_tiles(int64_t m, int64_t n, int64_t k, int sms, int64_t scratch_bytes) {
   const int64_t rounds = (k / kBK + 1) / 2;
   TcPlan best = {};
-  double best_cost = 1e300;
+  best.us = 1e300;
   for (int cg = 1; cg <= 2; ++cg) {
     if (cg == 2 && m <= 64) break;
     const int64_t most = 128 * cg, grain = 16 * cg;
@@ -197,21 +199,24 @@ static TcPlan plan_tiles(int64_t m, int64_t n, int64_t k, int sms, int64_t scrat
       const double round = round_us(cg, pl.tn);
       const int64_t waves = tiles / most_workers, rem = tiles % most_workers;
       pl.workers = (int)(tiles < most_workers ? tiles : most_workers);
-      double cost = (double)((waves + (rem > 0)) * rounds) * round;
-      if (cost < best_cost) { best_cost = cost; best = pl; }
+      const double cost = (double)((waves + (rem > 0)) * rounds) * round;
+      pl.us = pl.rounds_us = cost;
+      if (cost < best.us) best = pl;
       if (rem == 0) continue;
       // at least two rounds for every worker
       const int64_t by_work = rem * rounds / 2;
       int64_t workers = by_work < most_workers ? by_work : most_workers;
       if (waves > 0) workers = most_workers;
-      if (workers <= rem) continue;
+      if (workers <= rem || rem * rounds < workers) continue;  // every worker has a round: the sums are taken over all
       pl.workers = (int)workers;
       pl.sk_tiles = (int)rem;
       const int64_t slot_bytes = (int64_t)cg * pl.tn * kBN * 4;
       pl.partial_bytes = 2 * workers * slot_bytes;
-      cost = (double)(waves * rounds + (rem * rounds + workers - 1) / workers) * round + 2.5 +
-             2.0 * (double)((workers + rem) * slot_bytes) / 4e6;
-      if (pl.partial_bytes <= scratch_bytes && cost < best_cost) { best_cost = cost; best = pl; }
+      pl.rounds_us = (double)(waves * rounds + (rem * rounds + workers - 1) / workers) * round;
+      // a second segment behind whole tiles: its own pipeline fill and drain (1152 x 19392, 152 tiles of nine
+      // rounds: 15.2 us with the last four shared, 11.0 in two waves)
+      pl.us = pl.rounds_us + 2.5 + (waves > 0 ? 2.0 : 0.0) + 2.0 * (double)((workers + rem) * slot_bytes) / 4e6;
+      if (pl.partial_bytes <= scratch_bytes && pl.us < best.us) best = pl;
     }
   }
   return best;
@@ -306,6 +311,16 @@ int launch_tc_moe(const void* a, int64_t rows, const uint32_t* b, const void* sc
 int64_t tc_gemm_scratch_bytes(int64_t size_m, int64_t size_n, int64_t size_k) {
   if (size_k % tc::kBK != 0 || size_n % 64 != 0) return 0;
   return tc::plan_tiles(size_m, size_n, size_k, device_sm_count(), int64_t(1) << 40).partial_bytes;
+}
+
+// Estimated time of the kernel (and its reduce kernel) in us; `factor`: cost of the weight conversion, 1 = 4-bit.
+double tc_gemm_estimate_us(int64_t size_m, int64_t size_n, int64_t size_k, double factor) {
+  const tc::TcPlan pl = tc::plan_tiles(size_m, size_n, size_k, device_sm_count(), int64_t(1) << 40);
+  const double us = factor * pl.rounds_us;
+  if (pl.sk_tiles == 0) return 3.0 + us;
+  // the exchange of sums: more of it with more tokens, less where there are only a few rounds to exchange
+  const bool behind_whole_tiles = (size_n + tc::kBN * pl.cg - 1) / (tc::kBN * pl.cg) * pl.tok_tiles > pl.sk_tiles;
+  return 5.0 + (us < 2.7 ? 0.55 * us : 1.5) + 0.02 * (double)size_m + (behind_whole_tiles ? 1.0 : 0.0) + us;
 }
 
 int tc_error_flag(bool reset) {
