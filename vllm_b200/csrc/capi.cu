@@ -499,7 +499,6 @@ extern "C" int b200q_moe_wna16_marlin_gemm(
   p.c = c;
   p.m = (int)moe_block_size; p.n = (int)size_n; p.k = (int)size_k;
   p.kt_total = kt_total;
-  p.slices = (int)(size_n / 64);
   p.group_blocks = group_blocks;
   p.num_groups = (int)num_groups;
   p.moe_sorted_ids = sorted_token_ids;
@@ -514,14 +513,16 @@ extern "C" int b200q_moe_wna16_marlin_gemm(
   p.moe_z_stride = (long long)num_groups * size_n * bits / 32;
   p.moe_bias_stride = size_n;
   if (p.moe_blocks == 0) return B200Q_OK;
-  const int mb8 = (int)(moe_block_size / 8);  // 8-row blocks: 2, 4, 6, 8
+  const int mb8 = (int)(moe_block_size / 8);  // 8-row blocks: 1, 2, 4, 6, 8
+  const int ntw = mb8 == 1 && size_n % 128 == 0 ? 2 : 1;
+  p.slices = (int)(size_n / 64 / ntw);
   int rc;
   if (a_dtype == B200Q_F16)
-    rc = bits == 4 ? dispatch_stream<half, 4>(p, has_zp, gm, mb8, 1, 1 << 20, stream)
-                   : dispatch_stream<half, 8>(p, has_zp, gm, mb8, 1, 1 << 20, stream);
+    rc = bits == 4 ? dispatch_stream<half, 4>(p, has_zp, gm, mb8, ntw, 1 << 20, stream)
+                   : dispatch_stream<half, 8>(p, has_zp, gm, mb8, ntw, 1 << 20, stream);
   else
-    rc = bits == 4 ? dispatch_stream<__nv_bfloat16, 4>(p, has_zp, gm, mb8, 1, 1 << 20, stream)
-                   : dispatch_stream<__nv_bfloat16, 8>(p, has_zp, gm, mb8, 1, 1 << 20, stream);
+    rc = bits == 4 ? dispatch_stream<__nv_bfloat16, 4>(p, has_zp, gm, mb8, ntw, 1 << 20, stream)
+                   : dispatch_stream<__nv_bfloat16, 8>(p, has_zp, gm, mb8, ntw, 1 << 20, stream);
   if (rc == B200Q_EUNSUPPORTED && g_error[0] == 0) set_error("moe: unsupported configuration");
   return rc;
 }

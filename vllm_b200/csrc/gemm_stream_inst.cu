@@ -104,10 +104,12 @@ int fp4_weights(const StreamParams& p, int gm, int rows8, int ntw, int max_ctas,
 
 // mixture-of-experts form: the reference-order kernel over (block of sorted ids, column slice)
 template <bool HAS_ZP, int GM>
-int moe_blocks(const StreamParams& p, int rows8, int max_ctas, cudaStream_t stream) {
+int moe_blocks(const StreamParams& p, int rows8, int ntw, int max_ctas, cudaStream_t stream) {
   // blocks of up to 32 ids: the decode kernel; above: the reference-order kernel
   switch (rows8) {
-    case 1: return launch_stream<T, B, HAS_ZP, GM, 1, 1, true>(p, max_ctas, stream);
+    case 1:
+      return ntw == 2 ? launch_stream<T, B, HAS_ZP, GM, 1, 2, true>(p, max_ctas, stream)
+                      : launch_stream<T, B, HAS_ZP, GM, 1, 1, true>(p, max_ctas, stream);
     case 2: return launch_stream<T, B, HAS_ZP, GM, 2, 1, true>(p, max_ctas, stream);
     case 4: return launch_stream<T, B, HAS_ZP, GM, 4, 1, true>(p, max_ctas, stream);
   }
@@ -122,13 +124,13 @@ int moe_blocks(const StreamParams& p, int rows8, int max_ctas, cudaStream_t stre
 }
 
 int moe(const StreamParams& p, bool has_zp, int gm, int rows8, int ntw, int max_ctas, cudaStream_t stream) {
-  if (ntw != 1 || p.zp_float) return B200Q_EUNSUPPORTED;
+  if (p.zp_float || (ntw != 1 && rows8 != 1)) return B200Q_EUNSUPPORTED;
   if (gm == kChannel)
-    return has_zp ? moe_blocks<true, kChannel>(p, rows8, max_ctas, stream)
-                  : moe_blocks<false, kChannel>(p, rows8, max_ctas, stream);
+    return has_zp ? moe_blocks<true, kChannel>(p, rows8, ntw, max_ctas, stream)
+                  : moe_blocks<false, kChannel>(p, rows8, ntw, max_ctas, stream);
   if (gm == kGrouped)
-    return has_zp ? moe_blocks<true, kGrouped>(p, rows8, max_ctas, stream)
-                  : moe_blocks<false, kGrouped>(p, rows8, max_ctas, stream);
+    return has_zp ? moe_blocks<true, kGrouped>(p, rows8, ntw, max_ctas, stream)
+                  : moe_blocks<false, kGrouped>(p, rows8, ntw, max_ctas, stream);
   return B200Q_EUNSUPPORTED;
 }
 
