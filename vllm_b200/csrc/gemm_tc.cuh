@@ -256,9 +256,12 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// four 8 x 8 matrices of 16-bit values in the MMA fragment layout; lane 8 i + r gives row r of matrix i
 template <int OFF>
-__device__ __forceinline__ void sts32_off(uint32_t addr, uint32_t v) {
-  asm volatile("st.shared.u32 [%0+%2], %1;\n" ::"r"(addr), "r"(v), "n"(OFF) : "memory");
+__device__ __forceinline__ void stmatrix_x4_off(uint32_t addr, const uint32_t (&f)[4]) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0+%5], {%1,%2,%3,%4};\n" ::"r"(addr), "r"(f[0]), "r"(f[1]),
+               "r"(f[2]), "r"(f[3]), "n"(OFF)
+               : "memory");
 }
 
 // Shared-memory matrix descriptor: K-major tile, 128-byte swizzle, rows 128 B apart, 8-row atoms 1024 B
@@ -588,9 +591,10 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
     const int c8 = lane >> 2, q = lane & 3;
     const int group = warp >> 3;
     const int kt = warp & 3, nt = (warp >> 2) & 1;  // k-tile of both steps of the round, column tile
-    // byte offsets of this lane's two k-positions (k = 16 kt + 2q, + 8) inside a 128 B row
-    const uint32_t b_lo_rel = 2 * Cfg::kTokBytes + (nt * 64 + c8) * 128 + (((2 * kt) ^ c8) << 4) + 4 * q;
-    const uint32_t b_hi_rel = 2 * Cfg::kTokBytes + (nt * 64 + c8) * 128 + (((2 * kt + 1) ^ c8) << 4) + 4 * q;
+    // The fragments of a 16 x 16 sub-tile are four 8 x 8 matrices (k lo and hi of columns 0-7, of columns 8-15):
+    // one stmatrix.  This lane's row of it: matrix lane / 8, column lane % 8, a 16-byte chunk of a 128 B row.
+    const uint32_t b_rel = 2 * Cfg::kTokBytes + (nt * 64 + (lane & 7) + 8 * (lane >> 4)) * 128 +
+                           (((2 * kt + ((lane >> 3) & 1)) ^ (lane & 7)) << 4);
     const uint32_t w_rel = kt * (2 * Cfg::kTileBytes) + nt * Cfg::kTileBytes + lane * (BITS * 4);
     const uint32_t fa0 = kPair ? mapa(full(0), 0) : full(0);
     // scale rows of this warp's two k-tiles within the round's copy, where they are the same in every round
@@ -659,11 +663,11 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         if (lane == 0) mbar_arrive(empty_w(wr.i) + (got & p.zero));
         wr.next(2);
         if (live) {
-          const uint32_t b_lo0 = smem_base + ring.i * Cfg::kSlot + b_lo_rel, b_hi0 = smem_base + ring.i * Cfg::kSlot + b_hi_rel;
+          const uint32_t b0 = smem_base + ring.i * Cfg::kSlot + b_rel;
 #pragma unroll
           for (int st = 0; st < 2; ++st) {
             if (2 * r + st >= steps) break;  // the last round of an odd number of steps
-            const uint32_t b_lo = b_lo0 + st * Cfg::kABytes, b_hi = b_hi0 + st * Cfg::kABytes;
+            const uint32_t b = b0 + st * Cfg::kABytes;
             const uint32_t (&w)[NW] = w2[st];
             const uint32_t (&sc)[4] = sc2[st];
             const uint32_t (&zr)[4] = zr2[st];
@@ -718,10 +722,7 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) f[i] = Pair<T>::mul(f[i], Fp8Cvt<T>::kRebias);
               }
-              sts32_off<sub * 2048>(b_lo, f[0]);
-              sts32_off<sub * 2048>(b_hi, f[1]);
-              sts32_off<sub * 2048 + 1024>(b_lo, f[2]);
-              sts32_off<sub * 2048 + 1024>(b_hi, f[3]);
+              stmatrix_x4_off<sub * 2048>(b, f);
             };
             auto convert_all = [&](auto scaled_c) {
               convert(std::integral_constant<int, 0>{}, scaled_c);
