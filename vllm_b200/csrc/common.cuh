@@ -176,8 +176,17 @@ struct Pair<__nv_bfloat16> {
 };
 
 // Duplicate the low / high 16 bits of x into both halves.
-__device__ __forceinline__ uint32_t dup_lo(uint32_t x) { return __byte_perm(x, x, 0x1010); }
-__device__ __forceinline__ uint32_t dup_hi(uint32_t x) { return __byte_perm(x, x, 0x3232); }
+// (as 16-bit moves, which can become half selectors of the instruction that uses the pair)
+__device__ __forceinline__ uint32_t dup_lo(uint32_t x) {
+  uint32_t d;
+  asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tmov.b32 %0, {l, l};\n\t}\n" : "=r"(d) : "r"(x));
+  return d;
+}
+__device__ __forceinline__ uint32_t dup_hi(uint32_t x) {
+  uint32_t d;
+  asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tmov.b32 %0, {h, h};\n\t}\n" : "=r"(d) : "r"(x));
+  return d;
+}
 
 // ---- integer code -> 16-bit float pairs (exact) --------------------------------
 // One 32-bit word of the Marlin layout expands to pairs (k, k+1) for the two
