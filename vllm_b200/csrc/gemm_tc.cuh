@@ -650,14 +650,13 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         }
         if (!(ok = mbar_wait<kPair>(empty(ring.i), ring.ph ^ 1, (3 << 8) | 4, cta_abort, p.error))) break;
         // The slot goes back as soon as its words are in registers.  A release does not wait for loads still
-        // in flight (seen: a slot refilled before it was read), so the arrival is made to depend on them.
+        // in flight (seen: a slot refilled before it was read), so the arrival is made to depend on a word of
+        // each of them (the words of one vector load arrive together).
         uint32_t got = 0;
 #pragma unroll
         for (int st = 0; st < 2; ++st) {
-#pragma unroll
-          for (int i = 0; i < NW; ++i) got |= w2[st][i];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) got |= sc2[st][i] | zr2[st][i];
+          got |= w2[st][0] | w2[st][NW - 1] | sc2[st][0] | zr2[st][0];
+          if (I::kFp4 || BITS == 8) got |= sc2[st][1] | zr2[st][1];
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(empty_w(wr.i) + (got & p.zero));
