@@ -583,7 +583,7 @@ def time_fp4(torch, ops, dev, dt, stream, gen, ws, steps):
         b = k * n // 2 + (k // group) * n + 2 * m * k + 2 * m * n      # weights, scale bytes, A, C
         rows.append({"m": m, "us": round(us, 2), "gbs": round(b / us / 1e3, 1),
                      "tflops": round(2.0 * m * n * k / us / 1e6, 2)})
-    return {"workload": "nvfp4 (float4_e2m1f, group 16) gate_up 4096->28672, reference-order kernel",
+    return {"workload": "nvfp4 (float4_e2m1f, group 16) gate_up 4096->28672, tensor-core kernel",
             "steps": steps, "per_shape": rows}
 
 
@@ -634,7 +634,7 @@ def time_moe(torch, ops, dev, dt, stream, gen, ws, steps):
                      "gbs": round(b / us / 1e3, 1),
                      "tflops": round(2.0 * m * topk * n * k / us / 1e6, 2)})
     return {"workload": "moe_wna16_marlin_gemm: 8 experts, top-2, gate_up 4096 -> 28672, uint4b8 g128, "
-                        "reference-order kernel", "steps": steps, "per_shape": rows}
+                        "decode kernel, reference-order kernel for blocks above 32", "steps": steps, "per_shape": rows}
 
 
 def run_ar_check(torch, dist, D, lib, dev, custom_ar, ar_link, rank, world):
