@@ -1,0 +1,25 @@
+"""Order of the hand-offs in the tensor-core kernel, read from its source: a missing fence shows in no result, or in one
+of many thousand, so that running the kernel is no test of it."""
+import os
+import re
+
+SRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "vllm_b200", "csrc", "gemm_tc.cuh")
+
+
+def _code():
+    with open(SRC) as f:
+        return re.sub(r"//[^\n]*", "", f.read())
+
+
+def test_weight_slots_go_back_behind_a_proxy_fence():
+    """The producer refills a weight slot with a copy (async proxy): between the last read of a slot and the arrival
+    that gives it back stand the proxy fence of every reading lane and, after it, the warp barrier."""
+    code = _code()
+    dequant = code[code.index("mbar_wait<false>(full_w"):]
+    arrivals = [m.start() for m in re.finditer(r"mbar_arrive\(empty_w\(", dequant)]
+    assert arrivals and "mbar_arrive(empty_w(" not in code[:code.index("mbar_wait<false>(full_w")]
+    for at in arrivals:
+        before = dequant[:at]
+        read = max(before.rfind("lds128("), before.rfind("lds32("))
+        fence, sync = before.rfind("fence_proxy_async_smem();"), before.rfind("__syncwarp();")
+        assert read < fence < sync
