@@ -23,3 +23,17 @@ def test_weight_slots_go_back_behind_a_proxy_fence():
         read = max(before.rfind("lds128("), before.rfind("lds32("))
         fence, sync = before.rfind("fence_proxy_async_smem();"), before.rfind("__syncwarp();")
         assert read < fence < sync
+
+
+def test_arrivals_at_the_other_cta_release_at_cluster_scope():
+    """What the second CTA of a pair has stored is read by the first one's MMA: the arrival that says so is a release
+    at cluster scope, and the waits on the barriers that the pair shares acquire at cluster scope."""
+    code = _code()
+    remote = [m.start() for m in re.finditer(r"mbarrier\.arrive[\w.]*\.shared::cluster", code)]
+    assert len(remote) == 1
+    body = code[code.rfind("__device__", 0, remote[0]):remote[0] + 80]
+    assert "mbar_arrive_cluster" in body
+    assert body.index("fence.release.sync_restrict::shared::cta.cluster") < body.index("mbarrier.arrive.relaxed.cluster")
+    assert "try_wait.parity.acquire.cluster" in code
+    mma = code[code.index("warp == kMmaWarp) {"):code.index("warp < kDequantWarps) {")]
+    assert "mbar_wait<kPair>(full(" in mma and "mbar_wait<kPair>(tmem_empty(" in mma

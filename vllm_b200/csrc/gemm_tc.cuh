@@ -21,7 +21,10 @@
 //                     a round took 1450 cycles, half of them waits that all warps sat out together)
 //   MMA warp          one elected lane issues eight 128 (256) x tn x 16 MMAs per round, commits the slot back
 //                     (a satisfied barrier wait costs about 200 cycles beside twenty busy warps, so token rows
-//                     and converted weights share one barrier, and it is waited for once per round)
+//                     and converted weights share one barrier, and it is waited for once per round).  In the
+//                     second CTA of a pair this warp passes on, one cluster-scope release per round, that the
+//                     CTA's weights are converted (each dequant warp doing so itself cost its conversion: an
+//                     eight-expert layer at 500 tokens 431 us against 416)
 //   4 epilogue warps  TMEM -> registers -> scale, bias, rounding -> C, while the next tile is computed
 //
 // Work is cut into (tile, k-range) segments.  Whole waves of tiles run one tile per CTA (pair); what
@@ -116,10 +119,13 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
-// arrive on a barrier given by its cluster address (mapa).  (With .release.cluster the arrive took 1350
-// cycles; the operand data is ordered by the proxy fence in front of it.)
+// arrive on a barrier of the other CTA, given by its cluster address (mapa), as a release at cluster scope of what
+// this thread has written or seen written in its own CTA's shared memory: that is all the waiter (acquire at
+// cluster scope) reads.  (An arrival's default scope is its own CTA; arrive.release.cluster took 1350 cycles, the
+// fence limited to shared memory costs a layer 0 to 1 %, 3 % at 200 tokens.)
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
+  asm volatile("fence.release.sync_restrict::shared::cta.cluster;\n" ::: "memory");
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
   uint32_t r;
@@ -444,7 +450,7 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
   auto tok_slot = [&](int i) { return smem_base + i * Cfg::kSlot; };
   auto a_slot = [&](int i) { return smem_base + i * Cfg::kSlot + 2 * Cfg::kTokBytes; };
   // barriers (8 bytes each).  full (token rows landed and weights converted) and tmem_empty of the
-  // leader CTA serve the pair.
+  // leader CTA serve the pair; full of the other CTA counts its own conversion.
   auto full = [&](int i) { return bars + 8 * i; };
   auto empty = [&](int i) { return bars + 8 * (RING + i); };
   auto full_w = [&](int w) { return bars + 8 * (2 * RING + w); };
@@ -470,7 +476,8 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
   if (threadIdx.x == 0) {
     s_abort = 0;
     for (int i = 0; i < RING; ++i) {
-      mbar_init(full(i), 1 + kDequantWarps / 2 * CG);
+      // conversion of this CTA; the leader's also the token rows and the other CTA's conversion
+      mbar_init(full(i), kDequantWarps / 2 + (rank == 0 ? CG : 0));
       mbar_init(empty(i), 1);
     }
     for (int w = 0; w < WD; ++w) {
@@ -550,7 +557,7 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
       }
     }
   } else if (warp == kMmaWarp) {
-    // ================= MMA issuer (leader CTA) ==========================================
+    // ================= MMA issuer (leader CTA), relay (the other CTA of a pair) ==========
     // the whole warp walks the loop, one elected lane issues
     if (rank == 0) {
       Ring<RING> ring;
@@ -584,6 +591,18 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         }
         ++seg_i;
       }
+    } else {
+      Ring<RING> ring;
+      bool ok = true;
+      const uint32_t leader = mapa(full(0), 0);
+      while (ok && sched.next(sg)) {
+        for (int r = sg.r0; r < sg.r1; ++r) {
+          if (!(ok = mbar_wait<false>(full(ring.i), ring.ph, (2 << 8) | 6, cta_abort, p.error))) break;
+          if (elect_one()) mbar_arrive_cluster(leader + 8 * ring.i);
+          __syncwarp();
+          ring.next();
+        }
+      }
     }
   } else if (warp < kDequantWarps) {
     // ================= dequant warps ====================================================
@@ -595,7 +614,6 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
     const uint32_t b_rel = 2 * Cfg::kTokBytes + (nt * 64 + (lane & 7) + 8 * (lane >> 4)) * 128 +
                            (((2 * kt + ((lane >> 3) & 1)) ^ (lane & 7)) << 4);
     const uint32_t w_rel = kt * (2 * Cfg::kTileBytes) + nt * Cfg::kTileBytes + lane * (BITS * 4);
-    const uint32_t fa0 = kPair ? mapa(full(0), 0) : full(0);
     // scale rows of this warp's two k-tiles within the round's copy, where they are the same in every round
     const bool fixed_row = (gb & 7) == 0 || (8 % gb) == 0;
     const int row0 = (gb & 7) == 0 ? 0 : kt / gb, row1 = (gb & 7) == 0 ? 0 : (kt + 4) / gb;
@@ -738,8 +756,7 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         fence_proxy_async_smem();  // generic-proxy stores -> visible to the tensor core
         __syncwarp();
         if (lane == 0) {
-          if (kPair) mbar_arrive_cluster(fa0 + 8 * ring.i);
-          else mbar_arrive(full(ring.i));
+          mbar_arrive(full(ring.i));
           if constexpr (kReleaseLate) mbar_arrive(empty_w(wr.i));
         }
         wr.next(2);
@@ -821,7 +838,7 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
-          if (kPair) mbar_arrive_cluster(te0 + 8 * buf);
+          if (kPair && rank != 0) mbar_arrive_cluster(te0 + 8 * buf);
           else mbar_arrive(tmem_empty(buf));
         }
       };
