@@ -79,8 +79,9 @@ int dispatch_stream(const StreamParams& p, bool has_zp, int gm, int mb, int ntw,
 bool tc_gemm_supported(int64_t size_n, int64_t size_k, int gm);
 int launch_tc_gemm(const void* a, int64_t lda, const uint32_t* b, const void* scales, const uint32_t* zeros,
                    const void* bias, const void* global_scale, void* c, int a_dtype, int fmt, int64_t size_m,
-                   int64_t size_n, int64_t size_k, int group_blocks, int channelwise, void* scratch,
+                   int64_t size_n, int64_t size_k, int group_blocks, int channelwise, bool sums, void* scratch,
                    int64_t scratch_bytes, cudaStream_t stream);
+bool tc_group_sums_supported(int64_t group_size);
 // weight formats of the tensor-core kernel (gemm_tc.cuh)
 enum { kTcU4B8, kTcU4Z, kTcU8B128, kTcU8Z, kTcF8, kTcNV4, kTcMX4, kTcU4ZF, kTcU8ZF };
 int64_t tc_gemm_scratch_bytes(int64_t size_m, int64_t size_n, int64_t size_k);
@@ -127,27 +128,31 @@ DecodeSplit decode_split(int64_t m, int64_t n, int64_t k, int bits, int gm) {
 // Integer weights up to 32 rows: decode kernel or tensor-core kernel, by estimated time.  The decode kernel
 // takes a time per k-tile of its busiest SM that grows with the rows (its instructions), and how its whole
 // column slices divide among the SMs decides the rest; the tensor-core kernel divides the weights evenly and
-// its conversion does not depend on the rows.  The constants are fits to B200 times over 18 shapes from
-// 1024 x 1024 to 9472 x 18624.  (8-bit g128 fp16, 8 rows, us, decode / tensor cores: 7168 x 9024, 141 slices on
-// 148 SMs, 22.4 / 20.1; 3456 x 9024 13.0 / 13.1; 11008 x 5120, 160 half slices, 28.0 / 18.6.)
-bool few_rows_on_tc(int64_t m, int64_t n, int64_t k, int bits, int gm, bool has_zp, bool bf16) {
+// its conversion does not depend on the rows.  Either way group scales are applied to fp32 sums.  The constants are
+// fits to B200 times over 18 shapes from 1024 x 1024 to 9472 x 18624; of 182 calls over 13 of them six take the
+// slower kernel by more than 6 %, two by more than 13.  (8-bit g128 fp16, 8 rows, us, decode / tensor cores:
+// 7168 x 9024, 141 slices on 148 SMs, 22.7 / 22.1; 3456 x 9024 12.4 / 14.1; 11008 x 5120, 160 half slices,
+// 27.8 / 20.1.)
+bool few_rows_on_tc(int64_t m, int64_t n, int64_t k, int bits, int gm, int group_blocks, bool has_zp, bool bf16) {
   if (m > 32 || (bits == 4 && m <= 8)) return false;
   const bool grouped = gm == kGrouped;
+  if (grouped && !tc_group_sums_supported(16 * (int64_t)group_blocks)) return false;
   const DecodeSplit d = decode_split(m, n, k, bits, gm);
   const bool alone = d.ctas <= device_sm_count();  // one CTA on an SM where two would fit
   double base = 3.0, tile, factor;  // us: fixed and per tile of the decode kernel; conversion cost, 1 = 4-bit
   if (bits == 8) {
-    factor = bf16 ? (grouped ? 1.22 : 1.15) : (grouped ? 1.08 : 1.03);
+    factor = bf16 ? (grouped ? 1.33 : 1.15) : (grouped ? 1.24 : 1.03);
     if (m <= 8) tile = alone ? 0.048 : bf16 && d.one_tile ? 0.045 : 0.041;
     else if (m <= 16) tile = alone && !grouped ? 0.070 : d.one_tile ? 0.052 : 0.045;
     else tile = grouped ? 0.056 : bf16 && d.one_tile ? 0.090 : 0.047;
     if (m > 16) base = grouped ? 2.6 + 0.4 * (double)d.parts : 5.0;
   } else {
-    factor = has_zp ? 1.17 : 1.0;
+    factor = grouped ? (has_zp ? 1.3 : 1.28) : has_zp ? 1.17 : 1.0;
     if (m <= 16) tile = (grouped ? 0.0245 : 0.020) * (has_zp ? 1.06 : 1.0);
     else tile = (grouped ? 0.046 : 0.0295) * (has_zp ? 1.2 : 1.0);
     if (m > 16) base = grouped ? 2.6 + 0.4 * (double)d.parts : 5.0;
   }
+  if (grouped && group_blocks < 8) factor = 1.8;  // two buffers of group sums a round
   // clusters of eight that nearly fill the GPU start in turns
   if (d.parts == 8 && 2 * d.ctas > 3 * device_sm_count()) base += 2.0;
   return tc_gemm_estimate_us(m, n, k, factor) < 0.98 * (base + tile * (double)d.tiles);
@@ -362,14 +367,15 @@ static int gemm_impl(const void* a, int64_t lda, const uint32_t* b_q_weight, con
   // these run the tensor-core kernel at every row count (the reference-order one where it can not)
   const bool general_only = zp_float || w_fp8 || w_fp4;
   // ---- tensor-core kernel: many rows, and the float formats at every row count ------------
-  if ((size_m >= 33 || general_only || (!link && few_rows_on_tc(size_m, size_n, size_k, bits, gm, has_zp, a_dtype == B200Q_BF16))) && tc_path_enabled() && tc_gemm_supported(size_n, size_k, gm)) {
+  if ((size_m >= 33 || general_only || (!link && few_rows_on_tc(size_m, size_n, size_k, bits, gm, group_blocks, has_zp, a_dtype == B200Q_BF16))) && tc_path_enabled() && tc_gemm_supported(size_n, size_k, gm)) {
     const int fmt = zp_float ? (bits == 4 ? kTcU4ZF : kTcU8ZF)
                     : w_fp8 ? kTcF8
                     : w_fp4 ? (fp4_scales == 1 ? kTcNV4 : kTcMX4)
                     : bits == 4 ? (has_zp ? kTcU4Z : kTcU4B8)
                                 : (has_zp ? kTcU8Z : kTcU8B128);
     int rc = launch_tc_gemm(a_used, lda_used, b_q_weight, b_scales, b_zeros, b_bias, global_scale, c, a_dtype, fmt,
-                            size_m, size_n, size_k, group_blocks, gm == kChannel, scratch,
+                            size_m, size_n, size_k, group_blocks, gm == kChannel,
+                            gm == kGrouped && size_m <= 32 && !general_only, scratch,
                             (int64_t)((scratch_bytes - a_tmp_bytes) / 256 * 256), stream);
     if (rc != B200Q_OK || !link) return rc;
     return launch_all_reduce(*link, c, c, size_m * size_n, a_dtype, stream);

@@ -8,7 +8,7 @@ __device__ int g_tc_error;
 
 // one definition per (type, format), in the gemm_tc_inst.cu units
 template <typename T, int F>
-int launch_format(const TcMaps& maps, const TcParams& p, int cg, bool pdl, cudaStream_t stream);
+int launch_format(const TcMaps& maps, const TcParams& p, int cg, bool sums, bool pdl, cudaStream_t stream);
 
 static int format_bits(int fmt) { return (fmt == kU8B128 || fmt == kU8Z || fmt == kF8 || fmt == kU8ZF) ? 8 : 4; }
 
@@ -223,20 +223,20 @@ static TcPlan plan_tiles(int64_t m, int64_t n, int64_t k, int sms, int64_t scrat
 }
 
 template <typename T>
-static int launch_type(const TcMaps& maps, const TcParams& p, int fmt, int cg, bool pdl, cudaStream_t stream) {
+static int launch_type(const TcMaps& maps, const TcParams& p, int fmt, int cg, bool sums, bool pdl, cudaStream_t stream) {
   switch (fmt) {
-    case kU4B8: return launch_format<T, kU4B8>(maps, p, cg, pdl, stream);
-    case kU4Z: return launch_format<T, kU4Z>(maps, p, cg, pdl, stream);
-    case kU8B128: return launch_format<T, kU8B128>(maps, p, cg, pdl, stream);
-    case kU8Z: return launch_format<T, kU8Z>(maps, p, cg, pdl, stream);
-    case kF8: return launch_format<T, kF8>(maps, p, cg, pdl, stream);
-    case kNV4: return launch_format<T, kNV4>(maps, p, cg, pdl, stream);
+    case kU4B8: return launch_format<T, kU4B8>(maps, p, cg, sums, pdl, stream);
+    case kU4Z: return launch_format<T, kU4Z>(maps, p, cg, sums, pdl, stream);
+    case kU8B128: return launch_format<T, kU8B128>(maps, p, cg, sums, pdl, stream);
+    case kU8Z: return launch_format<T, kU8Z>(maps, p, cg, sums, pdl, stream);
+    case kF8: return launch_format<T, kF8>(maps, p, cg, sums, pdl, stream);
+    case kNV4: return launch_format<T, kNV4>(maps, p, cg, sums, pdl, stream);
   }
   if constexpr (std::is_same<T, half>::value) {
-    if (fmt == kU4ZF) return launch_format<T, kU4ZF>(maps, p, cg, pdl, stream);
-    if (fmt == kU8ZF) return launch_format<T, kU8ZF>(maps, p, cg, pdl, stream);
+    if (fmt == kU4ZF) return launch_format<T, kU4ZF>(maps, p, cg, sums, pdl, stream);
+    if (fmt == kU8ZF) return launch_format<T, kU8ZF>(maps, p, cg, sums, pdl, stream);
   } else {
-    if (fmt == kMX4) return launch_format<T, kMX4>(maps, p, cg, pdl, stream);
+    if (fmt == kMX4) return launch_format<T, kMX4>(maps, p, cg, sums, pdl, stream);
   }
   set_error("weight format %d is not available for this activation type", fmt);
   return B200Q_EUNSUPPORTED;
@@ -249,10 +249,16 @@ bool tc_gemm_supported(int64_t size_n, int64_t size_k, int gm) {
   return size_k % tc::kBK == 0 && size_n % 64 == 0 && gm != kLookup && tc::get_encode_fn() != nullptr;
 }
 
-// a: [M, K] 16-bit row-major with row stride lda (already gathered for act-order).
+// True when the tensor-core kernel can apply these group scales to fp32 sums: groups of a step or of whole rounds.
+bool tc_group_sums_supported(int64_t group_size) { return group_size == tc::kBK || (group_size > 0 && group_size % (2 * tc::kBK) == 0); }
+// rows of a tile at most in that form (cg = 1: single CTAs, 2: pairs)
+int tc_group_sums_rows(int cg) { return tc::group_sums_tokens(cg); }
+
+// a: [M, K] 16-bit row-major with row stride lda (already gathered for act-order).  sums: group scales on the fp32
+// sums (up to 64 rows).
 int launch_tc_gemm(const void* a, int64_t lda, const uint32_t* b, const void* scales, const uint32_t* zeros,
                    const void* bias, const void* global_scale, void* c, int a_dtype, int fmt, int64_t size_m,
-                   int64_t size_n, int64_t size_k, int group_blocks, int channelwise, void* scratch,
+                   int64_t size_n, int64_t size_k, int group_blocks, int channelwise, bool sums, void* scratch,
                    int64_t scratch_bytes, cudaStream_t stream) {
   tc::TcParams p = {};
   int rc = tc::error_word(&p.error);
@@ -272,15 +278,16 @@ int launch_tc_gemm(const void* a, int64_t lda, const uint32_t* b, const void* sc
   // early launch only where this kernel's fixed costs matter: with many rows the waiting CTAs would take
   // the SMs from an act-order gather still running in front
   const bool pdl = pdl_enabled() && size_m <= 128;
-  rc = a_dtype == B200Q_F16 ? tc::launch_type<half>(maps, p, fmt, plan.cg, pdl, stream)
-                            : tc::launch_type<__nv_bfloat16>(maps, p, fmt, plan.cg, pdl, stream);
+  rc = a_dtype == B200Q_F16 ? tc::launch_type<half>(maps, p, fmt, plan.cg, sums, pdl, stream)
+                            : tc::launch_type<__nv_bfloat16>(maps, p, fmt, plan.cg, sums, pdl, stream);
   if (rc != B200Q_OK || plan.sk_tiles == 0) return rc;
   return a_dtype == B200Q_F16 ? tc::launch_reduce<half>(p, plan.cg, stream)
                               : tc::launch_reduce<__nv_bfloat16>(p, plan.cg, stream);
 }
 
 // Mixture of experts: rows of A in sorted order, tiles {expert, first row, rows} in device memory, written by
-// a kernel in front.  `box`: token rows a CTA stages; a tile has at most that many rows (pairs: twice).
+// a kernel in front.  `box`: token rows a CTA stages; a tile has at most that many rows (pairs: twice).  Group scales
+// go on the fp32 sums, as in the decode kernel that the same layer runs at fewer rows.
 int launch_tc_moe(const void* a, int64_t rows, const uint32_t* b, const void* scales, const uint32_t* zeros,
                   const void* bias, void* c, int a_dtype, int fmt, int64_t experts, int64_t size_n, int64_t size_k,
                   int64_t num_groups, int pairs, int box, const int4* tile_list, const int32_t* tile_count,
@@ -302,9 +309,9 @@ int launch_tc_moe(const void* a, int64_t rows, const uint32_t* b, const void* sc
   p.tile_list = tile_list; p.tile_count = tile_count;
   p.ids = row_weights || scatter ? ids : nullptr; p.scatter = scatter; p.row_weights = row_weights; p.out_rows = (int)rows;
   p.s_stride = num_groups * size_n; p.bias_stride = size_n;
-  const bool pdl = pdl_enabled();
-  return a_dtype == B200Q_F16 ? tc::launch_type<half>(maps, p, fmt, cg, pdl, stream)
-                              : tc::launch_type<__nv_bfloat16>(maps, p, fmt, cg, pdl, stream);
+  const bool pdl = pdl_enabled(), sums = !p.channelwise;
+  return a_dtype == B200Q_F16 ? tc::launch_type<half>(maps, p, fmt, cg, sums, pdl, stream)
+                              : tc::launch_type<__nv_bfloat16>(maps, p, fmt, cg, sums, pdl, stream);
 }
 
 // Scratch the tensor-core kernel would like for this problem (fp32 partials of shared tiles).

@@ -10,9 +10,10 @@
 // 96 B per clock of shared memory for the MMA operands alone, and 176 of the 128 there are together with
 // the conversion; the pair needs 64 for the operands and leaves room for two accumulators.
 //
-// Roles (23 warps), hand-offs through mbarriers; a step is 64 deep in k, two steps make a round:
-//   producer warp     packed weights, scales and zero-points of a round into a ring of kWD slots, one
-//                     2-D copy each (deep: this is what comes from HBM; with a copy per step and per scale
+// Roles (23 warps, 27 where group scales go on the sums), hand-offs through mbarriers; a step is 64 deep in k, two
+// steps make a round:
+//   producer warp     packed weights, scales and zero-points of a round into a ring of kWD slots (two to eight,
+//                     what the operands leave room for), one 2-D copy each (with a copy per step and per scale
 //                     row the issuing thread was the bottleneck at 925 cycles a step)
 //   token warp        token rows of a round (TMA, 128B swizzle) into kRing slots
 //   16 dequant warps  packed words -> exact 16-bit codes -> scaled -> K-major swizzled operand in shared
@@ -25,7 +26,7 @@
 //                     second CTA of a pair this warp passes on, one cluster-scope release per round, that the
 //                     CTA's weights are converted (each dequant warp doing so itself cost its conversion: an
 //                     eight-expert layer at 500 tokens 431 us against 416)
-//   4 epilogue warps  TMEM -> registers -> scale, bias, rounding -> C, while the next tile is computed
+//   epilogue warps    4, or 8: TMEM -> registers -> scale, bias, rounding -> C, while the next tile is computed
 //
 // Work is cut into (tile, k-range) segments.  Whole waves of tiles run one tile per CTA (pair); what
 // would be a ragged last wave (or the only one) is cut into equal k-ranges instead: the workers of such a
@@ -71,11 +72,13 @@ constexpr int kBK = 64;            // k per step: one 128-byte swizzle row of 16
 constexpr int kRoundTiles = 8;     // k-tiles (16 rows) per round of two steps
 constexpr int kBN = 128;           // weight columns per CTA
 constexpr int kDequantWarps = 16;  // two groups of eight
-constexpr int kEpiWarp0 = kDequantWarps;  // 4 warps: TMEM lane quadrant = warp % 4
-constexpr int kProducerWarp = kEpiWarp0 + 4;
+constexpr int kProducerWarp = kDequantWarps;
 constexpr int kTokenWarp = kProducerWarp + 1;
 constexpr int kMmaWarp = kTokenWarp + 1;
-constexpr int kThreads = 32 * (kMmaWarp + 1);
+// epilogue warps: TMEM lane quadrant = warp % 4; with group scales on the sums two share a quadrant
+constexpr int kEpiWarp0 = kMmaWarp + 1;
+constexpr int epi_warps(bool sums) { return sums ? 8 : 4; }
+constexpr int threads(bool sums) { return 32 * (kEpiWarp0 + epi_warps(sums)); }
 constexpr uint32_t kSpinLimit = 1u << 24;
 
 struct TcParams {
@@ -237,6 +240,23 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
   else
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
 }
+// 32 lanes x 16 consecutive fp32 columns of TMEM <-> 16 registers per thread
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 // 32 lanes x 32 consecutive fp32 columns of TMEM -> 32 registers per thread
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
@@ -280,15 +300,19 @@ __device__ __forceinline__ uint32_t make_idesc(int m, int n) {
   return (1u << 4) | (f << 7) | (f << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-// Shared-memory plan.  TOK: token rows a CTA can stage per step.
-template <int F, int TOK>
+// Tokens of a tile at most, where group scales are applied to the sums (two buffers of group sums and the tile's
+// running sums in TMEM).
+__host__ __device__ constexpr int group_sums_tokens(int cg) { return cg == 1 ? 64 : 160; }
+
+// Shared-memory plan.  TOK: token rows a CTA can stage per step.  SUMS: group scales stay out of the weight ring.
+template <int F, int TOK, bool SUMS>
 struct TcCfg {
   using I = FmtInfo<F>;
   static constexpr int kTileBytes = 16 * 64 * I::kBits / 8;    // one packed 16 x 64 weight tile
   static constexpr int kWBytes = kRoundTiles * 2 * kTileBytes;  // 8 k-tiles x 2 column tiles
   // rows of scales (fp4: of byte pairs) a round can touch
   static constexpr int kSRow = 2 * kBN;
-  static constexpr int kSBytes = (F == kNV4 ? 4 : F == kMX4 ? 2 : kRoundTiles) * kSRow;
+  static constexpr int kSBytes = SUMS ? 0 : (F == kNV4 ? 4 : F == kMX4 ? 2 : kRoundTiles) * kSRow;
   static constexpr int kZRow = I::kZpF ? 2 * kBN : I::kZp ? kBN * I::kBits / 8 : 0;
   static constexpr int kWSlot = kWBytes + kSBytes + kRoundTiles * kZRow;  // a multiple of 128
   // a slot: token rows of the two steps, converted weights of the two steps
@@ -436,11 +460,22 @@ __device__ __forceinline__ uint32_t fp4_scale(uint32_t word, int byte) {
   }
 }
 
-template <typename T, int F, int CG, int TOK>
-__global__ void __launch_bounds__(kThreads, 1)
+// SUMS: group scales are applied to fp32 sums, as in the decode kernel, so that calls which either kernel may take
+// give results of one precision.  The MMAs take the exact codes, a group of k at a time into one of a ring of TMEM
+// buffers; the epilogue warps add scale x buffer to the tile's running sums (in registers, for pairs in TMEM) while
+// the next group is computed.  Groups of one step or of whole rounds only.  fp16 results that are not the correctly
+// rounded ones: 0.03 to 0.13 % over 2048 .. 8192 deep layers of every integer type (decode kernel 0.8 to 6 %, scaled
+// weights rounded to 16 bits 39 %).
+// What bounds it: the hand-overs.  A round of 4-bit weights takes 0.60 us at 16 rows (0.45 with scaled weights), 8-bit
+// 0.60 (0.56), two groups a round 0.80; pairs at 125 rows 0.69 (0.56).  Two terms per weight, the rounded product and
+// the rest, were as exact but doubled the operand traffic of shared memory, which bounds these shapes (0.65 to 0.8
+// us); with four epilogue warps, or a wait for every buffer, a round took 0.78 us.
+template <typename T, int F, int CG, int TOK, bool SUMS>
+__global__ void __launch_bounds__(threads(SUMS), 1)
 gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
-  using Cfg = TcCfg<F, TOK>;
+  using Cfg = TcCfg<F, TOK, SUMS>;
   using I = FmtInfo<F>;
+  static_assert(!SUMS || (!I::kFp4 && !I::kZpF && F != kF8), "sums of exact integer codes");
   constexpr int RING = Cfg::kRing, WD = Cfg::kWD, BITS = I::kBits;
   constexpr bool kPair = CG == 2;
   extern __shared__ unsigned char smem_raw[];
@@ -456,9 +491,15 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
   auto full_w = [&](int w) { return bars + 8 * (2 * RING + w); };
   auto empty_w = [&](int w) { return bars + 8 * (2 * RING + WD + w); };
   const uint32_t bars2 = bars + 8 * (2 * RING + 2 * WD);
+  // TMEM: accumulator buffers; SUMS of CTA pairs: then the running sums (of single CTAs they are in registers)
+  // buffers are given back REL at a time, so that the MMA warp rarely waits for one
+  constexpr int BUFS = SUMS && CG == 1 ? 8 : 2, REL = BUFS / 2;
+  constexpr uint32_t kBufCols = SUMS ? group_sums_tokens(CG) : CG * 128;
+  constexpr uint32_t kTmemCols = SUMS ? 512 : 2 * kBufCols;
+  static_assert((BUFS + (SUMS && CG == 2 ? 1 : 0)) * kBufCols <= kTmemCols, "TMEM");
   auto tmem_full = [&](int b) { return bars2 + 8 * b; };
-  auto tmem_empty = [&](int b) { return bars2 + 16 + 8 * b; };
-  const uint32_t tmem_slot = bars2 + 32;
+  auto tmem_empty = [&](int b) { return bars2 + 8 * (BUFS + b); };
+  const uint32_t tmem_slot = bars2 + 8 * (BUFS + 2);
 
   // the next kernel in the stream may be scheduled while this one runs (it waits for completion itself)
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
@@ -471,7 +512,7 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
   const int NT = p.n / 64;
   const int gb = p.group_blocks;
   const int steps = p.k / kBK;
-  constexpr uint32_t kTmemCols = 2 * CG * 128;
+  const int group_steps = gb / 4;  // SUMS: 1 or even
 
   if (threadIdx.x == 0) {
     s_abort = 0;
@@ -484,10 +525,8 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
       mbar_init(full_w(w), 1);
       mbar_init(empty_w(w), kDequantWarps / 2);
     }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(tmem_full(b), 1);
-      mbar_init(tmem_empty(b), 4 * CG);
-    }
+    for (int b = 0; b < BUFS; ++b) mbar_init(tmem_full(b), 1);
+    for (int b = 0; b < 2; ++b) mbar_init(tmem_empty(b), epi_warps(SUMS) * CG);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   if (warp == kMmaWarp) tmem_alloc<CG>(tmem_slot, kTmemCols);
@@ -511,7 +550,7 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
     Ring<WD> wr;
     bool ok = true;
     const int kt_all = p.k / 16;
-    const bool scales = I::kFp4 || !p.channelwise;
+    const bool scales = I::kFp4 || (!SUMS && !p.channelwise);
     const uint32_t bytes = Cfg::kWBytes + (scales ? (I::kFp4 ? Cfg::kSBytes : p.group_rows * Cfg::kSRow) : 0) +
                            p.group_rows * Cfg::kZRow;
     while (ok && sched.next(sg)) {
@@ -561,35 +600,76 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
     // the whole warp walks the loop, one elected lane issues
     if (rank == 0) {
       Ring<RING> ring;
-      int seg_i = 0;
+      int acc_i = 0;  // buffers filled so far
       bool ok = true;
       // the ring stays below 256 KB: slot offsets add up in the address field of the descriptors
       const uint32_t da0 = smem_desc_lo(a_slot(0)), db0 = smem_desc_lo(tok_slot(0));
       while (ok && sched.next(sg)) {
         const uint32_t idesc = make_idesc<T>(CG * 128, sched.template mma_n<CG>(sg));
-        const int buf = seg_i & 1;
-        if (!(ok = mbar_wait<kPair>(tmem_empty(buf), ((seg_i >> 1) & 1) ^ 1, (2 << 8) | 5, cta_abort, p.error))) break;
-        tc_fence_after();
-        const uint32_t d = tmem_base + buf * (CG * 128);
+        // a commit hands one buffer to the epilogue: the sums of the segment, or (SUMS) of each of its groups
+        uint32_t d = 0;
+        auto open = [&]() {
+          if (acc_i % REL == 0) {
+            if (!(ok = mbar_wait<kPair>(tmem_empty((acc_i / REL) & 1), ((acc_i / BUFS) & 1) ^ 1, (2 << 8) | 5, cta_abort, p.error)))
+              return;
+            tc_fence_after();
+          }
+          d = tmem_base + acc_i % BUFS * kBufCols;
+        };
+        // MMAs of a step; `fresh`: they begin a buffer
+        auto issue = [&](uint32_t a, uint32_t b, bool fresh) {
+#pragma unroll
+          for (int k16 = 0; k16 < 4; ++k16) umma_f16<CG>(d, a + 2 * k16, b + 2 * k16, kDescHi, idesc, k16 > 0 || !fresh);
+        };
+        constexpr uint32_t kA1 = Cfg::kABytes / 16, kB1 = Cfg::kTokBytes / 16;  // the second step of a slot
+        // rounds until the buffer is handed over (SUMS with groups of a single step: two buffers per round)
+        const int rounds_per_buf = SUMS ? group_steps / 2 : sg.r1 - sg.r0;
+        int left = SUMS && rounds_per_buf > 0 ? rounds_per_buf - sg.r0 % rounds_per_buf : sg.r1 - sg.r0;
+        bool fresh = true;
         for (int r = sg.r0; r < sg.r1; ++r) {
+          if (fresh) {
+            open();
+            if (!ok) break;
+          }
           if (!(ok = mbar_wait<kPair>(full(ring.i), ring.ph, (2 << 8) | 0, cta_abort, p.error))) break;
           tc_fence_after();
           const uint32_t da = da0 + ring.i * (Cfg::kSlot / 16), db = db0 + ring.i * (Cfg::kSlot / 16);
-          if (elect_one()) {
-#pragma unroll
-            for (int k16 = 0; k16 < 4; ++k16) umma_f16<CG>(d, da + 2 * k16, db + 2 * k16, kDescHi, idesc, k16 > 0 || r > sg.r0);
-            if (2 * r + 1 < steps) {
-#pragma unroll
-              for (int k16 = 0; k16 < 4; ++k16)
-                umma_f16<CG>(d, da + Cfg::kABytes / 16 + 2 * k16, db + Cfg::kTokBytes / 16 + 2 * k16, kDescHi, idesc, 1);
+          const bool second = 2 * r + 1 < steps;
+          if (!SUMS || rounds_per_buf > 0) {
+            const bool last = --left == 0 || r + 1 == sg.r1;
+            if (elect_one()) {
+              issue(da, db, fresh);
+              if (second) issue(da + kA1, db + kB1, false);
+              umma_commit<CG>(empty(ring.i));  // slot reusable once these MMAs have read it
+              if (last) umma_commit<CG>(tmem_full(acc_i % BUFS));
             }
-            umma_commit<CG>(empty(ring.i));  // slot reusable once these MMAs have read it
-            if (r + 1 == sg.r1) umma_commit<CG>(tmem_full(buf));
+            fresh = last;
+            if (last) {
+              ++acc_i;
+              left = rounds_per_buf;
+            }
+          } else {
+            if (elect_one()) {
+              issue(da, db, true);
+              umma_commit<CG>(tmem_full(acc_i % BUFS));
+              if (!second) umma_commit<CG>(empty(ring.i));
+            }
+            __syncwarp();
+            ++acc_i;
+            if (second) {
+              open();
+              if (!ok) break;
+              if (elect_one()) {
+                issue(da + kA1, db + kB1, true);
+                umma_commit<CG>(tmem_full(acc_i % BUFS));
+                umma_commit<CG>(empty(ring.i));
+              }
+              ++acc_i;
+            }
           }
           __syncwarp();
           ring.next();
         }
-        ++seg_i;
       }
     } else {
       Ring<RING> ring;
@@ -651,7 +731,7 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
             sc2[st][1] = lds32(src + 4);
           } else {
             const int row = fixed_row ? (st ? row1 : row0) : (r * kRoundTiles + rkt) / gb - (r * kRoundTiles) / gb;
-            if (!p.channelwise) {
+            if (!SUMS && !p.channelwise) {
               const uint4 s4 = lds128(wslot + Cfg::kWBytes + row * Cfg::kSRow + nt * 128 + c8 * 16);
               sc2[st][0] = s4.x; sc2[st][1] = s4.y; sc2[st][2] = s4.z; sc2[st][3] = s4.w;
             }
@@ -748,7 +828,7 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
             if constexpr (I::kFp4 || I::kZpF) {
               convert_all(std::true_type{});
             } else {
-              if (p.channelwise) convert_all(std::false_type{});
+              if (SUMS || p.channelwise) convert_all(std::false_type{});
               else convert_all(std::true_type{});
             }
           }
@@ -769,41 +849,47 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
     const int quad = warp & 3;  // TMEM lanes 32 quad .. 32 quad + 31
     const uint32_t te0 = kPair ? mapa(tmem_empty(0), 0) : tmem_empty(0);
     uint16_t* C = static_cast<uint16_t*>(p.c);
-    int seg_i = 0;
+    int acc_i = 0;  // buffers read so far
     bool ok = true;
     // C, the partial sums and the counters may still be in use by the kernel in front
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
     while (ok && sched.next(sg)) {
-      const int buf = seg_i & 1;
-      if (!(ok = mbar_wait<kPair, 100>(tmem_full(buf), (seg_i >> 1) & 1, (4 << 8) | 4, cta_abort, p.error))) break;
-      ++seg_i;
-      tc_fence_after();
       const int n = (sg.n_tile * CG + (int)rank) * kBN + quad * 32 + lane;  // this lane's output column
       const bool n_ok = n < p.n;                                            // uniform per warp: N % 64 == 0
-      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * (CG * 128);
+      const uint32_t lanes = tmem_base + ((uint32_t)(quad * 32) << 16);
+      uint32_t taddr = 0;
+      // wait for the next buffer
+      auto take = [&]() {
+        const int buf = acc_i % BUFS;
+        if (!(ok = mbar_wait<kPair, SUMS ? 0 : 100>(tmem_full(buf), (acc_i / BUFS) & 1, (4 << 8) | 4, cta_abort, p.error))) return;
+        ++acc_i;
+        tc_fence_after();
+        taddr = lanes + buf * kBufCols;
+      };
       float cs = 1.f, bs = 0.f;
       if (n_ok) {
-        if (p.channelwise)
+        if (!SUMS && p.channelwise)
           cs = Pair<T>::to_float(static_cast<const uint16_t*>(p.scales)[(size_t)sg.expert * p.s_stride + single_perm_pos(n)]) *
                p.chan_factor;
         if (F == kNV4) cs = Pair<T>::to_float(*static_cast<const uint16_t*>(p.global_scale));
         if (p.bias)
           bs = Pair<T>::to_float(static_cast<const uint16_t*>(p.bias)[(size_t)sg.expert * p.bias_stride + single_perm_pos(n)]);
       }
-      // Scale, bias, rounding and store of 32 consecutive tokens of the warp's 32 columns.  Lanes pair
+      // Scale, bias, rounding and store of COUNT (16 or 32) consecutive tokens of the warp's 32 columns.  Lanes pair
       // up: of two neighbouring tokens the even lane stores the first for both lanes' columns, the odd
       // lane the second, so that a store instruction writes 64 B of two rows.
-      auto store32 = [&](int t0, const float (&v)[32]) {
+      auto store = [&](int t0, const auto& v, auto count_c) {
+        constexpr int COUNT = decltype(count_c)::value;
         int my_id = 0;
         float my_w = 1.f;
         if (p.ids) {
-          my_id = t0 + lane < sg.rows ? p.ids[sg.tok0 + t0 + lane] : p.out_rows;
+          my_id = lane < COUNT && t0 + lane < sg.rows ? p.ids[sg.tok0 + t0 + lane] : p.out_rows;
           if (p.row_weights && my_id < p.out_rows) my_w = p.row_weights[my_id];
         }
         const bool odd = lane & 1;
-        uint32_t word[16];
+        uint32_t word[COUNT / 2];
 #pragma unroll
-        for (int t = 0; t < 32; t += 2) {
+        for (int t = 0; t < COUNT; t += 2) {
           float a = v[t] * cs + bs, b = v[t + 1] * cs + bs;
           if (p.ids) {
             a *= __shfl_sync(~0u, my_w, t);
@@ -817,57 +903,143 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         if (!p.scatter) {
           uint16_t* dst = C + (size_t)(sg.tok0 + t1) * p.n + (n & ~1);
           const size_t step2 = (size_t)2 * p.n;
-          if (t0 + 32 <= sg.rows) {
+          if (t0 + COUNT <= sg.rows) {
 #pragma unroll
-            for (int t = 0; t < 32; t += 2, dst += step2) *reinterpret_cast<uint32_t*>(dst) = word[t / 2];
+            for (int t = 0; t < COUNT; t += 2, dst += step2) *reinterpret_cast<uint32_t*>(dst) = word[t / 2];
           } else {
 #pragma unroll
-            for (int t = 0; t < 32; t += 2, dst += step2)
+            for (int t = 0; t < COUNT; t += 2, dst += step2)
               if (t1 + t < sg.rows) *reinterpret_cast<uint32_t*>(dst) = word[t / 2];
           }
         } else {
 #pragma unroll
-          for (int t = 0; t < 32; t += 2) {
+          for (int t = 0; t < COUNT; t += 2) {
             const int id = __shfl_sync(~0u, my_id, t + (odd ? 1 : 0));
             if (t1 + t < sg.rows && id < p.out_rows)
               *reinterpret_cast<uint32_t*>(C + (size_t)id * p.n + (n & ~1)) = word[t / 2];
           }
         }
       };
-      auto release = [&]() {
+      auto release = [&]() {  // the buffer taken last, with the REL - 1 before it
+        if (acc_i % REL != 0) return;
+        const int half = (acc_i / REL - 1) & 1;
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
-          if (kPair && rank != 0) mbar_arrive_cluster(te0 + 8 * buf);
-          else mbar_arrive(tmem_empty(buf));
+          if (kPair && rank != 0) mbar_arrive_cluster(te0 + 8 * half);
+          else mbar_arrive(tmem_empty(half));
         }
       };
-      if (!sg.shared) {
+      const size_t slot_floats = (size_t)p.tn * kBN;  // partial sums, token-major: a warp writes 128 B per token
+      float* mine = p.partials + ((size_t)sg.slot * CG + rank) * slot_floats + quad * 32 + lane;
+      if constexpr (!SUMS) {
+        take();
+        if (!ok) break;
         for (int t0 = 0; t0 < sg.rows; t0 += 32) {
           uint32_t r[32];
           tmem_ld32(taddr + t0, r);
           tmem_ld_wait();
-          if (n_ok) {
-            float v[32];
+          if (!sg.shared) {
+            if (n_ok) {
+              float v[32];
 #pragma unroll
-            for (int t = 0; t < 32; ++t) v[t] = __uint_as_float(r[t]);
-            store32(t0, v);
+              for (int t = 0; t < 32; ++t) v[t] = __uint_as_float(r[t]);
+              store(t0, v, std::integral_constant<int, 32>{});
+            }
+          } else {
+#pragma unroll
+            for (int t = 0; t < 32; ++t)
+              if (t0 + t < sg.rows) __stcg(mine + (size_t)(t0 + t) * kBN, __uint_as_float(r[t]));
           }
         }
         release();
       } else {
-        // partial sums, token-major: a warp writes 128 B per token
-        const size_t slot_floats = (size_t)p.tn * kBN;
-        float* mine = p.partials + ((size_t)sg.slot * CG + rank) * slot_floats + quad * 32 + lane;
-        for (int t0 = 0; t0 < sg.rows; t0 += 32) {
-          uint32_t r[32];
-          tmem_ld32(taddr + t0, r);
-          tmem_ld_wait();
+        // scale x group sums into the running sums, a group at a time.  The two warps of a quadrant take the lower
+        // and the upper tokens.  Scales are brought into L2 at the start of the segment, a lane a row, and into a
+        // register one group ahead (the latency of memory showed otherwise: 8192 x 18944 at 16 rows 47 us against 41).
+        const int step0 = 2 * sg.r0, step1 = min(steps, 2 * sg.r1);
+        const int g0 = step0 / group_steps, groups = (step1 - 1) / group_steps + 1 - g0;
+        const uint16_t* src = static_cast<const uint16_t*>(p.scales) + ((size_t)sg.expert * p.groups + g0) * p.n + grouped_perm_pos(n);
+        const int half = CG == 1 ? 32 : (sg.rows + 31) / 32 * 16;
+        const int t_lo = warp >= kEpiWarp0 + 4 ? half : 0, t_hi = min(sg.rows, t_lo + half);
+        const uint32_t sums = lanes + BUFS * kBufCols;
+        float acc[CG == 1 ? 32 : 1];  // CG == 1: the running sums
+        if (n_ok)
+          for (int c = lane; c < groups; c += 32) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(src + (size_t)c * p.n));
+        auto group = [&](float scale, auto first_c) {
+          constexpr bool FIRST = decltype(first_c)::value;
+          take();
+          if (!ok) return;
+          if constexpr (CG == 1) {
 #pragma unroll
-          for (int t = 0; t < 32; ++t)
-            if (t0 + t < sg.rows) __stcg(mine + (size_t)(t0 + t) * kBN, __uint_as_float(r[t]));
+            for (int b = 0; b < 2; ++b) {
+              if (t_lo + 16 * b >= t_hi) break;
+              uint32_t r[16];
+              tmem_ld16(taddr + t_lo + 16 * b, r);
+              tmem_ld_wait();
+#pragma unroll
+              for (int t = 0; t < 16; ++t)
+                acc[16 * b + t] = fmaf(scale, __uint_as_float(r[t]), FIRST ? 0.f : acc[16 * b + t]);
+            }
+          } else {
+            for (int t0 = t_lo; t0 < t_hi; t0 += 16) {
+              uint32_t r[16], a[16];
+              tmem_ld16(taddr + t0, r);
+              if constexpr (!FIRST) tmem_ld16(sums + t0, a);
+              tmem_ld_wait();
+#pragma unroll
+              for (int t = 0; t < 16; ++t)
+                a[t] = __float_as_uint(fmaf(scale, __uint_as_float(r[t]), FIRST ? 0.f : __uint_as_float(a[t])));
+              tmem_st16(sums + t0, a);
+            }
+            tmem_st_wait();
+          }
+          release();
+        };
+        auto scale_of = [&](int c) { return n_ok && c < groups ? __ldg(src + (size_t)c * p.n) : (uint16_t)0; };
+        uint16_t ahead[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ahead[i] = scale_of(i + 1);
+        group(Pair<T>::to_float(scale_of(0)), std::true_type{});
+        for (int c0 = 1; c0 < groups && ok; c0 += 4) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (c0 + i >= groups || !ok) break;
+            const float scale = Pair<T>::to_float(ahead[i]);
+            ahead[i] = scale_of(c0 + i + 4);
+            group(scale, std::false_type{});
+          }
         }
-        release();
+        if (!ok) break;
+        auto finish16 = [&](int t0, const float (&v)[16]) {
+          if (!sg.shared) {
+            if (n_ok) store(t0, v, std::integral_constant<int, 16>{});
+          } else {
+#pragma unroll
+            for (int t = 0; t < 16; ++t)
+              if (t0 + t < sg.rows) __stcg(mine + (size_t)(t0 + t) * kBN, v[t]);
+          }
+        };
+        if constexpr (CG == 1) {
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            if (t_lo + 16 * b >= t_hi) break;
+            float v[16];
+#pragma unroll
+            for (int t = 0; t < 16; ++t) v[t] = acc[16 * b + t];
+            finish16(t_lo + 16 * b, v);
+          }
+        } else {
+          for (int t0 = t_lo; t0 < t_hi; t0 += 16) {
+            uint32_t r[16];
+            tmem_ld16(sums + t0, r);
+            tmem_ld_wait();
+            float v[16];
+#pragma unroll
+            for (int t = 0; t < 16; ++t) v[t] = __uint_as_float(r[t]);
+            finish16(t0, v);
+          }
+        }
       }
     }
   }

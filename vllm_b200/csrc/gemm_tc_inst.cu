@@ -15,11 +15,11 @@ using InstT = __nv_bfloat16;
 using InstT = half;
 #endif
 
-template <typename T, int F, int CG, int TOK>
+template <typename T, int F, int CG, int TOK, bool SUMS = false>
 static int launch_one(const TcMaps& maps, const TcParams& p, bool pdl, cudaStream_t stream) {
-  using Cfg = TcCfg<F, TOK>;
+  using Cfg = TcCfg<F, TOK, SUMS>;
   static_assert(Cfg::kWD >= 2, "weight ring too shallow");
-  auto kernel = gemm_tc_kernel<T, F, CG, TOK>;
+  auto kernel = gemm_tc_kernel<T, F, CG, TOK, SUMS>;
   static bool attr_done[64] = {};  // per device; benign race: the call is idempotent
   int dev = 0;
   B200Q_CUDA_OK(cudaGetDevice(&dev));
@@ -29,7 +29,7 @@ static int launch_one(const TcMaps& maps, const TcParams& p, bool pdl, cudaStrea
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(p.workers * CG));
-  cfg.blockDim = dim3(kThreads);
+  cfg.blockDim = dim3(threads(SUMS));
   cfg.dynamicSmemBytes = Cfg::kSmemBytes;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
@@ -54,16 +54,27 @@ static int launch_one(const TcMaps& maps, const TcParams& p, bool pdl, cudaStrea
 }
 
 template <typename T, int F>
-int launch_format(const TcMaps& maps, const TcParams& p, int cg, bool pdl, cudaStream_t stream);
+int launch_format(const TcMaps& maps, const TcParams& p, int cg, bool sums, bool pdl, cudaStream_t stream);
 
-#define B200Q_TC_FORMAT(F)                                                                                  \
-  template <>                                                                                               \
-  int launch_format<InstT, F>(const TcMaps& maps, const TcParams& p, int cg, bool pdl, cudaStream_t stream) { \
-    if (cg == 2)                                                                                            \
-      return p.box <= 96 ? launch_one<InstT, F, 2, 96>(maps, p, pdl, stream)                                \
-                         : launch_one<InstT, F, 2, 128>(maps, p, pdl, stream);                              \
-    return p.box <= 64 ? launch_one<InstT, F, 1, 64>(maps, p, pdl, stream)                                  \
-                       : launch_one<InstT, F, 1, 128>(maps, p, pdl, stream);                                \
+template <typename T, int F>
+static int launch_sums(const TcMaps& maps, const TcParams& p, int cg, bool pdl, cudaStream_t stream) {
+  if constexpr (F == kU4B8 || F == kU4Z || F == kU8B128 || F == kU8Z) {
+    if (p.tn <= group_sums_tokens(cg))
+      return cg == 2 ? launch_one<T, F, 2, 96, true>(maps, p, pdl, stream) : launch_one<T, F, 1, 64, true>(maps, p, pdl, stream);
+  }
+  set_error("group scales on the sums: weight format %d, %d tokens per tile", F, p.tn);
+  return B200Q_EUNSUPPORTED;
+}
+
+#define B200Q_TC_FORMAT(F)                                                                                           \
+  template <>                                                                                                        \
+  int launch_format<InstT, F>(const TcMaps& maps, const TcParams& p, int cg, bool sums, bool pdl, cudaStream_t stream) { \
+    if (sums) return launch_sums<InstT, F>(maps, p, cg, pdl, stream);                                                \
+    if (cg == 2)                                                                                                     \
+      return p.box <= 96 ? launch_one<InstT, F, 2, 96>(maps, p, pdl, stream)                                         \
+                         : launch_one<InstT, F, 2, 128>(maps, p, pdl, stream);                                       \
+    return p.box <= 64 ? launch_one<InstT, F, 1, 64>(maps, p, pdl, stream)                                           \
+                       : launch_one<InstT, F, 1, 128>(maps, p, pdl, stream);                                         \
   }
 
 B200Q_TC_FORMAT(INST_F0)

@@ -11,6 +11,8 @@ int launch_tc_moe(const void* a, int64_t rows, const uint32_t* b, const void* sc
                   int64_t num_groups, int pairs, int box, const int4* tile_list, const int32_t* tile_count,
                   const int32_t* ids, int scatter, const float* row_weights, cudaStream_t stream);
 bool tc_gemm_supported(int64_t size_n, int64_t size_k, int gm);
+bool tc_group_sums_supported(int64_t group_size);
+int tc_group_sums_rows(int cg);
 
 namespace moe {
 
@@ -226,16 +228,32 @@ struct Plan {
   int64_t len;     // sorted ids (with padding: a whole number of blocks)
 };
 
-// Rows per expert on average decide: the decode kernel reads 4-bit weights at 3.2 TB/s for blocks of 8 and
-// at 2.0 for 16, the tensor-core kernel at about 2.0 up to 64 rows (8-bit: 3.7 against 2.7), pairs take
-// over where a tile is wide enough for the MMAs to matter.
-static Plan make_plan(int64_t rows, int64_t experts, int64_t global_experts, int64_t k, int64_t n, int bits, bool tc_ok) {
+// Whether the tensor-core kernel takes the GEMMs, by rows per expert on average.  `group`: the smaller group size of
+// the two matrices, 0 when both have a scale per column.  Lines and times (us, a layer of eight experts, top-2,
+// decode kernel / tensor cores; 4096 / 14336 unless stated):
+//   scales per column    4-bit from 7 rows, 8-bit always
+//   groups of 128, up    4-bit from 14 rows (12 rows 317 / 399, 14 rows 364 / 403, 16 rows 502 / 404), 8-bit from two
+//                        (one row 356 / 356, two 408 / 379, four 429 / 398; 2048 / 1408, two rows 44.6 / 45.2)
+//   groups of 64         two buffers of group sums a round: 4-bit from 28 rows (24 rows 536 / 572, 40 rows 975 / 587),
+//                        with zero-points or 8 bits from 14 (16 rows 647 / 610 and 596 / 562, 12 rows 399 / 555)
+//   other groups         never: the group sums come in whole steps
+static bool on_tensor_cores(int64_t rows, int64_t experts, int64_t k, int64_t n, int bits, bool zp, int64_t group) {
+  if (!tc_gemm_supported(2 * n, k, kChannel) || !tc_gemm_supported(k, n, kChannel)) return false;
+  const double avg = (double)rows / (double)experts;
+  if (group == 0) return bits == 8 || avg > 7.0;
+  if (!tc_group_sums_supported(group)) return false;
+  if (group < 128) return avg >= (bits == 4 && !zp ? 28.0 : 14.0);
+  return avg >= (bits == 4 ? 14.0 : 2.0);
+}
+
+static Plan make_plan(bool tc, int64_t rows, int64_t experts, int64_t global_experts, int64_t group) {
   Plan pl = {};
   const double avg = (double)rows / (double)experts;
-  pl.tc = tc_ok && tc_gemm_supported(2 * n, k, kChannel) && tc_gemm_supported(k, n, kChannel) && (bits == 8 || avg > 7.0);
+  pl.tc = tc;
   if (pl.tc) {
+    // pairs where a tile is wide enough for the MMAs to matter
     pl.pairs = avg > 40.0;
-    pl.box = !pl.pairs ? 64 : avg > 160.0 ? 128 : 96;
+    pl.box = group > 0 ? tc_group_sums_rows(pl.pairs ? 2 : 1) / (pl.pairs ? 2 : 1) : !pl.pairs ? 64 : avg > 160.0 ? 128 : 96;
     pl.max_rows = pl.box * (pl.pairs ? 2 : 1);
     pl.len = rows;
   } else {
@@ -293,10 +311,11 @@ extern "C" size_t b200q_fused_marlin_moe_scratch_bytes(int64_t size_m, int64_t t
                                                        int64_t global_experts, int64_t size_k, int64_t size_n, int bits) {
   if (size_m <= 0 || top_k <= 0 || num_experts <= 0) return 256;
   const int64_t rows = size_m * top_k;
-  // either kind of plan may be taken (the tensor-core kernel has conditions of its own)
+  // either kernel may be taken (alignment and the groups decide, too); a tile list is longest with the smallest tiles
+  (void)bits;
   size_t most = 0;
-  for (int tc = 0; tc < 2; ++tc) {
-    const moe::Plan pl = moe::make_plan(rows, num_experts, global_experts, size_k, size_n, bits, tc != 0);
+  for (int tc = 0; tc < 3; ++tc) {
+    const moe::Plan pl = moe::make_plan(tc != 0, rows, num_experts, global_experts, tc == 2 ? 64 : 0);
     const size_t b = (size_t)moe::make_layout(pl, rows, global_experts, size_k, size_n).bytes;
     if (b > most) most = b;
   }
@@ -333,7 +352,13 @@ extern "C" int b200q_fused_marlin_moe(
   const bool aligned = ((reinterpret_cast<uintptr_t>(w1) | reinterpret_cast<uintptr_t>(w2) | reinterpret_cast<uintptr_t>(w1_scale) |
                          reinterpret_cast<uintptr_t>(w2_scale) | reinterpret_cast<uintptr_t>(w1_zeros) |
                          reinterpret_cast<uintptr_t>(w2_zeros)) & 15) == 0;
-  const moe::Plan pl = moe::make_plan(rows, num_experts, global_experts, size_k, size_n, bits, aligned);
+  B200Q_REQUIRE(groups1 >= 1 && groups2 >= 1 && size_k % groups1 == 0 && size_n % groups2 == 0, B200Q_EINVAL,
+                "moe: invalid number of groups (%lld, %lld)", (long long)groups1, (long long)groups2);
+  const int64_t group1 = groups1 > 1 ? size_k / groups1 : 0, group2 = groups2 > 1 ? size_n / groups2 : 0;
+  const bool groups_fit = (group1 == 0 || tc_group_sums_supported(group1)) && (group2 == 0 || tc_group_sums_supported(group2));
+  const int64_t group = group1 == 0 ? group2 : group2 == 0 ? group1 : group1 < group2 ? group1 : group2;
+  const bool tc = aligned && groups_fit && moe::on_tensor_cores(rows, num_experts, size_k, size_n, bits, zp, group);
+  const moe::Plan pl = moe::make_plan(tc, rows, num_experts, global_experts, group);
   const moe::Layout l = moe::make_layout(pl, rows, global_experts, size_k, size_n);
   B200Q_REQUIRE((int64_t)scratch_bytes >= l.bytes && (reinterpret_cast<uintptr_t>(scratch) & 255) == 0, B200Q_ESCRATCH,
                 "moe: scratch of %zu bytes is below the required %lld", scratch_bytes, (long long)l.bytes);
