@@ -233,3 +233,53 @@ def test_moe_align_block_size_torch_matches_reference_golden():
         assert int(n[0]) == int(g[f"num_{i}"].reshape(-1)[0]), i
         assert np.array_equal(s.numpy(), g[f"sorted_{i}"]), i
         assert np.array_equal(ex.numpy(), g[f"experts_{i}"]), i
+
+
+@pytest.mark.parametrize("kind", ["parameter", "none", "parametrization", "buffer", "property", "attribute"])
+@pytest.mark.parametrize("row_parallel", [False, True])
+def test_layer_bias_is_whatever_the_layer_calls_bias(kind, row_parallel):
+    import torch
+    from torch.nn.utils import parametrize
+    from vllm_b200.linear import ColumnParallelLinear, RowParallelLinear
+
+    class Method:
+        def create_weights(self, layer, **kw):
+            pass
+
+        def apply(self, layer, x, bias=None):
+            return bias
+
+    class Config:
+        def get_quant_method(self, layer, prefix):
+            return Method()
+
+    class Twice(torch.nn.Module):
+        def forward(self, t):
+            return 2 * t
+
+    base = RowParallelLinear if row_parallel else ColumnParallelLinear
+    make = lambda cls, bias: cls(8, 4, bias=bias, quant_config=Config(), params_dtype=torch.float32, tp_rank=0, tp_size=1)
+    value = torch.arange(4.0)
+    layer = make(base, kind in ("parameter", "parametrization"))
+    if kind in ("parameter", "parametrization"):
+        layer.bias.data.copy_(value)
+        want = value
+        if kind == "parametrization":
+            layer.bias = torch.nn.Parameter(value.clone())
+            parametrize.register_parametrization(layer, "bias", Twice())
+            want = 2 * value
+    elif kind == "none":
+        want = None
+    elif kind == "buffer":
+        del layer.bias
+        layer.register_buffer("bias", value)
+        want = value
+    elif kind == "property":
+        del layer.bias
+        layer.__class__ = type("WithBias", (base,), {"bias": property(lambda self: value + 1)})
+        want = value + 1
+    else:
+        layer.__dict__["bias"] = value
+        want = value
+    got = layer(torch.zeros(1, 8))
+    assert (got is None and want is None) or torch.equal(got, want)
