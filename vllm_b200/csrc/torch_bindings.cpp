@@ -56,22 +56,43 @@ bool decode_type(int64_t id, TypeInfo* t) {
 
 // Scratch of the GEMM: fp32 partial sums, and the gathered activations of act-order
 // layers.  One grow-only buffer per (device, stream): calls on one stream are ordered,
-// so they can share it; calls on different streams must not.  A call that is being captured
-// gets memory of its own from the graph's pool (`own`): the shared buffer may be replaced by a larger
+// so they can share it; calls on different streams must not.  A call launches several kernels that use it, so a
+// lease lasts until the last of them is in the stream: with two threads on one stream the kernels of one call would
+// else come between those of the other, and a larger call would replace the buffer under it.  A call that is being
+// captured gets memory of its own from the graph's pool: the shared buffer may be replaced by a larger
 // one, and released, while the graph is still in use.
-at::Tensor& scratch_for(const at::Device& dev, cudaStream_t stream, size_t bytes, at::Tensor& own) {
-  static std::mutex mu;
-  static std::unordered_map<uint64_t, at::Tensor> cache;
-  const auto make = [&] { return at::empty({(int64_t)bytes}, at::TensorOptions().dtype(at::kByte).device(dev)); };
-  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) cudaGetLastError();
-  if (status != cudaStreamCaptureStatusNone) return own = make();
-  const uint64_t key = ((uint64_t)(uintptr_t)stream << 8) ^ (uint64_t)(dev.index() & 0xff);
-  std::lock_guard<std::mutex> lock(mu);
-  at::Tensor& t = cache[key];
-  if (!t.defined() || (size_t)t.numel() < bytes) t = make();
-  return t;
-}
+class ScratchLease {
+ public:
+  ScratchLease(const at::Device& dev, cudaStream_t stream, size_t bytes) {
+    const auto make = [&] { return at::empty({(int64_t)bytes}, at::TensorOptions().dtype(at::kByte).device(dev)); };
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) cudaGetLastError();
+    if (status != cudaStreamCaptureStatusNone) {
+      t_ = make();
+      return;
+    }
+    Shared& shared = shared_for(((uint64_t)(uintptr_t)stream << 8) ^ (uint64_t)(dev.index() & 0xff));
+    lock_ = std::unique_lock<std::mutex>(shared.mu);
+    if (!shared.t.defined() || (size_t)shared.t.numel() < bytes) shared.t = make();
+    t_ = shared.t;
+  }
+  void* data() const { return t_.data_ptr(); }
+  size_t bytes() const { return (size_t)t_.numel(); }
+
+ private:
+  struct Shared {
+    std::mutex mu;
+    at::Tensor t;
+  };
+  static Shared& shared_for(uint64_t key) {
+    static std::mutex mu;
+    static std::unordered_map<uint64_t, Shared> all;  // (entries stay where they are when the map grows)
+    std::lock_guard<std::mutex> lock(mu);
+    return all[key];
+  }
+  at::Tensor t_;
+  std::unique_lock<std::mutex> lock_;
+};
 
 struct GemmArgs {
   const void *a, *scales, *bias;
@@ -266,19 +287,18 @@ at::Tensor gptq_marlin_gemm(at::Tensor& a, std::optional<at::Tensor> c_or_none,
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream(a.get_device());
   const size_t nbytes =
       b200q_marlin_gemm_preferred_scratch_bytes(size_m, size_n, size_k, g.act_order ? 1 : 0);
-  at::Tensor own;
-  at::Tensor& scratch = scratch_for(a.device(), stream, nbytes, own);
+  const ScratchLease scratch(a.device(), stream, nbytes);
   int rc;
   if (g.fp4_scales != 0) {
     TORCH_CHECK(g.zeros == nullptr && !g.act_order,
                 "float4_e2m1f weights take neither zero-points nor act_order");
     rc = b200q_marlin_gemm_fp4(g.a, g.lda, g.b, g.scales, g.global_scale, g.fp4_scales, g.bias,
-                               c.data_ptr(), scratch.data_ptr(), (size_t)scratch.numel(),
+                               c.data_ptr(), scratch.data(), scratch.bytes(),
                                workspace.data_ptr<int32_t>(), workspace.numel(), g.dtype, size_m,
                                size_n, size_k, g.num_groups, stream);
   } else {
     rc = b200q_marlin_gemm(g.a, g.lda, g.b, g.scales, g.zeros, g.g_idx, g.perm, g.bias,
-                           c.data_ptr(), scratch.data_ptr(), (size_t)scratch.numel(),
+                           c.data_ptr(), scratch.data(), scratch.bytes(),
                            workspace.data_ptr<int32_t>(), workspace.numel(), b_q_type, g.dtype,
                            size_m, size_n, size_k, g.num_groups, g.flags, stream);
   }
@@ -316,11 +336,10 @@ at::Tensor gptq_marlin_gemm_all_reduce(
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream(a.get_device());
   const size_t nbytes =
       b200q_marlin_gemm_preferred_scratch_bytes(size_m, size_n, size_k, g.act_order ? 1 : 0);
-  at::Tensor own;
-  at::Tensor& scratch = scratch_for(a.device(), stream, nbytes, own);
+  const ScratchLease scratch(a.device(), stream, nbytes);
   const int rc = b200q_marlin_gemm_all_reduce(
-      g.a, g.lda, g.b, g.scales, g.zeros, g.g_idx, g.perm, g.bias, c.data_ptr(), scratch.data_ptr(),
-      (size_t)scratch.numel(), workspace.data_ptr<int32_t>(), workspace.numel(), b_q_type, g.dtype,
+      g.a, g.lda, g.b, g.scales, g.zeros, g.g_idx, g.perm, g.bias, c.data_ptr(), scratch.data(),
+      scratch.bytes(), workspace.data_ptr<int32_t>(), workspace.numel(), b_q_type, g.dtype,
       size_m, size_n, size_k, g.num_groups, g.flags,
       reinterpret_cast<void* const*>(peer_ptrs.data_ptr<int64_t>()),
       reinterpret_cast<uint32_t*>(state.data_ptr<int32_t>()), (int)rank, (int)world,
