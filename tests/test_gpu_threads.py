@@ -43,3 +43,46 @@ def test_threads_share_a_stream():
     for t in threads:
         t.join()
     assert not wrong
+
+
+def test_direct_call_lets_other_threads_run():
+    """While the direct call allocates and launches (and waits for room in the launch queue) another Python thread
+    gets the interpreter.  With a switch interval of minutes it does so only when the call gives it up."""
+    import sys
+    import time
+
+    import torch
+    from vllm_b200 import _custom_ops as ops
+    from vllm_b200 import marlin_utils as mu
+    M, K, N = 4096, 8192, 128
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    q = torch.randint(-2**31, 2**31 - 1, (K // 16, N * 2), dtype=torch.int32, device="cuda", generator=gen)
+    s = (torch.rand((K // 128, N), device="cuda", generator=gen) * 0.018 + 0.002).half()
+    a = torch.randn((M, K), device="cuda", dtype=torch.float16, generator=gen)
+    e = torch.empty(0, dtype=torch.int32, device="cuda")
+    args = (a, q, None, s, None, e, e, e, mu.marlin_make_workspace_new(torch.device("cuda")), mu.scalar_types.uint4b8.id,
+            -1, N, K, ops.K_FULL)
+    assert ops._linear(*args) is not None
+    turns, stop = [0], threading.Event()
+
+    def other():
+        while not stop.is_set():
+            turns[0] += 1
+            time.sleep(0)       # gives the interpreter back
+
+    interval = sys.getswitchinterval()
+    thread = threading.Thread(target=other)
+    try:
+        sys.setswitchinterval(600)
+        thread.start()
+        outs = [None] * 3000    # more calls than the launch queue holds; kept, since freeing a tensor may switch threads
+        before = turns[0]
+        for i in range(len(outs)):
+            outs[i] = ops._linear(*args)
+        during = turns[0] - before
+    finally:
+        sys.setswitchinterval(interval)
+        stop.set()
+        thread.join()
+    torch.cuda.synchronize()
+    assert during > 0

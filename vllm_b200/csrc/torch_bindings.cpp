@@ -635,6 +635,13 @@ bool optional_tensor(PyObject* o, std::optional<at::Tensor>* t) {
   return true;
 }
 
+// Lets other Python threads run, as the operator's own binding does: allocation may wait for memory and a launch
+// for room in the queue, and a host callback in the stream may need the interpreter before that comes.
+struct WithoutGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~WithoutGil() { PyEval_RestoreThread(state); }
+};
+
 PyObject* py_linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(nargs == 14, "linear takes 14 arguments");
@@ -653,15 +660,18 @@ PyObject* py_linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
                 size_n = PyLong_AsLongLong(args[11]), size_k = PyLong_AsLongLong(args[12]);
   const long flags = PyLong_AsLong(args[13]);  // 1: is_k_full, 2: is_zp_float
   if (PyErr_Occurred()) return nullptr;
-  at::Tensor a = x.dim() == 2 ? x : x.reshape({-1, x.size(-1)});
-  const int64_t rows = size_m < 0 ? a.size(0) : size_m;
-  at::Tensor w = THPVariable_Unpack(args[1]), s = THPVariable_Unpack(args[3]), ws = THPVariable_Unpack(args[8]);
-  at::Tensor c = gptq_marlin_gemm(a, std::nullopt, w, bias, s, global_scale, zeros, g_idx, perm, ws, type_id, rows, size_n,
-                                  size_k, flags & 1, false, true, (flags & 2) != 0);
-  if (x.dim() != 2) {
-    c10::SmallVector<int64_t, 6> shape(x.sizes().begin(), x.sizes().end());
-    shape.back() = size_n;
-    c = c.view(shape);
+  at::Tensor w = THPVariable_Unpack(args[1]), s = THPVariable_Unpack(args[3]), ws = THPVariable_Unpack(args[8]), c;
+  {
+    const WithoutGil others_run;
+    at::Tensor a = x.dim() == 2 ? x : x.reshape({-1, x.size(-1)});
+    const int64_t rows = size_m < 0 ? a.size(0) : size_m;
+    c = gptq_marlin_gemm(a, std::nullopt, w, bias, s, global_scale, zeros, g_idx, perm, ws, type_id, rows, size_n, size_k,
+                         flags & 1, false, true, (flags & 2) != 0);
+    if (x.dim() != 2) {
+      c10::SmallVector<int64_t, 6> shape(x.sizes().begin(), x.sizes().end());
+      shape.back() = size_n;
+      c = c.view(shape);
+    }
   }
   return THPVariable_Wrap(std::move(c));
   END_HANDLE_TH_ERRORS
