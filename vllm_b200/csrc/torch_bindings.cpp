@@ -655,7 +655,11 @@ PyObject* py_linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
       !optional_tensor(args[6], &g_idx) || !optional_tensor(args[7], &perm))
     Py_RETURN_NONE;
   const at::Tensor& x = THPVariable_Unpack(args[0]);
-  if (!x.is_cuda() || x.dim() < 1 || (x.requires_grad() && c10::GradMode::is_enabled())) Py_RETURN_NONE;
+  if (!x.is_cuda() || x.dim() < 1) Py_RETURN_NONE;
+  if (c10::GradMode::is_enabled() &&
+      (x.requires_grad() || THPVariable_Unpack(args[3]).requires_grad() || (bias && bias->requires_grad()) ||
+       (zeros && zeros->requires_grad())))
+    Py_RETURN_NONE;
   const int64_t type_id = PyLong_AsLongLong(args[9]), size_m = PyLong_AsLongLong(args[10]),
                 size_n = PyLong_AsLongLong(args[11]), size_k = PyLong_AsLongLong(args[12]);
   const long flags = PyLong_AsLong(args[13]);  // 1: is_k_full, 2: is_zp_float
