@@ -74,7 +74,7 @@ int device_max_smem_optin() {
 
 template <typename T, int BITS>
 int dispatch_stream(const StreamParams& p, bool has_zp, int gm, int mb, int ntw, int max_ctas,
-                    cudaStream_t stream);
+                    cudaStream_t stream, StreamSplit* split);
 
 bool tc_gemm_supported(int64_t size_n, int64_t size_k, int gm);
 int launch_tc_gemm(const void* a, int64_t lda, const uint32_t* b, const void* scales, const uint32_t* zeros,
@@ -104,25 +104,42 @@ bool tc_path_enabled() {
   return on;
 }
 
-// Work split of the decode kernel as launch_stream makes it, with the clusters that fit taken as three fewer
-// than the SMs would hold (true of 4 and 8 CTAs on 148 SMs).
+int launch_decode(const StreamParams& p, bool has_zp, int gm, int mb, int ntw, int bits, int a_dtype, int max_ctas,
+                  cudaStream_t stream, StreamSplit* split) {
+  if (a_dtype == B200Q_F16)
+    return bits == 4 ? dispatch_stream<half, 4>(p, has_zp, gm, mb, ntw, max_ctas, stream, split)
+                     : dispatch_stream<half, 8>(p, has_zp, gm, mb, ntw, max_ctas, stream, split);
+  return bits == 4 ? dispatch_stream<__nv_bfloat16, 4>(p, has_zp, gm, mb, ntw, max_ctas, stream, split)
+                   : dispatch_stream<__nv_bfloat16, 8>(p, has_zp, gm, mb, ntw, max_ctas, stream, split);
+}
+
+// Variant of the decode kernel for up to 64 rows.
+struct DecodeShape {
+  int mb;   // 8-row blocks of A: 1, 2, 4 or 8
+  int ntw;  // slice width in 64-column tiles: two where the accumulators fit in registers
+};
+DecodeShape decode_shape(int64_t rows, int64_t n, int gm, bool general_only) {
+  const int mb = rows <= 8 ? 1 : rows <= 16 ? 2 : rows <= 32 ? 4 : 8;
+  const bool two = n / 64 % 2 == 0 && !general_only && ((gm == kChannel && mb <= 4) || (gm == kGrouped && mb <= 2));
+  return {mb, two ? 2 : 1};
+}
+
+// Work split of the decode kernel, as its launcher makes it.
 struct DecodeSplit {
   int64_t ctas, parts, tiles;  // CTAs; CTAs per column slice; k-tiles (16 x 64) that the busiest SM reads
   bool one_tile;               // slices of one 64-column tile
 };
-DecodeSplit decode_split(int64_t m, int64_t n, int64_t k, int bits, int gm) {
-  const int64_t nt = n / 64, kt = k / 16, sms = device_sm_count();
-  const int mt = m <= 8 ? 1 : m <= 16 ? 2 : 4;
-  const int ntw = nt % 2 == 0 && (gm == kChannel || mt <= 2) ? 2 : 1;
-  const int per_sm = mt * ntw * (gm == kGrouped ? 2 : 1) <= 4 && mt <= 2 ? 2 : 1;
-  const int64_t slices = nt / ntw;
-  int64_t parts = 1;
-  for (int64_t more = 2; more <= 8; more *= 2) {
-    if (slices * more > sms * per_sm || kt / more < 8 || (more > 2 && slices > sms * per_sm / more - 3)) break;
-    if (slices * more > sms && kt / more < (more == 8 ? 24 : bits == 4 ? 17 : 12)) break;
-    parts = more;
-  }
-  return {slices * parts, parts, (slices * parts + sms - 1) / sms * ntw * ((kt + parts - 1) / parts), ntw == 1};
+bool decode_split(int64_t m, int64_t n, int64_t k, int bits, int gm, bool has_zp, int a_dtype, DecodeSplit* d) {
+  const DecodeShape shape = decode_shape(m, n, gm, false);
+  StreamParams p = {};
+  p.m = (int)m; p.n = (int)n; p.k = (int)k;
+  p.kt_total = (int)(k / 16);
+  p.slices = (int)(n / 64 / shape.ntw);
+  StreamSplit split;
+  if (launch_decode(p, has_zp, gm, shape.mb, shape.ntw, bits, a_dtype, 0, nullptr, &split) != B200Q_OK) return false;
+  const int64_t ctas = (int64_t)p.slices * split.parts, sms = device_sm_count();
+  *d = {ctas, split.parts, (ctas + sms - 1) / sms * shape.ntw * ((p.kt_total + split.parts - 1) / split.parts), shape.ntw == 1};
+  return true;
 }
 
 // Integer weights up to 32 rows: decode kernel or tensor-core kernel, by estimated time.  The decode kernel
@@ -133,11 +150,13 @@ DecodeSplit decode_split(int64_t m, int64_t n, int64_t k, int bits, int gm) {
 // slower kernel by more than 6 %, two by more than 13.  (8-bit g128 fp16, 8 rows, us, decode / tensor cores:
 // 7168 x 9024, 141 slices on 148 SMs, 22.7 / 22.1; 3456 x 9024 12.4 / 14.1; 11008 x 5120, 160 half slices,
 // 27.8 / 20.1.)
-bool few_rows_on_tc(int64_t m, int64_t n, int64_t k, int bits, int gm, int group_blocks, bool has_zp, bool bf16) {
+bool few_rows_on_tc(int64_t m, int64_t n, int64_t k, int bits, int gm, int group_blocks, bool has_zp, int a_dtype) {
   if (m > 32 || (bits == 4 && m <= 8)) return false;
   const bool grouped = gm == kGrouped;
   if (grouped && !tc_group_sums_supported(16 * (int64_t)group_blocks)) return false;
-  const DecodeSplit d = decode_split(m, n, k, bits, gm);
+  const bool bf16 = a_dtype == B200Q_BF16;
+  DecodeSplit d;
+  if (!decode_split(m, n, k, bits, gm, has_zp, a_dtype, &d)) return false;
   const bool alone = d.ctas <= device_sm_count();  // one CTA on an SM where two would fit
   double base = 3.0, tile, factor;  // us: fixed and per tile of the decode kernel; conversion cost, 1 = 4-bit
   if (bits == 8) {
@@ -367,7 +386,7 @@ static int gemm_impl(const void* a, int64_t lda, const uint32_t* b_q_weight, con
   // these run the tensor-core kernel at every row count (the reference-order one where it can not)
   const bool general_only = zp_float || w_fp8 || w_fp4;
   // ---- tensor-core kernel: many rows, and the float formats at every row count ------------
-  if ((size_m >= 33 || general_only || (!link && few_rows_on_tc(size_m, size_n, size_k, bits, gm, group_blocks, has_zp, a_dtype == B200Q_BF16))) && tc_path_enabled() && tc_gemm_supported(size_n, size_k, gm)) {
+  if ((size_m >= 33 || general_only || (!link && few_rows_on_tc(size_m, size_n, size_k, bits, gm, group_blocks, has_zp, a_dtype))) && tc_path_enabled() && tc_gemm_supported(size_n, size_k, gm)) {
     const int fmt = zp_float ? (bits == 4 ? kTcU4ZF : kTcU8ZF)
                     : w_fp8 ? kTcF8
                     : w_fp4 ? (fp4_scales == 1 ? kTcNV4 : kTcMX4)
@@ -388,14 +407,7 @@ static int gemm_impl(const void* a, int64_t lda, const uint32_t* b_q_weight, con
   int64_t max_ctas = workspace_len < kMaxGrid ? workspace_len : kMaxGrid;
   for (int64_t m0 = 0; m0 < size_m; m0 += kMaxRowsPerLaunch) {
     const int rows = (int)((size_m - m0) < kMaxRowsPerLaunch ? (size_m - m0) : kMaxRowsPerLaunch);
-    // 8-row blocks of A handled per launch: 1, 2, 4 or 8
-    int mb = rows <= 8 ? 1 : rows <= 16 ? 2 : rows <= 32 ? 4 : 8;
-    // slice width in 64-column tiles: two where the accumulators fit in registers
-    int ntw = 1;
-    if (nt % 2 == 0 && !general_only) {
-      if (gm == kChannel && mb <= 4) ntw = 2;
-      if (gm == kGrouped && mb <= 2) ntw = 2;
-    }
+    const auto [mb, ntw] = decode_shape(rows, size_n, gm, general_only);
     StreamParams p = {};
     p.a = static_cast<const char*>(a_used) + (size_t)m0 * lda_used * 2;
     p.lda = lda_used;
@@ -420,15 +432,7 @@ static int gemm_impl(const void* a, int64_t lda, const uint32_t* b_q_weight, con
     p.global_scale = global_scale;
     p.ar = ArLink{};
     if (fuse_ar) p.ar = *link;
-    int rc;
-    if (a_dtype == B200Q_F16) {
-      rc = bits == 4 ? dispatch_stream<half, 4>(p, has_zp, gm, mb, ntw, (int)max_ctas, stream)
-                     : dispatch_stream<half, 8>(p, has_zp, gm, mb, ntw, (int)max_ctas, stream);
-    } else {
-      rc = bits == 4
-               ? dispatch_stream<__nv_bfloat16, 4>(p, has_zp, gm, mb, ntw, (int)max_ctas, stream)
-               : dispatch_stream<__nv_bfloat16, 8>(p, has_zp, gm, mb, ntw, (int)max_ctas, stream);
-    }
+    const int rc = launch_decode(p, has_zp, gm, mb, ntw, bits, a_dtype, (int)max_ctas, stream, nullptr);
     if (rc == B200Q_EUNSUPPORTED && g_error[0] == 0)
       set_error("Unsupported shapes: MNK = [%lld, %lld, %lld]", (long long)size_m,
                 (long long)size_n, (long long)size_k);
@@ -522,13 +526,7 @@ extern "C" int b200q_moe_wna16_marlin_gemm(
   const int mb8 = (int)(moe_block_size / 8);  // 8-row blocks: 1, 2, 4, 6, 8
   const int ntw = mb8 == 1 && size_n % 128 == 0 ? 2 : 1;
   p.slices = (int)(size_n / 64 / ntw);
-  int rc;
-  if (a_dtype == B200Q_F16)
-    rc = bits == 4 ? dispatch_stream<half, 4>(p, has_zp, gm, mb8, ntw, 1 << 20, stream)
-                   : dispatch_stream<half, 8>(p, has_zp, gm, mb8, ntw, 1 << 20, stream);
-  else
-    rc = bits == 4 ? dispatch_stream<__nv_bfloat16, 4>(p, has_zp, gm, mb8, ntw, 1 << 20, stream)
-                   : dispatch_stream<__nv_bfloat16, 8>(p, has_zp, gm, mb8, ntw, 1 << 20, stream);
+  const int rc = launch_decode(p, has_zp, gm, mb8, ntw, bits, a_dtype, 1 << 20, stream, nullptr);
   if (rc == B200Q_EUNSUPPORTED && g_error[0] == 0) set_error("moe: unsupported configuration");
   return rc;
 }

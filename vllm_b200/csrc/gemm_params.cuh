@@ -48,6 +48,12 @@ struct StreamParams {
   ArLink ar;
 };
 
+// How the decode kernel splits a problem, for whoever weighs it against another kernel.
+struct StreamSplit {
+  int parts;   // CTAs per column slice
+  int per_sm;  // CTAs that fit on an SM
+};
+
 constexpr int kStreamWarps = 8;
 constexpr int kStreamThreads = kStreamWarps * 32;
 

@@ -802,9 +802,9 @@ int max_clusters(K kernel, int smem, int size, std::atomic<int>& known) {
   return n;
 }
 
-// Host launcher for one (type, bits, zp, group mode, MT, NTW) variant.
+// Host launcher for one (type, bits, zp, group mode, MT, NTW) variant.  With `split` it only tells the split.
 template <typename T, int BITS, bool HAS_ZP, int GM, int MT, int NTW, bool MOE = false>
-int launch_stream(StreamParams p, int max_ctas, cudaStream_t stream) {
+int launch_stream(StreamParams p, cudaStream_t stream, StreamSplit* split) {
   using Cfg = StreamCfg<BITS, HAS_ZP, GM, MT, NTW>;
   using E = Emb<T, BITS>;
   // accumulator registers: acc (+ grp when grouped)
@@ -841,7 +841,10 @@ int launch_stream(StreamParams p, int max_ctas, cudaStream_t stream) {
     if (p.slices * blocks * more > device_sm_count() && p.kt_total / more < least) break;
     ksplit = more;
   }
-  (void)max_ctas;
+  if (split) {
+    *split = {ksplit, kMinBlocks};
+    return B200Q_OK;
+  }
   const int grid = p.slices * ksplit;
   // programmatic dependent launch: the kernel may start while its predecessor in
   // the stream drains; it orders itself with griddepcontrol.wait

@@ -18,7 +18,7 @@ using InstT = half;
 
 template <typename T, int BITS>
 int dispatch_stream(const StreamParams& p, bool has_zp, int gm, int mb, int ntw, int max_ctas,
-                    cudaStream_t stream);
+                    cudaStream_t stream, StreamSplit* split);
 
 namespace {
 
@@ -28,28 +28,28 @@ constexpr int B = INST_BITS;
 // `rows8` = 8-row blocks of A (1, 2, 4, 8); 8 blocks (64 rows) hold too many
 // accumulators for the streaming kernel and run the reference-order kernel.
 template <bool HAS_ZP>
-int channel(const StreamParams& p, int rows8, int ntw, int max_ctas, cudaStream_t stream) {
+int channel(const StreamParams& p, int rows8, int ntw, int max_ctas, cudaStream_t stream, StreamSplit* split) {
   switch (rows8 * 10 + ntw) {
-    case 11: return launch_stream<T, B, HAS_ZP, kChannel, 1, 1>(p, max_ctas, stream);
-    case 12: return launch_stream<T, B, HAS_ZP, kChannel, 1, 2>(p, max_ctas, stream);
-    case 21: return launch_stream<T, B, HAS_ZP, kChannel, 2, 1>(p, max_ctas, stream);
-    case 22: return launch_stream<T, B, HAS_ZP, kChannel, 2, 2>(p, max_ctas, stream);
-    case 41: return launch_stream<T, B, HAS_ZP, kChannel, 4, 1>(p, max_ctas, stream);
-    case 42: return launch_stream<T, B, HAS_ZP, kChannel, 4, 2>(p, max_ctas, stream);
-    case 81: return launch_lookup<T, B, HAS_ZP, kChannel, 4, 1>(p, max_ctas, stream);
+    case 11: return launch_stream<T, B, HAS_ZP, kChannel, 1, 1>(p, stream, split);
+    case 12: return launch_stream<T, B, HAS_ZP, kChannel, 1, 2>(p, stream, split);
+    case 21: return launch_stream<T, B, HAS_ZP, kChannel, 2, 1>(p, stream, split);
+    case 22: return launch_stream<T, B, HAS_ZP, kChannel, 2, 2>(p, stream, split);
+    case 41: return launch_stream<T, B, HAS_ZP, kChannel, 4, 1>(p, stream, split);
+    case 42: return launch_stream<T, B, HAS_ZP, kChannel, 4, 2>(p, stream, split);
+    case 81: return split ? B200Q_EUNSUPPORTED : launch_lookup<T, B, HAS_ZP, kChannel, 4, 1>(p, max_ctas, stream);
   }
   return B200Q_EUNSUPPORTED;
 }
 
 template <bool HAS_ZP>
-int grouped(const StreamParams& p, int rows8, int ntw, int max_ctas, cudaStream_t stream) {
+int grouped(const StreamParams& p, int rows8, int ntw, int max_ctas, cudaStream_t stream, StreamSplit* split) {
   switch (rows8 * 10 + ntw) {
-    case 11: return launch_stream<T, B, HAS_ZP, kGrouped, 1, 1>(p, max_ctas, stream);
-    case 12: return launch_stream<T, B, HAS_ZP, kGrouped, 1, 2>(p, max_ctas, stream);
-    case 21: return launch_stream<T, B, HAS_ZP, kGrouped, 2, 1>(p, max_ctas, stream);
-    case 22: return launch_stream<T, B, HAS_ZP, kGrouped, 2, 2>(p, max_ctas, stream);
-    case 41: return launch_stream<T, B, HAS_ZP, kGrouped, 4, 1>(p, max_ctas, stream);
-    case 81: return launch_lookup<T, B, HAS_ZP, kGrouped, 4, 1>(p, max_ctas, stream);
+    case 11: return launch_stream<T, B, HAS_ZP, kGrouped, 1, 1>(p, stream, split);
+    case 12: return launch_stream<T, B, HAS_ZP, kGrouped, 1, 2>(p, stream, split);
+    case 21: return launch_stream<T, B, HAS_ZP, kGrouped, 2, 1>(p, stream, split);
+    case 22: return launch_stream<T, B, HAS_ZP, kGrouped, 2, 2>(p, stream, split);
+    case 41: return launch_stream<T, B, HAS_ZP, kGrouped, 4, 1>(p, stream, split);
+    case 81: return split ? B200Q_EUNSUPPORTED : launch_lookup<T, B, HAS_ZP, kGrouped, 4, 1>(p, max_ctas, stream);
   }
   return B200Q_EUNSUPPORTED;
 }
@@ -111,10 +111,10 @@ int moe_blocks(const StreamParams& p, int rows8, int ntw, int max_ctas, cudaStre
   // blocks of up to 32 ids: the decode kernel; above: the reference-order kernel
   switch (rows8) {
     case 1:
-      return ntw == 2 ? launch_stream<T, B, HAS_ZP, GM, 1, 2, true>(p, max_ctas, stream)
-                      : launch_stream<T, B, HAS_ZP, GM, 1, 1, true>(p, max_ctas, stream);
-    case 2: return launch_stream<T, B, HAS_ZP, GM, 2, 1, true>(p, max_ctas, stream);
-    case 4: return launch_stream<T, B, HAS_ZP, GM, 4, 1, true>(p, max_ctas, stream);
+      return ntw == 2 ? launch_stream<T, B, HAS_ZP, GM, 1, 2, true>(p, stream, nullptr)
+                      : launch_stream<T, B, HAS_ZP, GM, 1, 1, true>(p, stream, nullptr);
+    case 2: return launch_stream<T, B, HAS_ZP, GM, 2, 1, true>(p, stream, nullptr);
+    case 4: return launch_stream<T, B, HAS_ZP, GM, 4, 1, true>(p, stream, nullptr);
   }
   const int mb = (rows8 + 1) / 2;  // 16-row blocks
   switch (mb) {
@@ -152,7 +152,8 @@ int lookup(const StreamParams& p, int rows8, int ntw, int max_ctas, cudaStream_t
 
 template <>
 int dispatch_stream<InstT, INST_BITS>(const StreamParams& p, bool has_zp, int gm, int mb, int ntw,
-                                      int max_ctas, cudaStream_t stream) {
+                                      int max_ctas, cudaStream_t stream, StreamSplit* split) {
+  if (split && (p.moe_sorted_ids || p.w_fp8 || p.w_fp4 || p.zp_float || gm == kLookup)) return B200Q_EUNSUPPORTED;
   if (p.moe_sorted_ids) return (p.w_fp8 || p.w_fp4) ? B200Q_EUNSUPPORTED : moe(p, has_zp, gm, mb, ntw, max_ctas, stream);
   if (p.w_fp8) return has_zp ? B200Q_EUNSUPPORTED : fp8_weights(p, gm, mb, ntw, max_ctas, stream);
   if (p.w_fp4) return has_zp ? B200Q_EUNSUPPORTED : fp4_weights(p, gm, mb, ntw, max_ctas, stream);
@@ -160,11 +161,11 @@ int dispatch_stream<InstT, INST_BITS>(const StreamParams& p, bool has_zp, int gm
     return (has_zp && gm == kGrouped) ? grouped_zp_float(p, mb, ntw, max_ctas, stream)
                                       : B200Q_EUNSUPPORTED;
   if (gm == kChannel)
-    return has_zp ? channel<true>(p, mb, ntw, max_ctas, stream)
-                  : channel<false>(p, mb, ntw, max_ctas, stream);
+    return has_zp ? channel<true>(p, mb, ntw, max_ctas, stream, split)
+                  : channel<false>(p, mb, ntw, max_ctas, stream, split);
   if (gm == kGrouped)
-    return has_zp ? grouped<true>(p, mb, ntw, max_ctas, stream)
-                  : grouped<false>(p, mb, ntw, max_ctas, stream);
+    return has_zp ? grouped<true>(p, mb, ntw, max_ctas, stream, split)
+                  : grouped<false>(p, mb, ntw, max_ctas, stream, split);
   if (has_zp) return B200Q_EUNSUPPORTED;
   return lookup(p, mb, ntw, max_ctas, stream);
 }
