@@ -116,6 +116,15 @@ size_t b200q_marlin_gemm_preferred_scratch_bytes(int64_t size_m, int64_t size_n,
                                                  int64_t size_k, int has_act_order);
 
 /*
+ * The same for one call whose types and options are known (the arguments of b200q_marlin_gemm and
+ * b200q_marlin_gemm_fp4): only what the kernel that it runs uses, 256 bytes where that is nothing.  The two sizes
+ * above hold for every call of these sizes.
+ */
+size_t b200q_marlin_gemm_call_scratch_bytes(int64_t b_q_type_id, int a_dtype, int64_t size_m,
+                                            int64_t size_n, int64_t size_k, int64_t num_groups,
+                                            int has_zp, int has_act_order, unsigned flags);
+
+/*
  * C[M,N] = A[M,K] * dequant(B) (+ bias): the mixed-precision GEMM.
  * Replaces: gptq_marlin_gemm, csrc/quantization/gptq_marlin/gptq_marlin.cu:674-959
  *           (op schema csrc/torch_bindings.cpp:308-315).
@@ -126,7 +135,8 @@ size_t b200q_marlin_gemm_preferred_scratch_bytes(int64_t size_m, int64_t size_n,
  *   g_idx, perm  int32 [size_k] (sorted group ids / sort permutation), both or neither
  *   b_bias       [size_n] of a's type, marlin_permute_bias'd, or NULL
  *   c            [size_m, size_n] contiguous, written
- *   scratch      >= b200q_marlin_gemm_scratch_bytes(...) bytes, 256 B aligned
+ *   scratch      >= b200q_marlin_gemm_scratch_bytes(...) bytes (or what b200q_marlin_gemm_call_scratch_bytes
+ *                gives for this call), 256 B aligned
  *   workspace    int32 [workspace_len], all zero on entry, zero again when the
  *                kernels finish; workspace_len >= 1 (the reference passes #SMs)
  *   b_q_type_id  ScalarType id (csrc/core/scalar_type.hpp:124-157): uint4b8,

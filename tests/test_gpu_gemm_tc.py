@@ -194,6 +194,29 @@ def test_captured_call_keeps_its_scratch(env):
     assert all(torch.equal(o, w) for o, w in zip(outs, want))
 
 
+def test_captured_decode_call_takes_no_partial_sums(env):
+    torch, G, ops, mu, lib = env
+    M, K, N = 4, 2048, 28672
+    q = torch.zeros((K // 16, N * 2), dtype=torch.int32, device="cuda")
+    s = torch.ones((K // 128, N), dtype=torch.float16, device="cuda")
+    a = torch.ones((M, K), dtype=torch.float16, device="cuda")
+    ws, e = mu.marlin_make_workspace_new(torch.device("cuda")), torch.empty(0, dtype=torch.int32, device="cuda")
+    run = lambda: ops.gptq_marlin_gemm(a, None, q, None, s, None, e, e, e, ws, mu.scalar_types.uint4b8, M, N, K, True, False,
+                                       True, False)
+    run()
+    g = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g):
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        out = run()
+        peak = torch.cuda.max_memory_allocated() - before
+    assert peak <= out.numel() * 2 + 4096
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, torch.full_like(out, -8.0 * K))
+
+
 @pytest.mark.parametrize("M,qtype,group", [(100, "uint4b8", 128), (300, "uint8b128", -1), (700, "uint8b128", 128)])
 def test_tc_gemm_is_reproducible(env, M, qtype, group):
     """The same call gives the same bits every time: a weight slot that is refilled before it was read

@@ -283,3 +283,21 @@ def test_layer_bias_is_whatever_the_layer_calls_bias(kind, row_parallel):
         want = value
     got = layer(torch.zeros(1, 8))
     assert (got is None and want is None) or torch.equal(got, want)
+
+
+def test_scratch_of_a_call_is_what_its_kernel_uses():
+    from vllm_b200 import _lib
+    lib = _lib.load()
+    of = lambda t, m, n, k, groups=32, zp=0, act=0, flags=_lib.FLAG_K_FULL, dtype=_lib.BF16: \
+        lib.b200q_marlin_gemm_call_scratch_bytes(t, dtype, m, n, k, groups, zp, act, flags)
+    any_call = lib.b200q_marlin_gemm_preferred_scratch_bytes
+    # decode kernel: nothing but the gathered rows of an act-order layer
+    assert of(mo.UINT4B8_ID, 1, 28672, 4096) == 256
+    assert of(mo.UINT4B8_ID, 8, 28672, 4096, act=1) == 8 * 4096 * 2
+    # part of an act-order layer's k: partial sums of the reference-order kernel
+    assert of(mo.UINT4B8_ID, 1, 4096, 4096, act=1, flags=0) > 4096 * 2 + (1 << 20)
+    for t, m, groups, zp, act in ((mo.UINT4B8_ID, 1, 32, 0, 1), (mo.UINT8B128_ID, 16, 1, 0, 0), (mo.UINT4_ID, 32, 32, 1, 0),
+                                  (mo.UINT4B8_ID, 48, 32, 0, 0), (mo.UINT4B8_ID, 4096, 32, 0, 0)):
+        assert 256 <= of(t, m, 4096, 4096, groups, zp, act) <= any_call(m, 4096, 4096, act)
+    # what the call itself will refuse
+    assert of(123, 16, 4096, 4096) == any_call(16, 4096, 4096, 0)

@@ -23,6 +23,7 @@ EXPORTS = (
     "b200q_permute_cols",
     "b200q_marlin_gemm_scratch_bytes",
     "b200q_marlin_gemm_preferred_scratch_bytes",
+    "b200q_marlin_gemm_call_scratch_bytes",
     "b200q_marlin_gemm",
     "b200q_marlin_gemm_fp4",
     "b200q_moe_wna16_marlin_gemm",
@@ -82,6 +83,8 @@ def load() -> ctypes.CDLL:
     lib.b200q_marlin_gemm_scratch_bytes.argtypes = [i64, i64, i64, i32]
     lib.b200q_marlin_gemm_preferred_scratch_bytes.restype = c.c_size_t
     lib.b200q_marlin_gemm_preferred_scratch_bytes.argtypes = [i64, i64, i64, i32]
+    lib.b200q_marlin_gemm_call_scratch_bytes.restype = c.c_size_t
+    lib.b200q_marlin_gemm_call_scratch_bytes.argtypes = [i64, i32, i64, i64, i64, i64, i32, i32, u32]
     lib.b200q_marlin_gemm.restype = i32
     lib.b200q_marlin_gemm.argtypes = [
         vp, i64, vp, vp, vp, vp, vp, vp, vp, vp, c.c_size_t, vp, i64, i64, i32,

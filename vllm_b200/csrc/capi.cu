@@ -179,7 +179,36 @@ bool few_rows_on_tc(int64_t m, int64_t n, int64_t k, int bits, int gm, int group
 
 inline int64_t align_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
 
-// partial-sum scratch: (grid + slices) slots of (rows x slice width) floats
+// Which kernel a call runs.
+struct Route {
+  bool tc;        // tensor-core kernel; else decode or reference-order kernels
+  bool partials;  // the reference-order kernel, which leaves partial sums in the scratch
+};
+Route route_of(int64_t m, int64_t n, int64_t k, int bits, int gm, int group_blocks, bool has_zp, int a_dtype,
+               bool general_only, bool link) {
+  // A caller asks for the scratch of a call, then makes it: the second time the answer (a function of these values
+  // and the device) is at hand.  Weighing the two kernels takes 0.4 us of a call's 7.
+  struct Last {
+    int64_t m, n, k;
+    int what, group_blocks, device;
+    Route r;
+  };
+  static thread_local Last last = {};
+  int device = 0;
+  cudaGetDevice(&device);
+  const int what = bits | gm << 4 | a_dtype << 6 | has_zp << 8 | general_only << 9 | link << 10;
+  if (last.m == m && last.n == n && last.k == k && last.what == what && last.group_blocks == group_blocks && last.device == device)
+    return last.r;
+  Route r;
+  // the tensor-core kernel: many rows, and the float formats at every row count
+  r.tc = tc_path_enabled() && tc_gemm_supported(n, k, gm) &&
+         (m >= 33 || general_only || (!link && few_rows_on_tc(m, n, k, bits, gm, group_blocks, has_zp, a_dtype)));
+  r.partials = !r.tc && (m > 32 || general_only || gm == kLookup);
+  last = {m, n, k, what, group_blocks, device, r};
+  return r;
+}
+
+// partial sums of the reference-order kernel: (grid + slices) slots of (rows x slice width) floats
 int64_t partial_bytes(int64_t size_n) {
   // a slot holds at most 4096 floats (rows x slice width: 32 x 128 or 64 x 64);
   // slots are indexed cta + slice < grid + slices <= kMaxGrid + N/64
@@ -187,7 +216,8 @@ int64_t partial_bytes(int64_t size_n) {
   return (kMaxGrid + nt) * 64 * 64 * 4;
 }
 
-// first region of the scratch: decode partial sums or the tensor-core kernel's k-split partials
+// first region of the scratch, whatever kernel runs: the reference-order kernel's partial sums or the tensor-core
+// kernel's
 int64_t work_bytes(int64_t size_m, int64_t size_n, int64_t size_k) {
   const int64_t tc = tc_path_enabled() ? tc_gemm_scratch_bytes(size_m, size_n, size_k) : 0;
   const int64_t dec = partial_bytes(size_n);
@@ -237,7 +267,7 @@ static bool fused_ar_enabled() {
   return on;
 }
 
-// The GEMM behind both entry points.  With `link` the output is all-reduced over the
+// The GEMM behind the entry points (with `wanted_scratch`: the bytes that this call would use, nothing runs).  With `link` the output is all-reduced over the
 // peer link: inside the GEMM kernel where one decode launch covers the problem,
 // otherwise by the stand-alone kernel on the finished output.
 static int gemm_impl(const void* a, int64_t lda, const uint32_t* b_q_weight, const void* b_scales,
@@ -246,7 +276,7 @@ static int gemm_impl(const void* a, int64_t lda, const uint32_t* b_q_weight, con
                      int32_t* workspace, int64_t workspace_len, int64_t b_q_type_id, int a_dtype,
                      int64_t size_m, int64_t size_n, int64_t size_k, int64_t num_groups,
                      unsigned flags, cudaStream_t stream, const ArLink* link,
-                     const void* global_scale = nullptr, int fp4_scales = 0) {
+                     const void* global_scale = nullptr, int fp4_scales = 0, size_t* wanted_scratch = nullptr) {
   // ---- type contract ---------------------------------------------------------------
   int bits = 0;
   bool type_has_zp = false;
@@ -284,7 +314,7 @@ static int gemm_impl(const void* a, int64_t lda, const uint32_t* b_q_weight, con
                 (long long)size_m, (long long)size_n, (long long)size_k);
   B200Q_REQUIRE(size_n < (1ll << 31) && size_k < (1ll << 31) && size_m < (1ll << 31), B200Q_EINVAL,
                 "size too large");
-  B200Q_REQUIRE(a && b_q_weight && b_scales && c && workspace, B200Q_EINVAL,
+  B200Q_REQUIRE(wanted_scratch || (a && b_q_weight && b_scales && c && workspace), B200Q_EINVAL,
                 "null tensor pointer");
   B200Q_REQUIRE(lda >= size_k && lda % 8 == 0, B200Q_EINVAL, "A.stride(0) must divisible by 8");
   B200Q_REQUIRE((reinterpret_cast<uintptr_t>(a) & 15) == 0, B200Q_EINVAL,
@@ -335,10 +365,19 @@ static int gemm_impl(const void* a, int64_t lda, const uint32_t* b_q_weight, con
     group_blocks = kt_total;  // single group: zero-points (if any) load once
   }
 
+  // these run the tensor-core kernel at every row count (the reference-order one where it can not)
+  const bool general_only = zp_float || w_fp8 || w_fp4;
+  const Route route = route_of(size_m, size_n, size_k, bits, gm, group_blocks, has_zp, a_dtype, general_only, link != nullptr);
   // ---- scratch -----------------------------------------------------------------------
   // the k-split of the tensor-core kernel is optional: it shrinks to what the scratch holds
   const int64_t a_tmp_bytes = has_act_order ? align_up(size_m * size_k * 2, 256) : 0;
-  const size_t need = b200q_marlin_gemm_scratch_bytes(size_m, size_n, size_k, has_act_order);
+  if (wanted_scratch) {
+    int64_t work = route.partials ? partial_bytes(size_n) : route.tc ? tc_gemm_scratch_bytes(size_m, size_n, size_k) : 0;
+    work = align_up(work, 256) + a_tmp_bytes;
+    *wanted_scratch = (size_t)(work > 256 ? work : 256);
+    return B200Q_OK;
+  }
+  const size_t need = (size_t)((route.partials ? align_up(partial_bytes(size_n), 256) : 0) + a_tmp_bytes);
   B200Q_REQUIRE(scratch && scratch_bytes >= need, B200Q_ESCRATCH,
                 "scratch of %zu bytes is below the required %zu", scratch_bytes, need);
   B200Q_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 255) == 0, B200Q_EINVAL,
@@ -383,10 +422,8 @@ static int gemm_impl(const void* a, int64_t lda, const uint32_t* b_q_weight, con
     B200Q_REQUIRE(global_scale == nullptr && fp4_scales == 0, B200Q_EINVAL,
                   "global_scale can only be used for nvfp4 format.");
   }
-  // these run the tensor-core kernel at every row count (the reference-order one where it can not)
-  const bool general_only = zp_float || w_fp8 || w_fp4;
-  // ---- tensor-core kernel: many rows, and the float formats at every row count ------------
-  if ((size_m >= 33 || general_only || (!link && few_rows_on_tc(size_m, size_n, size_k, bits, gm, group_blocks, has_zp, a_dtype))) && tc_path_enabled() && tc_gemm_supported(size_n, size_k, gm)) {
+  // ---- tensor-core kernel -------------------------------------------------------------------
+  if (route.tc) {
     const int fmt = zp_float ? (bits == 4 ? kTcU4ZF : kTcU8ZF)
                     : w_fp8 ? kTcF8
                     : w_fp4 ? (fp4_scales == 1 ? kTcNV4 : kTcMX4)
@@ -440,6 +477,22 @@ static int gemm_impl(const void* a, int64_t lda, const uint32_t* b_q_weight, con
   }
   if (link && !fuse_ar) return launch_all_reduce(*link, c, c, size_m * size_n, a_dtype, stream);
   return B200Q_OK;
+}
+
+extern "C" size_t b200q_marlin_gemm_call_scratch_bytes(int64_t b_q_type_id, int a_dtype, int64_t size_m, int64_t size_n,
+                                                       int64_t size_k, int64_t num_groups, int has_zp, int has_act_order,
+                                                       unsigned flags) {
+  // present or not is all that counts of the optional tensors
+  alignas(16) static const int32_t here = 0;
+  size_t bytes = 256;
+  const bool fp4 = b_q_type_id == kTypeFE2M1f;
+  const int scales = fp4 && num_groups > 0 && size_k / num_groups == 16 ? B200Q_FP4_SCALES_E4M3 : B200Q_FP4_SCALES_E8M0;
+  const int rc = gemm_impl(nullptr, size_k, nullptr, nullptr, has_zp ? reinterpret_cast<const uint32_t*>(&here) : nullptr,
+                           has_act_order ? &here : nullptr, has_act_order ? &here : nullptr, nullptr, nullptr, nullptr, 0,
+                           nullptr, 1, b_q_type_id, a_dtype, size_m, size_n, size_k, num_groups, flags, nullptr, nullptr,
+                           nullptr, fp4 ? scales : 0, &bytes);
+  // a call that will be refused with a message of its own
+  return rc == B200Q_OK ? bytes : b200q_marlin_gemm_preferred_scratch_bytes(size_m, size_n, size_k, has_act_order);
 }
 
 extern "C" int b200q_marlin_gemm(const void* a, int64_t lda, const uint32_t* b_q_weight,

@@ -316,7 +316,7 @@ int launch_tc_moe(const void* a, int64_t rows, const uint32_t* b, const void* sc
 
 // Scratch the tensor-core kernel would like for this problem (fp32 partials of shared tiles).
 int64_t tc_gemm_scratch_bytes(int64_t size_m, int64_t size_n, int64_t size_k) {
-  if (size_k % tc::kBK != 0 || size_n % 64 != 0) return 0;
+  if (size_k % tc::kBK != 0 || size_n % 64 != 0 || device_sm_count() < 2) return 0;  // (0: no device to plan for)
   return tc::plan_tiles(size_m, size_n, size_k, device_sm_count(), int64_t(1) << 40).partial_bytes;
 }
 

@@ -285,8 +285,8 @@ at::Tensor gptq_marlin_gemm(at::Tensor& a, std::optional<at::Tensor> c_or_none,
   if (size_m == 0) return c;
   const c10::cuda::OptionalCUDAGuard guard(device_of(a));
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream(a.get_device());
-  const size_t nbytes =
-      b200q_marlin_gemm_preferred_scratch_bytes(size_m, size_n, size_k, g.act_order ? 1 : 0);
+  const size_t nbytes = b200q_marlin_gemm_call_scratch_bytes(
+      b_q_type, g.dtype, size_m, size_n, size_k, g.num_groups, g.zeros != nullptr, g.act_order, g.flags);
   const ScratchLease scratch(a.device(), stream, nbytes);
   int rc;
   if (g.fp4_scales != 0) {
@@ -334,8 +334,8 @@ at::Tensor gptq_marlin_gemm_all_reduce(
               "state must be an int32 CUDA tensor of b200q_all_reduce_state_bytes()");
   const c10::cuda::OptionalCUDAGuard guard(device_of(a));
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream(a.get_device());
-  const size_t nbytes =
-      b200q_marlin_gemm_preferred_scratch_bytes(size_m, size_n, size_k, g.act_order ? 1 : 0);
+  const size_t nbytes = b200q_marlin_gemm_call_scratch_bytes(
+      b_q_type, g.dtype, size_m, size_n, size_k, g.num_groups, g.zeros != nullptr, g.act_order, g.flags);
   const ScratchLease scratch(a.device(), stream, nbytes);
   const int rc = b200q_marlin_gemm_all_reduce(
       g.a, g.lda, g.b, g.scales, g.zeros, g.g_idx, g.perm, g.bias, c.data_ptr(), scratch.data(),
