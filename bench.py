@@ -604,7 +604,9 @@ def time_moe(torch, ops, dev, dt, stream, gen, ws, steps):
         a = torch.randn((m, k), dtype=dt, device=dev, generator=gen)
         topk_ids = torch.stack([torch.randperm(e, device=dev, generator=gen)[:topk] for _ in range(m)])
         tw = torch.rand((m * topk,), device=dev, generator=gen)
-        for bs in (8, 16, 32):                      # as fused_moe.fused_marlin_moe picks it
+        # the operator's block sizes by rows per expert; the layer (fused_moe.fused_marlin_moe) takes the
+        # tensor-core kernel instead at the second size
+        for bs in (8, 16, 32):
             if m * topk / e / bs < 0.9:
                 break
         sorted_ids, expert_ids, num = fused_moe.moe_align_block_size(topk_ids.to(torch.int32), bs, e)
@@ -634,7 +636,8 @@ def time_moe(torch, ops, dev, dt, stream, gen, ws, steps):
                      "gbs": round(b / us / 1e3, 1),
                      "tflops": round(2.0 * m * topk * n * k / us / 1e6, 2)})
     return {"workload": "moe_wna16_marlin_gemm: 8 experts, top-2, gate_up 4096 -> 28672, uint4b8 g128, "
-                        "decode kernel, reference-order kernel for blocks above 32", "steps": steps, "per_shape": rows}
+                        "decode kernel (the operator alone; the layer takes the tensor-core kernel at 256 tokens)",
+            "steps": steps, "per_shape": rows}
 
 
 def run_ar_check(torch, dist, D, lib, dev, custom_ar, ar_link, rank, world):
@@ -780,9 +783,9 @@ def report(args, world, shapes, ms, total_ms, ms2, e2e_steps, launches, clocks, 
     stream_gbs = div(str_b, str_t) / 1e6  # per GPU: every rank runs the same shapes
     # DRAM bytes (read + write) of one launch of the dominant decode kernel, from the ncu capture
     # summarised in profiles/gemm_stream_gate_up_m16.txt: gate_up with act-order, M = 16,
-    # 60.73 MB read + 0.32 MB written for 61.6 MB algorithmic (the gather kernel in front of it
+    # 60.72 MB read + 0.18 MB written for 61.6 MB algorithmic (the gather kernel in front of it
     # adds 0.15 MB: profiles/permute_cols_gate_up_m16.txt)
-    traffic = 61.04e6
+    traffic = 60.91e6
     line = {
         "metric": METRIC, "value": value, "unit": "GB/s", "n_gpus": world, "steps": k_steps,
         "warmup": args.warmup, "ms_per_step": total_ms / k_steps, "higher_is_better": True,

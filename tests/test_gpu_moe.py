@@ -174,20 +174,30 @@ def test_moe_align_kernel(numel, E, block, idtype, mapped):
 
 
 @pytest.mark.parametrize("M,E,topk,qtype,dtype,expert_parallel,on_input", [
-    (1, 8, 2, "uint8b128", "bfloat16", False, False),      # tensor-core kernel, one row per expert
+    (1, 8, 2, "uint8b128", "bfloat16", False, False),      # decode kernel, one row per expert
     (70, 2, 2, "uint4", "float16", False, False),          # runs longer than a tile of single CTAs
     (150, 3, 2, "uint4b8", "bfloat16", True, False),       # CTA pairs, experts of another rank
     (513, 2, 1, "uint8", "float16", False, True),          # runs split over several tiles, weight on the input
     (3, 16, 4, "uint4b8", "bfloat16", True, True),         # decode kernel
 ])
 def test_fused_marlin_moe_kernels(M, E, topk, qtype, dtype, expert_parallel, on_input):
+    _check_layer(M, E, topk, qtype, dtype, expert_parallel, on_input, 64)
+
+
+@pytest.mark.parametrize("M,E,qtype", [(1, 8, "uint8b128"), (20, 4, "uint4"), (200, 2, "uint8")])
+def test_fused_marlin_moe_scale_per_column(M, E, qtype):
+    """Tensor-core kernel down to one row per expert, scales in the epilogue."""
+    _check_layer(M, E, 2, qtype, "bfloat16", False, False, -1)
+
+
+def _check_layer(M, E, topk, qtype, dtype, expert_parallel, on_input, group):
     import torch
     from vllm_b200 import _lib, fused_moe
     from vllm_b200.scalar_type import scalar_types
     K, N = 320, 192
     rng = np.random.default_rng(M + E)
     local = [e for e in range(E) if not expert_parallel or e % 2 == 0]
-    w1 = _experts(len(local), K, 2 * N, qtype, 64, dtype, with_bias=True, seed=1)
+    w1 = _experts(len(local), K, 2 * N, qtype, group, dtype, with_bias=True, seed=1)
     w2 = _experts(len(local), N, K, qtype, -1, dtype, seed=2)
     a = 0.1 * H.make_activations(M, K, dtype)
     a = mo.round_to_dtype(a, dtype)

@@ -165,9 +165,11 @@ struct TcPlan {
   double rounds_us;  // the part of it that is rounds
 };
 
-// Microseconds of a round (128 deep in k) of one tile, measured on B200 as the slope over K at one tile per
-// worker (4-bit: 0.45 at 48 tokens, 0.58 at 128; pairs 0.57 at 160, 0.78 at 256; other formats run 0 to 15 %
-// longer, which moves the choice little).
+// Microseconds of a round (128 deep in k) of one tile, measured on B200 for 4-bit weights as the slope over K at
+// one tile per worker: 0.45 at 48 tokens, 0.58 at 128; pairs 0.57 at 160, 0.78 at 256.  Other formats are not in
+// here, and whole layers run longer: 8-bit fp16 pairs of 192 tokens 0.90 (table 0.64), NVFP4 pairs of 256 1.0
+// (0.78), 4-bit at 4096 tokens under the power cap 0.90 (0.78).  A factor common to all candidates leaves the choice
+// as it is except where sharing is weighed, see below.
 static double round_us(int cg, int tn) {
   if (cg == 1) return tn <= 64 ? 0.45 : 0.46 + 0.00096 * tn;
   const double t = 0.22 + 0.00217 * tn;
@@ -213,6 +215,8 @@ static TcPlan plan_tiles(int64_t m, int64_t n, int64_t k, int sms, int64_t scrat
       const int64_t slot_bytes = (int64_t)cg * pl.tn * kBN * 4;
       pl.partial_bytes = 2 * workers * slot_bytes;
       pl.rounds_us = (double)(waves * rounds + (rem * rounds + workers - 1) / workers) * round;
+      // (fixed costs for the choice between plans; tc_gemm_estimate_us has its own, fitted to whole calls.  The
+      // two put sharing up to 1.5 us apart, and fp8 at 24 x 4096 x 28672 is shared by a margin of 0.4 us.)
       // a second segment behind whole tiles: its own pipeline fill and drain (1152 x 19392, 152 tiles of nine
       // rounds: 15.2 us with the last four shared, 11.0 in two waves)
       pl.us = pl.rounds_us + 2.5 + (waves > 0 ? 2.0 : 0.0) + 2.0 * (double)((workers + rem) * slot_bytes) / 4e6;
@@ -320,7 +324,8 @@ int64_t tc_gemm_scratch_bytes(int64_t size_m, int64_t size_n, int64_t size_k) {
   return tc::plan_tiles(size_m, size_n, size_k, device_sm_count(), int64_t(1) << 40).partial_bytes;
 }
 
-// Estimated time of the kernel (and its reduce kernel) in us; `factor`: cost of the weight conversion, 1 = 4-bit.
+// Estimated time of the kernel (and its reduce kernel) in us, fitted to whole calls of up to 32 rows; `factor`: time
+// of a round, 1 = 4-bit with scaled weights.
 double tc_gemm_estimate_us(int64_t size_m, int64_t size_n, int64_t size_k, double factor) {
   const tc::TcPlan pl = tc::plan_tiles(size_m, size_n, size_k, device_sm_count(), int64_t(1) << 40);
   const double us = factor * pl.rounds_us;

@@ -955,8 +955,9 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
         release();
       } else {
         // scale x group sums into the running sums, a group at a time.  The two warps of a quadrant take the lower
-        // and the upper tokens.  Scales are brought into L2 at the start of the segment, a lane a row, and into a
-        // register one group ahead (the latency of memory showed otherwise: 8192 x 18944 at 16 rows 47 us against 41).
+        // and the upper tokens.  Scales are brought into L2 at the start of the segment, a lane a row, and into
+        // registers four groups ahead (without the first the latency of memory showed, 8192 x 18944 at 16 rows 47 us
+        // against 41).
         const int step0 = 2 * sg.r0, step1 = min(steps, 2 * sg.r1);
         const int g0 = step0 / group_steps, groups = (step1 - 1) / group_steps + 1 - g0;
         const uint16_t* src = static_cast<const uint16_t*>(p.scales) + ((size_t)sg.expert * p.groups + g0) * p.n + grouped_perm_pos(n);
