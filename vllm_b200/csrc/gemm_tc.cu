@@ -66,9 +66,16 @@ static int rows_per_round(int gb) {
 static int make_weight_maps(TcMaps* m, TcParams* p, const void* b, const void* scales, const void* zeros, int fmt,
                             int64_t n, int64_t k, int64_t experts) {
   const int bits = format_bits(fmt);
-  // packed weights as rows of k-tiles of 8-byte elements; box = a round x 128 columns
-  int rc = make_map(&m->b, b, CU_TENSOR_MAP_DATA_TYPE_UINT64, 8, n * bits / 4, experts * (k / 16), 32 * bits, kRoundTiles);
-  if (rc != B200Q_OK) return rc;
+  // packed weights: k-tiles of pieces of 128 bytes; box = a round x 128 columns, swizzled piece by piece
+  const cuuint64_t gdim[3] = {16, (cuuint64_t)(n * bits / 64), (cuuint64_t)(experts * (k / 16))};
+  const cuuint64_t gstride[2] = {128, (cuuint64_t)(n * 2 * bits)};
+  const cuuint32_t box[3] = {16, (cuuint32_t)(2 * bits), (cuuint32_t)kRoundTiles};
+  const cuuint32_t estride[3] = {1, 1, 1};
+  const CUresult r = get_encode_fn()(&m->b, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, const_cast<uint32_t*>(static_cast<const uint32_t*>(b)),
+                                     gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  B200Q_REQUIRE(r == CUDA_SUCCESS, B200Q_ECUDA, "cuTensorMapEncodeTiled failed with %d", (int)r);
+  int rc = B200Q_OK;
   p->groups = (int)(k / 16 / p->group_blocks);
   p->group_rows = rows_per_round(p->group_blocks);
   if (fmt == kNV4 || fmt == kMX4) {

@@ -17,7 +17,7 @@ using InstT = half;
 
 template <typename T, int F, int CG, int TOK, bool SUMS = false>
 static int launch_one(const TcMaps& maps, const TcParams& p, bool pdl, cudaStream_t stream) {
-  using Cfg = TcCfg<F, TOK, SUMS>;
+  using Cfg = TcCfg<F, CG, TOK, SUMS>;
   static_assert(Cfg::kWD >= 2, "weight ring too shallow");
   auto kernel = gemm_tc_kernel<T, F, CG, TOK, SUMS>;
   static bool attr_done[64] = {};  // per device; benign race: the call is idempotent
@@ -29,7 +29,7 @@ static int launch_one(const TcMaps& maps, const TcParams& p, bool pdl, cudaStrea
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(p.workers * CG));
-  cfg.blockDim = dim3(threads(SUMS));
+  cfg.blockDim = dim3(Cfg::kThreads);
   cfg.dynamicSmemBytes = Cfg::kSmemBytes;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
@@ -60,7 +60,7 @@ template <typename T, int F>
 static int launch_sums(const TcMaps& maps, const TcParams& p, int cg, bool pdl, cudaStream_t stream) {
   if constexpr (F == kU4B8 || F == kU4Z || F == kU8B128 || F == kU8Z) {
     if (p.tn <= group_sums_tokens(cg))
-      return cg == 2 ? launch_one<T, F, 2, 96, true>(maps, p, pdl, stream) : launch_one<T, F, 1, 64, true>(maps, p, pdl, stream);
+      return cg == 2 ? launch_one<T, F, 2, 80, true>(maps, p, pdl, stream) : launch_one<T, F, 1, 64, true>(maps, p, pdl, stream);
   }
   set_error("group scales on the sums: weight format %d, %d tokens per tile", F, p.tn);
   return B200Q_EUNSUPPORTED;
@@ -71,8 +71,10 @@ static int launch_sums(const TcMaps& maps, const TcParams& p, int cg, bool pdl, 
   int launch_format<InstT, F>(const TcMaps& maps, const TcParams& p, int cg, bool sums, bool pdl, cudaStream_t stream) { \
     if (sums) return launch_sums<InstT, F>(maps, p, cg, pdl, stream);                                                \
     if (cg == 2)                                                                                                     \
-      return p.box <= 96 ? launch_one<InstT, F, 2, 96>(maps, p, pdl, stream)                                         \
-                         : launch_one<InstT, F, 2, 128>(maps, p, pdl, stream);                                       \
+      return p.box <= 64   ? launch_one<InstT, F, 2, 64>(maps, p, pdl, stream)                                       \
+             : p.box <= 80 ? launch_one<InstT, F, 2, 80>(maps, p, pdl, stream)                                       \
+             : p.box <= 96 ? launch_one<InstT, F, 2, 96>(maps, p, pdl, stream)                                       \
+                           : launch_one<InstT, F, 2, 128>(maps, p, pdl, stream);                                     \
     return p.box <= 64 ? launch_one<InstT, F, 1, 64>(maps, p, pdl, stream)                                           \
                        : launch_one<InstT, F, 1, 128>(maps, p, pdl, stream);                                         \
   }
