@@ -79,7 +79,7 @@ int dispatch_stream(const StreamParams& p, bool has_zp, int gm, int mb, int ntw,
 bool tc_gemm_supported(int64_t size_n, int64_t size_k, int gm);
 int launch_tc_gemm(const void* a, int64_t lda, const uint32_t* b, const void* scales, const uint32_t* zeros,
                    const void* bias, const void* global_scale, void* c, int a_dtype, int fmt, int64_t size_m,
-                   int64_t size_n, int64_t size_k, int group_blocks, int channelwise, bool sums, void* scratch,
+                   int64_t size_n, int64_t size_k, int group_blocks, int channelwise, bool sums, bool gathered, void* scratch,
                    int64_t scratch_bytes, cudaStream_t stream);
 bool tc_group_sums_supported(int64_t group_size);
 // weight formats of the tensor-core kernel (gemm_tc.cuh)
@@ -431,7 +431,7 @@ static int gemm_impl(const void* a, int64_t lda, const uint32_t* b_q_weight, con
                                 : (has_zp ? kTcU8Z : kTcU8B128);
     int rc = launch_tc_gemm(a_used, lda_used, b_q_weight, b_scales, b_zeros, b_bias, global_scale, c, a_dtype, fmt,
                             size_m, size_n, size_k, group_blocks, gm == kChannel,
-                            gm == kGrouped && size_m <= 32 && !general_only, scratch,
+                            gm == kGrouped && size_m <= 32 && !general_only, has_act_order, scratch,
                             (int64_t)((scratch_bytes - a_tmp_bytes) / 256 * 256), stream);
     if (rc != B200Q_OK || !link) return rc;
     return launch_all_reduce(*link, c, c, size_m * size_n, a_dtype, stream);

@@ -471,10 +471,9 @@ struct Schedule {
     }
     return false;
   }
-  // tokens of the MMA for this segment
+  // tokens of the MMA for this segment (333 rows, tiles of 192: 192 and 160 instead of twice 192, 88.2 -> 86.1 us)
   template <int CG>
   __device__ __forceinline__ int mma_n(const Segment& s) const {
-    if (!p.tile_list) return p.tn;
     constexpr int g = 16 * CG;
     return (s.rows + g - 1) / g * g;
   }
