@@ -31,10 +31,9 @@
 // 64-column tiles.  A slice is owned by a thread-block cluster of 1, 2, 4 or 8
 // CTAs that split K evenly (enough CTAs to fill the GPU); inside a CTA the 8
 // warps split the CTA's k-range again.  Warp sums meet in shared memory; CTA
-// sums meet through distributed shared memory: every CTA publishes its tile,
-// and after a cluster barrier each CTA adds the ranks' copies of its share of
-// the rows in rank order and stores C.  No global scratch, no atomics, no
-// spinning, and the result is bitwise reproducible.
+// sums meet through distributed shared memory: each CTA adds all ranks' sums of
+// its share of the tile in rank order and stores C.  No global scratch, no
+// atomics, no spinning, and the result is bitwise reproducible.
 #pragma once
 
 #include <atomic>
@@ -174,10 +173,12 @@ struct StreamCfg {
   // reduction buffer: one 8-row block of every warp's accumulators, [row][column]
   static constexpr int kRedStride = 64 * NTW + 4;  // floats; +4 keeps the scalar stores conflict-free
   static constexpr int kRedBytes = kStreamWarps * 8 * kRedStride * 4;
-  // the CTA's finished tile, published to the cluster after the reduction
+  // cluster exchange (kShared: by columns, else by 8-row blocks; see the kernel): the CTA's share of the tile's columns as
+  // sent by every rank, not in the ring, which may still be in use when a faster CTA sends; else the CTA's finished tile
+  static constexpr bool kShared = MT == 1;
   static constexpr int kXBytes = MT * 8 * 64 * NTW * 4;
-  static constexpr int kSmemBytes =
-      kRingBytes > kRedBytes + kXBytes ? kRingBytes : kRedBytes + kXBytes;
+  static constexpr int kXOff = kShared && kRingBytes > kRedBytes ? kRingBytes : kRedBytes;
+  static constexpr int kSmemBytes = kXOff + kXBytes > kRingBytes ? kXOff + kXBytes : kRingBytes;
   static constexpr int kEpt = 2 * NTW;  // output elements per thread per 8-row block
 };
 
@@ -237,8 +238,11 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
   const uint32_t ring = smem_u32(smem) + warp * Cfg::kWarpBytes;
   const uint32_t slots = ring + D * Cfg::kStageBytes;
   float* red = reinterpret_cast<float*>(smem);
-  // this CTA's finished tile, read by the other CTAs of the cluster
-  float* xbuf = reinterpret_cast<float*>(smem + Cfg::kRedBytes);
+  // kShared: sums sent by the CTAs of the cluster, [rank][row][columns of this CTA's share]; else this CTA's finished
+  // tile, read by the others
+  float* xbuf = reinterpret_cast<float*>(smem + Cfg::kXOff);
+  // (a CTA may be written to once it is known to run: waited for before the first remote store)
+  if (Cfg::kShared && ksplit > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
 
   // ---- lane-constant addressing of the A rows inside a stage -------------------------
   // A is staged as rows of 32 B (16 k-values); 16 B chunk (row r, half h) lives at
@@ -593,6 +597,7 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
       __syncthreads();  // ring (or previous block's sums) no longer in use
       {
         float* mine = red + warp * (8 * Cfg::kRedStride);
+        if (!Cfg::kShared || 2 * q < p.m)  // rows that there are
 #pragma unroll
         for (int j = 0; j < NTW; ++j)
 #pragma unroll
@@ -605,6 +610,7 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
       __syncthreads();
 #pragma unroll
       for (int e = 0; e < Cfg::kEpt; ++e) outv[i][e] = 0.f;
+      if (!Cfg::kShared || o_row < p.m)
 #pragma unroll
       for (int w8 = 0; w8 < kStreamWarps; ++w8) {
         const float* src = red + w8 * (8 * Cfg::kRedStride) + o_row * Cfg::kRedStride + o_col;
@@ -619,11 +625,54 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
     }
 
     // ---- cross-CTA reduction inside the cluster, through distributed shared memory ----
-    // Every CTA publishes its tile in its own shared memory; after a cluster
-    // barrier the 8-row blocks of the tile are shared out among the CTAs (block % ksplit),
-    // and each sums the ranks' copies in rank order (bitwise reproducible).
+    // Up to eight rows (kShared): the tile's columns are shared out among the CTAs; every CTA sends each of the others the
+    // sums of that one's columns, and after one cluster barrier adds what it was sent in rank order (bitwise
+    // reproducible).  (Rank 0 fetching all of them and a second barrier that kept the others from leaving took 3300 of
+    // 9100 cycles of 4 x 4096 x 4096: 5.9 -> 5.3 us, 1 x 4096 x 6144 with its gather 7.4 -> 6.5, 1024 x 1024 3.3 -> 2.7.)
+    // More rows: every CTA publishes its tile in its own shared memory; after a cluster barrier the 8-row blocks are
+    // shared out (block % ksplit), and each CTA adds the ranks' copies in rank order.  (By columns 12 x 4096 x 6144 took
+    // 8.9 instead of 9.0 us, but 16 x 14336 x 4096 14.1 instead of 13.9 and 24 x 4096 x 6144 16.9 instead of 16.0.)
     bool do_store = true;
-    if (ksplit > 1) {
+    uint32_t owner = 0;  // kShared: rank that stores this thread's columns
+    if (Cfg::kShared && ksplit > 1) {
+      const uint32_t lanes = 32 / ksplit;  // of a warp, per share
+      owner = lane / lanes;
+      const uint32_t slot = smem_u32(xbuf) + (o_row * lanes + lane % lanes) * Cfg::kEpt * 4;
+      const uint32_t rank_bytes = 8 * lanes * Cfg::kEpt * 4;
+      uint32_t remote;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(slot + krank * rank_bytes), "r"(owner));
+      asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory");
+      if (o_row < p.m) {
+        if constexpr (Cfg::kEpt == 4)
+          asm volatile("st.shared::cluster.v4.f32 [%0], {%1,%2,%3,%4};\n" ::"r"(remote), "f"(outv[0][0]), "f"(outv[0][1]),
+                       "f"(outv[0][2]), "f"(outv[0][3])
+                       : "memory");
+        else
+          asm volatile("st.shared::cluster.v2.f32 [%0], {%1,%2};\n" ::"r"(remote), "f"(outv[0][0]), "f"(outv[0][1]) : "memory");
+      }
+      asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+      asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+      do_store = owner == krank;
+      if (do_store && o_row < p.m) {
+#pragma unroll
+        for (int e = 0; e < Cfg::kEpt; ++e) outv[0][e] = 0.f;
+        for (uint32_t r = 0; r < ksplit; ++r) {
+          if constexpr (Cfg::kEpt == 4) {
+            float4 v;
+            asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];\n"
+                         : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                         : "r"(slot + r * rank_bytes)
+                         : "memory");
+            outv[0][0] += v.x; outv[0][1] += v.y; outv[0][2] += v.z; outv[0][3] += v.w;
+          } else {
+            float2 v;
+            asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "r"(slot + r * rank_bytes) : "memory");
+            outv[0][0] += v.x; outv[0][1] += v.y;
+          }
+        }
+      }
+    }
+    if (!Cfg::kShared && ksplit > 1) {
 #pragma unroll
       for (int i = 0; i < MT; ++i) {
         float* dst = xbuf + (i * 8 + o_row) * (64 * NTW) + o_col;
@@ -664,11 +713,8 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
           }
         }
       }
-    }
-
-    // no CTA may exit while others still read its shared memory; after this barrier
-    // CTAs without output rows leave at once and make room for the next kernel
-    if (ksplit > 1) {
+      // no CTA may exit while others still read its shared memory; after this barrier
+      // CTAs without output rows leave at once and make room for the next kernel
       asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
       asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
     }
@@ -702,7 +748,7 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
       }
     }
     auto blk_mine = [&](int i) {
-      return do_store && i * 8 + o_row < p.m && (ksplit == 1 || (uint32_t)i % ksplit == krank);
+      return do_store && i * 8 + o_row < p.m && (Cfg::kShared || ksplit == 1 || (uint32_t)i % ksplit == krank);
     };
     if (p.ar.world == 0) {
 #pragma unroll
