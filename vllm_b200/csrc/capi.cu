@@ -142,6 +142,20 @@ bool decode_split(int64_t m, int64_t n, int64_t k, int bits, int gm, bool has_zp
   return true;
 }
 
+// Whether the decode kernel gathers the columns of A itself (act-order): up to eight rows, where its launcher says that the
+// part of A that a CTA needs is small enough.
+bool gather_inside(int64_t m, int64_t n, int64_t k, int bits, int a_dtype, const int32_t* perm) {
+  if (m > 8 || (reinterpret_cast<uintptr_t>(perm) & 15) != 0) return false;
+  const DecodeShape shape = decode_shape(m, n, kGrouped, false);
+  StreamParams p = {};
+  p.m = (int)m; p.n = (int)n; p.k = (int)k;
+  p.kt_total = (int)(k / 16);
+  p.slices = (int)(n / 64 / shape.ntw);
+  p.perm = perm;
+  StreamSplit split;
+  return launch_decode(p, false, kGrouped, shape.mb, shape.ntw, bits, a_dtype, 0, nullptr, &split) == B200Q_OK && split.fits;
+}
+
 // Integer weights up to 32 rows: decode kernel or tensor-core kernel, by estimated time.  The decode kernel
 // takes a time per k-tile of its busiest SM that grows with the rows (its instructions), and how its whole
 // column slices divide among the SMs decides the rest; the tensor-core kernel divides the weights evenly and
@@ -385,7 +399,9 @@ static int gemm_impl(const void* a, int64_t lda, const uint32_t* b_q_weight, con
   float* partials = static_cast<float*>(scratch);
   const void* a_used = a;
   int64_t lda_used = lda;
-  if (has_act_order) {
+  const bool inside = gm == kGrouped && has_act_order && !route.tc && !route.partials &&
+                      gather_inside(size_m, size_n, size_k, bits, a_dtype, perm);
+  if (has_act_order && !inside) {
     // gather the activation columns into sorted-row order once
     // (gptq_marlin.cu:549-564); the GEMM then reads a contiguous matrix
     void* a_tmp = static_cast<char*>(scratch) + (scratch_bytes - a_tmp_bytes) / 256 * 256;
@@ -452,6 +468,7 @@ static int gemm_impl(const void* a, int64_t lda, const uint32_t* b_q_weight, con
     p.scales = b_scales;
     p.zeros = b_zeros;
     p.g_idx = g_idx;
+    p.perm = inside ? perm : nullptr;
     p.bias = b_bias;
     p.c = static_cast<char*>(c) + (size_t)m0 * size_n * 2;
     p.partials = partials;

@@ -19,6 +19,7 @@ struct StreamParams {
   const void* scales;      // [G, N] 16-bit, permuted
   const uint32_t* zeros;   // [G, N/pf] or null
   const int32_t* g_idx;    // [K] or null
+  const int32_t* perm;     // [K]: the decode kernel takes column perm[k] of A for row k of the weights; or null
   const void* bias;        // [N] permuted or null
   void* c;                 // [M, N]
   float* partials;         // scratch for split slices
@@ -51,7 +52,7 @@ struct StreamParams {
 // How the decode kernel splits a problem, for whoever weighs it against another kernel.
 struct StreamSplit {
   int parts;   // CTAs per column slice
-  int per_sm;  // CTAs that fit on an SM
+  bool fits;   // with `perm`: the CTA's part of A fits beside the rings, and an item a thread covers it
 };
 
 constexpr int kStreamWarps = 8;

@@ -185,11 +185,15 @@ struct StreamCfg {
 // MOE: the mixture-of-experts form (see gemm_lookup.cuh): blockIdx.y is a block of p.m sorted
 // ids, the rows of A come through the ids (row = id / top_k), the block's expert selects the
 // weights, output rows are the ids themselves.
-template <typename T, int BITS, bool HAS_ZP, int GM, int MT, int NTW, int MINB, bool MOE = false>
+// GATHER: act-order, up to eight rows: every CTA gathers its k-range of A through p.perm into shared memory, an item of
+// eight k of a row a thread; the gather kernel in front costs a launch and a hand-over (captured, us: 1 x 4096 x 6144 7.8 ->
+// 7.2, 1 x 4096 x 4096 6.2 -> 5.6, 2 x 2048 x 9472 7.45 -> 5.9; called 9.1 -> 7.6).
+template <typename T, int BITS, bool HAS_ZP, int GM, int MT, int NTW, int MINB, bool MOE = false, bool GATHER = false>
 __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const StreamParams p) {
   using Cfg = StreamCfg<BITS, HAS_ZP, GM, MT, NTW>;
   using E = Emb<T, BITS>;
   static_assert(GM == kChannel || GM == kGrouped, "lookup mode runs gemm_lookup_kernel");
+  static_assert(!GATHER || (MT == 1 && !MOE), "");
   constexpr int D = Cfg::kDepth;
   constexpr bool kBiased = !HAS_ZP;
   constexpr int kWordsPerTile = BITS == 4 ? 4 : 8;  // words per lane per tile
@@ -350,7 +354,7 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
     };
     auto issue_a = [&]() {
 #pragma unroll
-      for (int i = 0; i < kABlocks; ++i)
+      for (int i = 0; i < (GATHER ? 0 : kABlocks); ++i)
         if constexpr (MOE)
           cp_async16(i_st + Cfg::kAOff + i * 512 + a_fill_off, a_bytes[i] ? i_a + a_delta[i] : i_a,
                      a_bytes[i]);
@@ -383,6 +387,14 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
       issue_w();
       issue_a();
     };
+
+    // GATHER: rows of A of a k-tile in shared memory (a power of two of them), where this lane's row of the warp's first
+    // k-tile is, and the distance to the next k-tile; lanes of rows that do not exist read 16 zero bytes
+    const int g_rows = p.m <= 1 ? 1 : p.m <= 2 ? 2 : p.m <= 4 ? 4 : 8;
+    const bool g_row = lr < p.m;
+    uint32_t g_a = smem_u32(smem) + Cfg::kSmemBytes + (g_row ? 32 + (wb - kt0) * (32 * g_rows) + a_ld_off : 0);
+    const uint32_t g_next = g_row ? 32 * g_rows : 0;
+    (void)g_a; (void)g_next;
 
     // ---- group end: fold the open group's sums into acc ---------------------------------
     auto close_group = [&](int g) {
@@ -452,7 +464,30 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
 #pragma unroll
       for (int s = 0; s < D - 1; ++s)
         if (s < pw) issue_w();
+      // GATHER: the indexes of the thread's item before the wait
+      int4 from[2];
+      const int chunks = 2 * len, row = threadIdx.x / chunks, chunk = threadIdx.x - row * chunks;
+      if constexpr (GATHER) {
+        if (row < p.m) {
+          const int4* src = reinterpret_cast<const int4*>(p.perm + (size_t)kt0 * 16) + 2 * chunk;
+          from[0] = __ldg(src);
+          from[1] = __ldg(src + 1);
+        }
+      }
       asm volatile("griddepcontrol.wait;\n" ::: "memory");
+      if constexpr (GATHER) {
+        if (threadIdx.x < 4) reinterpret_cast<uint32_t*>(smem + Cfg::kSmemBytes)[threadIdx.x] = 0;
+        if (row < p.m) {
+          const uint16_t* src = static_cast<const uint16_t*>(p.a) + (size_t)row * p.lda;
+          uint4 v;
+          v.x = (uint32_t)src[from[0].x] | ((uint32_t)src[from[0].y] << 16);
+          v.y = (uint32_t)src[from[0].z] | ((uint32_t)src[from[0].w] << 16);
+          v.z = (uint32_t)src[from[1].x] | ((uint32_t)src[from[1].y] << 16);
+          v.w = (uint32_t)src[from[1].z] | ((uint32_t)src[from[1].w] << 16);
+          const int pos = 2 * row + ((chunk & 1) ^ ((row >> 2) & 1));
+          *reinterpret_cast<uint4*>(smem + Cfg::kSmemBytes + 32 + (chunk >> 1) * (32 * g_rows) + pos * 16) = v;
+        }
+      }
 #pragma unroll
       for (int s = 0; s < D - 1; ++s)
         if (s < pw) issue_a();
@@ -470,6 +505,7 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
       }
     }
 
+    if constexpr (GATHER) __syncthreads();
     uint32_t c_st = ring;
     int c_g = (GM == kGrouped) ? wb / gb : 0;
     int c_left = (GM == kGrouped) ? gb - wb % gb : 0;
@@ -489,7 +525,12 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
       // activations: act[mt][0] = k 0..7, act[mt][1] = k 8..15 of 8 rows
       uint32_t act[MT][2];
       if constexpr (MT == 1) {
-        ldmatrix_x2(act[0][0], act[0][1], st + Cfg::kAOff + a_ld_off);
+        if constexpr (GATHER) {
+          ldmatrix_x2(act[0][0], act[0][1], g_a);
+          g_a += g_next;
+        } else {
+          ldmatrix_x2(act[0][0], act[0][1], st + Cfg::kAOff + a_ld_off);
+        }
       } else {
 #pragma unroll
         for (int i = 0; i < MT / 2; ++i) {
@@ -849,20 +890,22 @@ int max_clusters(K kernel, int smem, int size, std::atomic<int>& known) {
 }
 
 // Host launcher for one (type, bits, zp, group mode, MT, NTW) variant.  With `split` it only tells the split.
-template <typename T, int BITS, bool HAS_ZP, int GM, int MT, int NTW, bool MOE = false>
+template <typename T, int BITS, bool HAS_ZP, int GM, int MT, int NTW, bool MOE = false, bool GATHER = false>
 int launch_stream(StreamParams p, cudaStream_t stream, StreamSplit* split) {
   using Cfg = StreamCfg<BITS, HAS_ZP, GM, MT, NTW>;
   using E = Emb<T, BITS>;
   // accumulator registers: acc (+ grp when grouped)
   constexpr int kAccRegs = MT * NTW * 16 * (GM == kGrouped ? 2 : 1);
   constexpr int kMinBlocks = (kAccRegs <= 64 && MT <= 2 && Cfg::kSmemBytes <= 112 * 1024) ? 2 : 1;
-  auto kernel = gemm_stream_kernel<T, BITS, HAS_ZP, GM, MT, NTW, kMinBlocks, MOE>;
+  auto kernel = gemm_stream_kernel<T, BITS, HAS_ZP, GM, MT, NTW, kMinBlocks, MOE, GATHER>;
+  // with A's part: no more than leaves room for the second CTA of an SM
+  constexpr int kMostSmem = GATHER ? 112 * 1024 : Cfg::kSmemBytes;
+  static_assert(Cfg::kSmemBytes <= kMostSmem, "");
   static bool attr_done[64] = {};  // per device; benign race: the call is idempotent
   int dev = 0;
   B200Q_CUDA_OK(cudaGetDevice(&dev));
   if (!attr_done[dev & 63]) {
-    B200Q_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       Cfg::kSmemBytes));
+    B200Q_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem));
     attr_done[dev & 63] = true;
   }
   p.c_ex = E::kEx;
@@ -880,24 +923,30 @@ int launch_stream(StreamParams p, cudaStream_t stream, StreamSplit* split) {
   for (int s = 1; ksplit < 8 && s < 4; ++s) {
     const int more = 1 << s;
     if (p.slices * blocks * more > target || p.kt_total / more < 8) break;
-    if (p.slices * blocks > max_clusters(kernel, Cfg::kSmemBytes, more, fit[dev & 63][s])) break;
+    if (p.slices * blocks > max_clusters(kernel, kMostSmem, more, fit[dev & 63][s])) break;
     // two CTAs on an SM instead of one: only with enough k to pay for the wider exchange of sums (4-bit,
     // 1024 x 4096 at one row 6.1 us in eight parts, 4.3 in four; 4096 x 4096 6.0 against 7.2)
     const int least = more == 8 ? 24 : BITS == 4 ? 17 : 12;
     if (p.slices * blocks * more > device_sm_count() && p.kt_total / more < least) break;
     ksplit = more;
   }
+  int smem = Cfg::kSmemBytes;
+  if (GATHER) smem += 32 + (p.kt_total + ksplit - 1) / ksplit * 32 * (p.m <= 1 ? 1 : p.m <= 2 ? 2 : p.m <= 4 ? 4 : 8);
+  // (more than an item a thread delay every CTA: with two, 2 x 14336 x 4096 took 16.0 us instead of 13.7 with the gather
+  // in front, 4 x 4096 x 6144 9.7 instead of 8.6)
+  const bool fits = smem <= kMostSmem && 2 * ((p.kt_total + ksplit - 1) / ksplit) * p.m <= kStreamThreads;
   if (split) {
-    *split = {ksplit, kMinBlocks};
+    *split = {ksplit, fits};
     return B200Q_OK;
   }
+  B200Q_REQUIRE(!GATHER || fits, B200Q_EUNSUPPORTED, "too many rows for a gather inside the kernel");
   const int grid = p.slices * ksplit;
   // programmatic dependent launch: the kernel may start while its predecessor in
   // the stream drains; it orders itself with griddepcontrol.wait
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid, blocks);
   cfg.blockDim = dim3(kStreamThreads);
-  cfg.dynamicSmemBytes = Cfg::kSmemBytes;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;

@@ -43,6 +43,14 @@ int channel(const StreamParams& p, int rows8, int ntw, int max_ctas, cudaStream_
 
 template <bool HAS_ZP>
 int grouped(const StreamParams& p, int rows8, int ntw, int max_ctas, cudaStream_t stream, StreamSplit* split) {
+  if (p.perm) {  // act-order inside the kernel: up to eight rows, no zero-points
+    if constexpr (!HAS_ZP) {
+      if (rows8 == 1)
+        return ntw == 2 ? launch_stream<T, B, false, kGrouped, 1, 2, false, true>(p, stream, split)
+                        : launch_stream<T, B, false, kGrouped, 1, 1, false, true>(p, stream, split);
+    }
+    return B200Q_EUNSUPPORTED;
+  }
   switch (rows8 * 10 + ntw) {
     case 11: return launch_stream<T, B, HAS_ZP, kGrouped, 1, 1>(p, stream, split);
     case 12: return launch_stream<T, B, HAS_ZP, kGrouped, 1, 2>(p, stream, split);
