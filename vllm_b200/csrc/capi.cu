@@ -160,10 +160,10 @@ bool gather_inside(int64_t m, int64_t n, int64_t k, int bits, int a_dtype, const
 // takes a time per k-tile of its busiest SM that grows with the rows (its instructions), and how its whole
 // column slices divide among the SMs decides the rest; the tensor-core kernel divides the weights evenly and
 // its conversion does not depend on the rows.  Either way group scales are applied to fp32 sums.  The constants are
-// fits to B200 times over 18 shapes from 1024 x 1024 to 9472 x 18624; of 182 calls over 13 of them six take the
-// slower kernel by more than 6 %, two by more than 13.  (8-bit g128 fp16, 8 rows, us, decode / tensor cores:
-// 7168 x 9024, 141 slices on 148 SMs, 22.7 / 22.1; 3456 x 9024 12.4 / 14.1; 11008 x 5120, 160 half slices,
-// 27.8 / 20.1.)
+// fits to B200 times; of 252 calls (nine shapes from 1024 x 8192 to 4096 x 28672, 4 to 32 rows, six formats; both kernels
+// timed) thirteen take the one that is slower by more than 4 %, all of them 1024 or 2048 deep, where both take 5 to
+// 7 us.  (us, decode / tensor cores: 4-bit fp16 per column 14336 x 4096 at 32 rows 17.6 / 16.1, 4-bit groups of 64
+// 3584 x 18944 at 20 rows 26.5 / 22.4, 8-bit g128 fp16 at 8 rows 7168 x 9024 22.7 / 22.1, 3456 x 9024 12.4 / 14.1.)
 bool few_rows_on_tc(int64_t m, int64_t n, int64_t k, int bits, int gm, int group_blocks, bool has_zp, int a_dtype) {
   if (m > 32 || (bits == 4 && m <= 8)) return false;
   const bool grouped = gm == kGrouped;
@@ -172,7 +172,7 @@ bool few_rows_on_tc(int64_t m, int64_t n, int64_t k, int bits, int gm, int group
   DecodeSplit d;
   if (!decode_split(m, n, k, bits, gm, has_zp, a_dtype, &d)) return false;
   const bool alone = d.ctas <= device_sm_count();  // one CTA on an SM where two would fit
-  double base = 3.0, tile, factor;  // us: fixed and per tile of the decode kernel; conversion cost, 1 = 4-bit
+  double base = 3.0, tile, factor;  // us: fixed and per tile of the decode kernel; a round against the table of gemm_tc.cu
   if (bits == 8) {
     factor = bf16 ? (grouped ? 1.33 : 1.15) : (grouped ? 1.24 : 1.03);
     if (m <= 8) tile = alone ? 0.048 : bf16 && d.one_tile ? 0.045 : 0.041;
@@ -185,7 +185,8 @@ bool few_rows_on_tc(int64_t m, int64_t n, int64_t k, int bits, int gm, int group
     else tile = (grouped ? 0.046 : 0.0295) * (has_zp ? 1.2 : 1.0);
     if (m > 16) base = grouped ? 2.6 + 0.4 * (double)d.parts : 5.0;
   }
-  if (grouped && group_blocks < 8) factor = 1.8;  // two buffers of group sums a round
+  if (grouped && group_blocks < 8) factor = 1.65;  // two buffers of group sums a round
+  if (m > 16) factor *= 0.85;  // (nearer to what a round takes; below, the decode kernel's part of the estimate is as high)
   // clusters of eight that nearly fill the GPU start in turns
   if (d.parts == 8 && 2 * d.ctas > 3 * device_sm_count()) base += 2.0;
   return tc_gemm_estimate_us(m, n, k, factor) < 0.98 * (base + tile * (double)d.tiles);

@@ -173,11 +173,10 @@ struct TcPlan {
   double rounds_us;  // the part of it that is rounds
 };
 
-// Microseconds of a round (128 deep in k) of one tile, measured on B200 for 4-bit weights as the slope over K at
-// one tile per worker: 0.45 at 48 tokens, 0.58 at 128; pairs 0.57 at 160, 0.78 at 256.  Other formats are not in
-// here, and whole layers run longer: 8-bit fp16 pairs of 192 tokens 0.90 (table 0.64), NVFP4 pairs of 256 1.0
-// (0.78), 4-bit at 4096 tokens under the power cap 0.90 (0.78).  A factor common to all candidates leaves the choice
-// as it is except where sharing is weighed, see below.
+// Microseconds of a round (128 deep in k) of one tile: the table that plans are compared by, measured on B200 for 4-bit
+// weights while all operands went through shared memory.  Now (690 to 1020 cycles, gemm_tc.cuh) single CTAs take 0.37,
+// pairs 0.41 at 160 tokens, 0.44 at 192 and 0.54 at 256, more at the clocks of long runs: about a common factor, which
+// leaves the choice as it is except where sharing is weighed, see below.
 static double round_us(int cg, int tn) {
   if (cg == 1) return tn <= 64 ? 0.45 : 0.46 + 0.00096 * tn;
   const double t = 0.22 + 0.00217 * tn;
@@ -333,7 +332,7 @@ int64_t tc_gemm_scratch_bytes(int64_t size_m, int64_t size_n, int64_t size_k) {
 }
 
 // Estimated time of the kernel (and its reduce kernel) in us, fitted to whole calls of up to 32 rows; `factor`: time
-// of a round, 1 = 4-bit with scaled weights.
+// of a round against the table.
 double tc_gemm_estimate_us(int64_t size_m, int64_t size_n, int64_t size_k, double factor) {
   const tc::TcPlan pl = tc::plan_tiles(size_m, size_n, size_k, device_sm_count(), int64_t(1) << 40);
   const double us = factor * pl.rounds_us;
