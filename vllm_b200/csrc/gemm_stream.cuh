@@ -195,6 +195,7 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
   static_assert(GM == kChannel || GM == kGrouped, "lookup mode runs gemm_lookup_kernel");
   static_assert(!GATHER || (MT == 1 && !MOE), "");
   constexpr int D = Cfg::kDepth;
+  constexpr bool kShared = Cfg::kShared && !MOE;
   constexpr bool kBiased = !HAS_ZP;
   constexpr int kWordsPerTile = BITS == 4 ? 4 : 8;  // words per lane per tile
   extern __shared__ __align__(128) unsigned char smem[];
@@ -246,7 +247,7 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
   // tile, read by the others
   float* xbuf = reinterpret_cast<float*>(smem + Cfg::kXOff);
   // (a CTA may be written to once it is known to run: waited for before the first remote store)
-  if (Cfg::kShared && ksplit > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
+  if (kShared && ksplit > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
 
   // ---- lane-constant addressing of the A rows inside a stage -------------------------
   // A is staged as rows of 32 B (16 k-values); 16 B chunk (row r, half h) lives at
@@ -638,7 +639,7 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
       __syncthreads();  // ring (or previous block's sums) no longer in use
       {
         float* mine = red + warp * (8 * Cfg::kRedStride);
-        if (!Cfg::kShared || 2 * q < p.m)  // rows that there are
+        if (!kShared || 2 * q < p.m)  // rows that there are
 #pragma unroll
         for (int j = 0; j < NTW; ++j)
 #pragma unroll
@@ -651,7 +652,7 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
       __syncthreads();
 #pragma unroll
       for (int e = 0; e < Cfg::kEpt; ++e) outv[i][e] = 0.f;
-      if (!Cfg::kShared || o_row < p.m)
+      if (!kShared || o_row < p.m)
 #pragma unroll
       for (int w8 = 0; w8 < kStreamWarps; ++w8) {
         const float* src = red + w8 * (8 * Cfg::kRedStride) + o_row * Cfg::kRedStride + o_col;
@@ -666,7 +667,7 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
     }
 
     // ---- cross-CTA reduction inside the cluster, through distributed shared memory ----
-    // Up to eight rows (kShared): the tile's columns are shared out among the CTAs; every CTA sends each of the others the
+    // Up to eight rows, experts apart (kShared): the tile's columns are shared out among the CTAs; every CTA sends each of the others the
     // sums of that one's columns, and after one cluster barrier adds what it was sent in rank order (bitwise
     // reproducible).  (Rank 0 fetching all of them and a second barrier that kept the others from leaving took 3300 of
     // 9100 cycles of 4 x 4096 x 4096: 5.9 -> 5.3 us, 1 x 4096 x 6144 with its gather 7.4 -> 6.5, 1024 x 1024 3.3 -> 2.7.)
@@ -675,7 +676,7 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
     // 8.9 instead of 9.0 us, but 16 x 14336 x 4096 14.1 instead of 13.9 and 24 x 4096 x 6144 16.9 instead of 16.0.)
     bool do_store = true;
     uint32_t owner = 0;  // kShared: rank that stores this thread's columns
-    if (Cfg::kShared && ksplit > 1) {
+    if (kShared && ksplit > 1) {
       const uint32_t lanes = 32 / ksplit;  // of a warp, per share
       owner = lane / lanes;
       const uint32_t slot = smem_u32(xbuf) + (o_row * lanes + lane % lanes) * Cfg::kEpt * 4;
@@ -713,7 +714,7 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
         }
       }
     }
-    if (!Cfg::kShared && ksplit > 1) {
+    if (!kShared && ksplit > 1) {
 #pragma unroll
       for (int i = 0; i < MT; ++i) {
         float* dst = xbuf + (i * 8 + o_row) * (64 * NTW) + o_col;
@@ -789,7 +790,7 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
       }
     }
     auto blk_mine = [&](int i) {
-      return do_store && i * 8 + o_row < p.m && (Cfg::kShared || ksplit == 1 || (uint32_t)i % ksplit == krank);
+      return do_store && i * 8 + o_row < p.m && (kShared || ksplit == 1 || (uint32_t)i % ksplit == krank);
     };
     if (p.ar.world == 0) {
 #pragma unroll
