@@ -232,17 +232,18 @@ struct Plan {
 // the two matrices, 0 when both have a scale per column.  Lines and times (us, a layer of eight experts, top-2,
 // decode kernel / tensor cores; 4096 / 14336 unless stated):
 //   scales per column    4-bit from 7 rows, 8-bit always
-//   groups of 128, up    4-bit from 14 rows (12 rows 317 / 399, 14 rows 364 / 403, 16 rows 502 / 404), 8-bit from two
-//                        (one row 356 / 356, two 408 / 379, four 429 / 398; 2048 / 1408, two rows 44.6 / 45.2)
-//   groups of 64         two buffers of group sums a round: 4-bit from 28 rows (24 rows 536 / 572, 40 rows 975 / 587),
-//                        with zero-points or 8 bits from 14 (16 rows 647 / 610 and 596 / 562, 12 rows 399 / 555)
+//   groups of 128, up    4-bit from 14 rows (12 rows 323 / 362, 14 rows 370 / 362, 16 rows 530 / 362), 8-bit from two
+//                        (two rows 404 / 340, four 424 / 357; 2048 / 1408, two rows 43.3 / 44.3)
+//   groups of 64         two buffers of group sums a round: 4-bit above 14.4, where the decode kernel's blocks get wider (14
+//                        rows 384 / 449, 16 rows 569 / 447), with zero-points or 8 bits from 14 (8-bit 14 rows 581 / 448;
+//                        2048 / 1408 58.0 / 56.7, 12 rows 52.2 / 56.0)
 //   other groups         never: the group sums come in whole steps
 static bool on_tensor_cores(int64_t rows, int64_t experts, int64_t k, int64_t n, int bits, bool zp, int64_t group) {
   if (!tc_gemm_supported(2 * n, k, kChannel) || !tc_gemm_supported(k, n, kChannel)) return false;
   const double avg = (double)rows / (double)experts;
   if (group == 0) return bits == 8 || avg > 7.0;
   if (!tc_group_sums_supported(group)) return false;
-  if (group < 128) return avg >= (bits == 4 && !zp ? 28.0 : 14.0);
+  if (group < 128) return avg >= (bits == 4 && !zp ? 14.5 : 14.0);
   return avg >= (bits == 4 ? 14.0 : 2.0);
 }
 
