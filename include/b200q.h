@@ -6,6 +6,19 @@
  * and returns 0 on success or a negative B200Q_E* status.  After a non-zero
  * return b200q_last_error() gives a message for the calling thread.
  *
+ * Order on the stream.  Kernels are launched with programmatic dependent launch: a call
+ * may start while the kernel in front of it is still running, if that kernel lets it
+ * (griddepcontrol.launch_dependents / cudaTriggerProgrammaticLaunchCompletion; the
+ * kernels of this library do).  Activations, outputs, scratch and whatever else a call
+ * uses are touched only after all kernels in front have finished, with one exception: a
+ * layer's constants.  GEMMs of up to 128 rows fetch b_q_weight, b_scales, b_zeros, g_idx /
+ * perm, and the normalisation and permute_cols kernels their weight / perm, before
+ * that.  The constants may be written by anything that does not let the next kernel start early: copies,
+ * memsets, ordinary kernels, b200q_*_repack.  A kernel that does and writes constants has
+ * to be followed by an ordinary kernel, a copy, or an event or synchronisation waited for
+ * before such a call.  GEMMs of more than 128 rows and the mixture-of-experts entry points
+ * read everything in stream order.
+ *
  * Each declaration names the interface of the reference project that it
  * replaces (paths relative to the reference's root).
  */

@@ -37,3 +37,14 @@ def test_arrivals_at_the_other_cta_release_at_cluster_scope():
     assert "try_wait.parity.acquire.cluster" in code
     mma = code[code.index("warp == kMmaWarp) {"):code.index("warp < kDequantWarps) {")]
     assert "mbar_wait<kPair>(full(" in mma and "mbar_wait<kPair>(tmem_empty(" in mma
+
+
+def test_weights_of_prompts_are_fetched_behind_the_wait():
+    """What a kernel in front writes is visible after griddepcontrol.wait alone: above 128 rows, where calls make no
+    exception for a layer's constants, the producer waits before its first copy."""
+    code = _code()
+    producer = code[code.index("warp == kProducerWarp) {"):code.index("warp == kTokenWarp) {")]
+    wait = re.search(r'if \(!p\.weights_ahead\) asm volatile\("griddepcontrol\.wait;', producer)
+    assert wait and wait.start() < producer.index("tma_load")
+    with open(os.path.join(os.path.dirname(SRC), "gemm_tc.cu")) as f:
+        assert re.findall(r"weights_ahead = ([^;]*);", f.read()) == ["size_m <= 128"]

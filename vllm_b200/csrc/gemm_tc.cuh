@@ -94,6 +94,7 @@ struct TcParams {
   int tok_tiles;             // token tiles
   int workers;               // CTAs, or CTA pairs, of the grid
   int sk_tiles;              // the first tiles are shared out by k-range among all workers
+  int weights_ahead;         // packed weights, scales and zero-points may be fetched before the kernel in front is through
   float chan_factor;         // of the channel-wise scales (fp8: takes the exponent re-bias out)
   float* partials;           // [worker][2][CG][tn][128] fp32
   // mixture of experts: tiles come from a list in device memory {expert, first row, rows}; the rows of A
@@ -712,7 +713,8 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
     if constexpr (Cfg::kSplitRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(Cfg::kOtherRegs));
     if (warp == kProducerWarp) {
       // ================= producer =========================================================
-      // Packed weights do not depend on the kernel in front: they run ahead from the start.
+      // Weights run ahead of the kernel in front where callers know that (include/b200q.h), else they wait as all else does.
+      if (!p.weights_ahead) asm volatile("griddepcontrol.wait;\n" ::: "memory");
       Ring<WD> wr;
       bool ok = true;
       const int kt_all = p.k / 16;
