@@ -295,7 +295,9 @@ int b200q_fused_marlin_moe(
  * decode launch covers the problem (size_m <= 32) the GEMM kernel itself pushes its
  * rounded output tile to the peers and reduces: one kernel, no second launch;
  * otherwise the all-reduce kernel runs on C in place.  The result equals
- * b200q_marlin_gemm + b200q_all_reduce bit for bit.
+ * b200q_marlin_gemm + b200q_all_reduce bit for bit where that GEMM runs the same kernel
+ * (without the all-reduce, calls of up to 32 rows take the tensor-core kernel where it is
+ * the faster one, which adds the same products in another order).
  * size_m * size_n * 2 <= max_message_bytes; the other arguments as in the two calls.
  */
 int b200q_marlin_gemm_all_reduce(
