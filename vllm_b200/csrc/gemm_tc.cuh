@@ -13,9 +13,9 @@
 // Converted weights go to TMEM, where tcgen05.mma takes its 128-lane operand from as well: a thread converts one
 // column, which is a lane there, and shared memory carries neither the store nor the MMAs' reads of them.  Only tiles
 // of more than 192 tokens, whose accumulators fill TMEM, keep them in shared memory.  A round (below), cycles, with the
-// operand in shared memory / in TMEM: single CTAs 4-bit 48 tokens 822 / 690, 128 tokens 821 / 690, 8-bit 48 tokens 835 /
-// 610 (then HBM), fp8 24 tokens 882 / 670; pairs 4-bit 160 tokens 860 / 776, 192 tokens 865 / 830, 8-bit 160 tokens 1046 /
-// 700, 192 tokens 1035 / 793.  What bounds it now: instruction issue (60 to 66 % with one or two warps of a kind on a
+// operand in shared memory / in TMEM: single CTAs 4-bit 48 tokens 822 / 687, 128 tokens 821 / 681, 8-bit 48 tokens 835 /
+// 612 (then HBM), fp8 24 tokens 882 / 662; pairs 4-bit 160 tokens 860 / 779, 192 tokens 865 / 827, 8-bit 160 tokens 1046 /
+// 679, 192 tokens 1035 / 798.  What bounds it now: instruction issue (60 to 66 % with one or two warps of a kind on a
 // scheduler), of which eight instructions a packed word are the conversion; pairs in long runs the power limit.
 //
 // Roles, hand-offs through mbarriers; a step is 64 deep in k, two steps make a round:
@@ -546,69 +546,21 @@ __device__ __forceinline__ void convert_word(uint32_t w, uint32_t h8, const Offs
     hi = Pair<T>::sub(__byte_perm(w, 0x64646464u, 0x4341), o.hi);
   } else {
     // The low seven bits fit bf16's mantissa: (128 + low) - (128 or 256, by the eighth bit) = code - 128.
+    static_assert(F != kU8ZF, "float zero-points are fp16's alone");
     const uint32_t m = reg_const<0x007f007fu>(), e = reg_const<0x43004300u>(), t = 0x00800080u, f = 0x43804380u;
     const uint32_t w8 = w >> 8;
     lo = Pair<T>::sub(mask_or(w, m, e), (w & t) ^ f);
     hi = Pair<T>::sub(mask_or(w8, m, e), (w8 & t) ^ f);
-    if constexpr (F == kU8Z || F == kU8ZF) {
+    if constexpr (F == kU8Z) {
       lo = Pair<T>::sub(lo, o.lo);
       hi = Pair<T>::sub(hi, o.hi);
     }
   }
 }
 
-// fp4: a scale byte as a 16-bit pair
+// fp4: a scale byte, given in both halves of a word, as a 16-bit pair
 template <typename T, int F>
-__device__ __forceinline__ uint32_t fp4_scale(uint32_t byte) {
-  const uint32_t b = byte | (byte << 16);
-  if constexpr (F == kMX4 || std::is_same<T, half>::value) {
-    return b << 7;  // e8m0 -> bf16 exponent; S0E5M3 -> fp16 bits 14..7
-  } else {
-    const uint32_t t = b << 4;  // -> bf16: top exponent bit, then the seven lower bits
-    return (t & 0x07f007f0u) | ((t & 0x08000800u) << 3);
-  }
-}
-
-// The same by MMA fragments, for weights that go to shared memory: a thread takes the words of a lane of the packed
-// layout, a warp stores a 16 x 16 sub-tile with one stmatrix (half the reads and a quarter of the stores of the form by
-// columns, which made 256 tokens 1200 cycles a round instead of 1035).  Four 16-bit pairs of sub-tile `sub`: f[0], f[1] = column c8, k lo / hi; f[2], f[3] = column c8 + 8.
-template <typename T, int F>
-__device__ __forceinline__ void codes_to_16bit(const uint32_t* w, int sub, uint32_t (&f)[4]) {
-  using I = FmtInfo<F>;
-  constexpr bool kBiased = F == kU4B8 || F == kU8B128;
-  if constexpr (I::kFp4) {
-    // sign, two exponent bits, one mantissa bit into the fields of the 16-bit format; nibble i of the
-    // word sits where the uint4 codes do
-    constexpr int kShift = std::is_same<T, half>::value ? 3 : 6;
-    const uint32_t q = w[sub];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t x = q << (4 * (3 - i));
-      f[i] = (x & 0x80008000u) | ((x & 0x70007000u) >> kShift);
-    }
-    if constexpr (F == kMX4) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) f[i] = Pair<T>::mul(f[i], 0x7e807e80u);  // exact re-bias, 2^126
-    }
-  } else if constexpr (I::kBits == 4) {
-    dequant4<T, kBiased>(w[sub], f);
-  } else {
-    uint32_t t0[2], t1[2];
-    if constexpr (F == kF8) {
-      dequant_fp8<T>(w[2 * sub], t0);
-      dequant_fp8<T>(w[2 * sub + 1], t1);
-    } else {
-      dequant8<T, kBiased>(w[2 * sub], t0);
-      dequant8<T, kBiased>(w[2 * sub + 1], t1);
-    }
-    f[0] = t0[0]; f[1] = t0[1]; f[2] = t1[0]; f[3] = t1[1];
-  }
-}
-
-// fp4: one of a lane's scale bytes as a 16-bit pair
-template <typename T, int F>
-__device__ __forceinline__ uint32_t fp4_scale_of(uint32_t word, int byte) {
-  const uint32_t b = __byte_perm(word, 0, 0x4040 | byte | (byte << 8));  // the byte in both halves
+__device__ __forceinline__ uint32_t fp4_scale(uint32_t b) {
   if constexpr (F == kMX4 || std::is_same<T, half>::value) {
     return b << 7;  // e8m0 -> bf16 exponent; S0E5M3 -> fp16 bits 14..7
   } else {
@@ -619,13 +571,13 @@ __device__ __forceinline__ uint32_t fp4_scale_of(uint32_t word, int byte) {
 
 // SUMS: group scales are applied to fp32 sums, as in the decode kernel, so that calls which either kernel may take
 // give results of one precision.  The MMAs take the exact codes, a group of k at a time into one of a ring of TMEM
-// buffers; the epilogue warps add scale x buffer to the tile's running sums (in registers, for pairs in TMEM) while
-// the next group is computed.  Groups of one step or of whole rounds only.  fp16 results that are not the correctly
-// rounded ones: 0.03 to 0.13 % over 2048 .. 8192 deep layers of every integer type (decode kernel 0.8 to 6 %, scaled
-// weights rounded to 16 bits 39 %).
+// buffers; the epilogue warps add scale x buffer to the tile's running sums in registers while the next group is
+// computed.  Groups of one step or of whole rounds only.  fp16 results that are not the correctly rounded ones: 0.03 to
+// 0.13 % over 2048 .. 8192 deep layers of every integer type (decode kernel 0.8 to 6 %, scaled weights rounded to 16 bits
+// 39 %).
 // What bounds it: the hand-overs, and instruction issue (58 to 64 %) with the conversion beside it.  Cycles a round, with
-// the running sums of pairs in TMEM and the operand in shared memory / now: single CTAs 4-bit 32 rows 1090 / 885, 8-bit 16
-// rows 1059 / 935; pairs at 125 rows (eight experts, 4096 / 14336, 500 tokens) 1320 / 1190.  Two terms per weight, the
+// the operand in shared memory and the running sums of pairs in TMEM / now: single CTAs 4-bit 32 rows 1090 / 905, 8-bit 16
+// rows 1059 / 948; pairs at 125 rows (eight experts, 4096 / 14336, 500 tokens) 1320 / 1190.  Two terms per weight, the
 // rounded product and the rest, are as exact but take the MMAs twice; with four epilogue warps, or a wait for every
 // buffer, a round took 0.78 us.
 template <typename T, int F, int CG, int TOK, bool SUMS>
@@ -958,7 +910,7 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
             if constexpr (I::kZp) z = (zr[i] >> z_shift) & (BITS == 4 ? 15u : 255u);
             const Offset<T, F> off = make_offset<T, F>(z);
             if constexpr (kScaled) {
-              if constexpr (I::kFp4) s = fp4_scale<T, F>(sc[i]);
+              if constexpr (I::kFp4) s = fp4_scale<T, F>(sc[i] | (sc[i] << 16));
               else s = dup_lo(sc[i]);
               // q * s - zp * s with the product zp * s rounded, one fma per pair (as gemm_lookup.cuh)
               if constexpr (I::kZpF) zs = Pair<T>::mul(dup_lo(zr[i]), s) ^ 0x80008000u;
@@ -1031,8 +983,10 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
           tmem_st_wait();
           tc_fence_before();
         } else {
+          // By fragments: a thread takes the words of a lane of the packed layout, k-tile `kt` of both steps, column tile
+          // `fnt`, and a warp stores a 16 x 16 sub-tile with one stmatrix: half the reads and a quarter of the stores of the
+          // form by columns, which made 256 tokens 1200 cycles a round instead of 1035.
           constexpr int NW = BITS == 4 ? 4 : 8;
-          // by fragments: k-tile `kt` of both steps, column tile `fnt`
           const int fc8 = lane >> 2, kt = warp & 3, fnt = (warp >> 2) & 1;
           const bool flive = (sg.n_tile * CG + (int)rank) * 2 + fnt < NT;
           // The fragments of a 16 x 16 sub-tile are four 8 x 8 matrices (k lo and hi of columns 0-7, of columns 8-15):
@@ -1089,32 +1043,21 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
               const uint32_t (&zr)[4] = zr2[st];
               auto convert = [&](auto sub_c, auto scaled_c) {
                 constexpr int sub = decltype(sub_c)::value;
-                uint32_t f[4];
-                codes_to_16bit<T, F>(w, sub, f);
-                if constexpr (I::kZp) {
-                  // zero-points of columns c8 + 16 sub (low half) and + 8 (high half), exact integers in T
-                  uint32_t zpair;
-                  if constexpr (BITS == 4) {
-                    uint32_t z4[4];
-                    dequant4<T, false>(zr[0] >> (4 * sub), z4);  // nibbles sub and sub + 4
-                    zpair = z4[0];
-                  } else {
-                    uint32_t z8[2];
-                    dequant8<T, false>((sub & 2) ? zr[1] : zr[0], z8);  // word sub / 2, bytes (0, 2) or (1, 3)
-                    zpair = (sub & 1) ? z8[1] : z8[0];
-                  }
-                  const uint32_t z_lo = dup_lo(zpair), z_hi = dup_hi(zpair);
-                  f[0] = Pair<T>::sub(f[0], z_lo);
-                  f[1] = Pair<T>::sub(f[1], z_lo);
-                  f[2] = Pair<T>::sub(f[2], z_hi);
-                  f[3] = Pair<T>::sub(f[3], z_hi);
+                // columns c8 + 16 sub (f[0], f[1]: k lo and hi) and + 8 (f[2], f[3])
+                uint32_t f[4], z[2] = {0, 0};
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                  if constexpr (I::kZp) z[h] = BITS == 4 ? (zr[0] >> (4 * (sub + 4 * h))) & 15u
+                                                         : (zr[sub >> 1] >> (8 * (2 * h + (sub & 1)))) & 255u;
+                  convert_word<T, F>(BITS == 4 ? w[sub] : w[2 * sub + h], BITS == 4 ? 8 * h : 0, make_offset<T, F>(z[h]),
+                                     f[2 * h], f[2 * h + 1]);
                 }
                 if constexpr (decltype(scaled_c)::value) {
                   uint32_t s_lo, s_hi;
                   if constexpr (I::kFp4) {
                     // byte 4 (sub / 2) + 2 h + sub % 2 of the lane's eight belongs to column c8 + 16 sub + 8 h
-                    s_lo = fp4_scale_of<T, F>(sc[sub >> 1], sub & 1);
-                    s_hi = fp4_scale_of<T, F>(sc[sub >> 1], 2 + (sub & 1));
+                    s_lo = fp4_scale<T, F>(__byte_perm(sc[sub >> 1], 0, sub & 1 ? 0x4141 : 0x4040));
+                    s_hi = fp4_scale<T, F>(__byte_perm(sc[sub >> 1], 0, sub & 1 ? 0x4343 : 0x4242));
                   } else {
                     s_lo = dup_lo(sc[sub]);
                     s_hi = dup_hi(sc[sub]);
