@@ -86,6 +86,7 @@ bool tc_group_sums_supported(int64_t group_size);
 enum { kTcU4B8, kTcU4Z, kTcU8B128, kTcU8Z, kTcF8, kTcNV4, kTcMX4, kTcU4ZF, kTcU8ZF };
 int64_t tc_gemm_scratch_bytes(int64_t size_m, int64_t size_n, int64_t size_k);
 double tc_gemm_estimate_us(int64_t size_m, int64_t size_n, int64_t size_k, double factor);
+TcSplit tc_gemm_split(int64_t size_m, int64_t size_n, int64_t size_k);
 int tc_error_flag(bool reset);
 int ar_error_flag(bool reset);
 
@@ -156,14 +157,44 @@ bool gather_inside(int64_t m, int64_t n, int64_t k, int bits, int a_dtype, const
   return launch_decode(p, false, kGrouped, shape.mb, shape.ntw, bits, a_dtype, 0, nullptr, &split) == B200Q_OK && split.fits;
 }
 
+// 17 to 32 rows, integer weights: whether the tensor-core kernel's estimated time is below the decode kernel's, us.  The
+// tensor-core kernel: its rounds, a reduce kernel where k is shared out, and a start that the kernel in front hides only as
+// far as SMs are free.  The decode kernel: the tiles of its busiest SM, the exchange between the CTAs of a slice, further
+// waves.  Fits to B200 times of 1287 captured calls (33 shapes from 1024 x 1024 to 12288 x 28672 and 4096 x 28672, 17 to 32
+// rows, thirteen formats, both kernels timed): 27 take the kernel that is slower by more than 3 %, at most 7.5 %; of 630
+// calls of other shapes ten, at most 7 %.  (us, decode / tensor cores: 4-bit g128 fp16 with zero-points at 17 rows 2048 x 6144 8.8 / 10.4, 14336 x 4096 25.8 / 20.8; 4-bit
+// per column at 32 rows 1024 x 4096 5.9 / 4.7, 2048 x 2048 6.6 / 6.0, 4096 x 2048 8.2 / 8.6.)
+bool rows_17_to_32_on_tc(int64_t m, int64_t n, int64_t k, int bits, bool grouped, int group_blocks, bool has_zp, bool bf16,
+                         const DecodeSplit& d) {
+  const int64_t sms = device_sm_count();
+  const double more = (double)(m - 24) / 8;
+  const TcSplit t = tc_gemm_split(m, n, k);
+  double round = bits == 8 ? (grouped ? (bf16 ? 0.58 : 0.53) : (bf16 ? 0.40 : 0.36)) : grouped ? 0.505 : 0.345;
+  if (has_zp) round *= 1.09;
+  if (grouped && group_blocks < 8) round *= 1.27;  // two buffers of group sums a round
+  const double busy = (double)t.workers / (double)sms;
+  const double tc = 1.8 + (t.shared ? 2.6 : 0.0) + 2.6 * (busy > 0.8 ? (busy - 0.8) / 0.2 : 0.0) + t.rounds * round;
+  const double waves = (double)((d.ctas - 1) / sms);  // beyond the first
+  double base, tile;
+  if (grouped) {
+    base = (bits == 8 ? 1.8 : 2.0) + (d.parts > 1 ? 1.2 : 0.0) + 1.1 * (d.ctas < sms ? (double)d.ctas / (double)sms : 1.0) + 2.2 * waves;
+    tile = bits == 8 ? 0.054 + 0.004 * more : (0.0425 + 0.0014 * more) * (has_zp ? 1.17 : 1.0) * (group_blocks < 8 ? 1.1 : 1.0);
+  } else {
+    base = (d.one_tile ? 3.1 : 3.9) + (d.parts > 1 ? 1.1 : 0.0) + 1.9 * waves;
+    tile = bits == 4 ? (0.0267 + 0.001 * more + (d.one_tile ? 0.0065 : 0.0)) * (has_zp ? 1.12 : 1.0)
+           : bf16 && d.one_tile ? 0.09 : 0.0445 + 0.0027 * more + (d.one_tile ? 0.0095 : 0.0);
+  }
+  return tc < base + tile * (double)d.tiles;
+}
+
 // Integer weights up to 32 rows: decode kernel or tensor-core kernel, by estimated time.  The decode kernel
 // takes a time per k-tile of its busiest SM that grows with the rows (its instructions), and how its whole
 // column slices divide among the SMs decides the rest; the tensor-core kernel divides the weights evenly and
-// its conversion does not depend on the rows.  Either way group scales are applied to fp32 sums.  The constants are
-// fits to B200 times; of 252 calls (nine shapes from 1024 x 8192 to 4096 x 28672, 4 to 32 rows, six formats; both kernels
-// timed) thirteen take the one that is slower by more than 4 %, all of them 1024 or 2048 deep, where both take 5 to
-// 7 us.  (us, decode / tensor cores: 4-bit fp16 per column 14336 x 4096 at 32 rows 17.6 / 16.1, 4-bit groups of 64
-// 3584 x 18944 at 20 rows 26.5 / 22.4, 8-bit g128 fp16 at 8 rows 7168 x 9024 22.7 / 22.1, 3456 x 9024 12.4 / 14.1.)
+// its conversion does not depend on the rows.  Either way group scales are applied to fp32 sums.  Up to 16 rows the
+// constants are older fits to B200 times, of rounds that took longer and a decode kernel whose launches did, too.  The
+// kernels as they are, 1530 captured calls (the shapes and formats of above, 4-bit 9 to 16 rows, 8-bit 2 to 16): ten take the
+// tensor cores where these are slower by more than 3 %, 108 the decode kernel (most 1024 or 2048 deep with a scale per
+// column, up to 49 %).  (us, decode / tensor cores: 8-bit g128 fp16 at 8 rows 7168 x 9024 22.7 / 22.1.)
 bool few_rows_on_tc(int64_t m, int64_t n, int64_t k, int bits, int gm, int group_blocks, bool has_zp, int a_dtype) {
   if (m > 32 || (bits == 4 && m <= 8)) return false;
   const bool grouped = gm == kGrouped;
@@ -171,22 +202,18 @@ bool few_rows_on_tc(int64_t m, int64_t n, int64_t k, int bits, int gm, int group
   const bool bf16 = a_dtype == B200Q_BF16;
   DecodeSplit d;
   if (!decode_split(m, n, k, bits, gm, has_zp, a_dtype, &d)) return false;
+  if (m > 16) return rows_17_to_32_on_tc(m, n, k, bits, grouped, group_blocks, has_zp, bf16, d);
   const bool alone = d.ctas <= device_sm_count();  // one CTA on an SM where two would fit
   double base = 3.0, tile, factor;  // us: fixed and per tile of the decode kernel; a round against the table of gemm_tc.cu
   if (bits == 8) {
     factor = bf16 ? (grouped ? 1.33 : 1.15) : (grouped ? 1.24 : 1.03);
     if (m <= 8) tile = alone ? 0.048 : bf16 && d.one_tile ? 0.045 : 0.041;
-    else if (m <= 16) tile = alone && !grouped ? 0.070 : d.one_tile ? 0.052 : 0.045;
-    else tile = grouped ? 0.056 : bf16 && d.one_tile ? 0.090 : 0.047;
-    if (m > 16) base = grouped ? 2.6 + 0.4 * (double)d.parts : 5.0;
+    else tile = alone && !grouped ? 0.070 : d.one_tile ? 0.052 : 0.045;
   } else {
     factor = grouped ? (has_zp ? 1.3 : 1.28) : has_zp ? 1.17 : 1.0;
-    if (m <= 16) tile = (grouped ? 0.0245 : 0.020) * (has_zp ? 1.06 : 1.0);
-    else tile = (grouped ? 0.046 : 0.0295) * (has_zp ? 1.2 : 1.0);
-    if (m > 16) base = grouped ? 2.6 + 0.4 * (double)d.parts : 5.0;
+    tile = (grouped ? 0.0245 : 0.020) * (has_zp ? 1.06 : 1.0);
   }
   if (grouped && group_blocks < 8) factor = 1.65;  // two buffers of group sums a round
-  if (m > 16) factor *= 0.85;  // (nearer to what a round takes; below, the decode kernel's part of the estimate is as high)
   // clusters of eight that nearly fill the GPU start in turns
   if (d.parts == 8 && 2 * d.ctas > 3 * device_sm_count()) base += 2.0;
   return tc_gemm_estimate_us(m, n, k, factor) < 0.98 * (base + tile * (double)d.tiles);

@@ -54,6 +54,12 @@ struct StreamSplit {
   int parts;   // CTAs per column slice
   bool fits;   // with `perm`: the CTA's part of A fits beside the rings, and an item a thread covers it
 };
+// The same of the tensor-core kernel.
+struct TcSplit {
+  int rounds;   // rounds (128 deep in k) of the busiest worker
+  int workers;  // CTAs or CTA pairs
+  bool shared;  // tiles cut by k-range, whose sums a second kernel adds
+};
 
 constexpr int kStreamWarps = 8;
 constexpr int kStreamThreads = kStreamWarps * 32;

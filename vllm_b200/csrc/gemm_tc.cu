@@ -171,6 +171,7 @@ struct TcPlan {
   int64_t partial_bytes;
   double us;         // estimate that the plans are compared by
   double rounds_us;  // the part of it that is rounds
+  int rounds;        // of the busiest worker
 };
 
 // Microseconds of a round (128 deep in k) of one tile: the table that plans are compared by, measured on B200 for 4-bit
@@ -208,7 +209,8 @@ static TcPlan plan_tiles(int64_t m, int64_t n, int64_t k, int sms, int64_t scrat
       const double round = round_us(cg, pl.tn);
       const int64_t waves = tiles / most_workers, rem = tiles % most_workers;
       pl.workers = (int)(tiles < most_workers ? tiles : most_workers);
-      const double cost = (double)((waves + (rem > 0)) * rounds) * round;
+      pl.rounds = (int)((waves + (rem > 0)) * rounds);
+      const double cost = pl.rounds * round;
       pl.us = pl.rounds_us = cost;
       if (cost < best.us) best = pl;
       if (rem == 0) continue;
@@ -221,7 +223,8 @@ static TcPlan plan_tiles(int64_t m, int64_t n, int64_t k, int sms, int64_t scrat
       pl.sk_tiles = (int)rem;
       const int64_t slot_bytes = (int64_t)cg * pl.tn * kBN * 4;
       pl.partial_bytes = 2 * workers * slot_bytes;
-      pl.rounds_us = (double)(waves * rounds + (rem * rounds + workers - 1) / workers) * round;
+      pl.rounds = (int)(waves * rounds + (rem * rounds + workers - 1) / workers);
+      pl.rounds_us = pl.rounds * round;
       // (fixed costs for the choice between plans; tc_gemm_estimate_us has its own, fitted to whole calls.  The
       // two put sharing up to 1.5 us apart, and fp8 at 24 x 4096 x 28672 is shared by a margin of 0.4 us.)
       // a second segment behind whole tiles: its own pipeline fill and drain (1152 x 19392, 152 tiles of nine
@@ -335,7 +338,12 @@ int64_t tc_gemm_scratch_bytes(int64_t size_m, int64_t size_n, int64_t size_k) {
   return tc::plan_tiles(size_m, size_n, size_k, device_sm_count(), int64_t(1) << 40).partial_bytes;
 }
 
-// Estimated time of the kernel (and its reduce kernel) in us, fitted to whole calls of up to 32 rows; `factor`: time
+TcSplit tc_gemm_split(int64_t size_m, int64_t size_n, int64_t size_k) {
+  const tc::TcPlan pl = tc::plan_tiles(size_m, size_n, size_k, device_sm_count(), int64_t(1) << 40);
+  return {pl.rounds, pl.workers, pl.sk_tiles > 0};
+}
+
+// Estimated time of the kernel (and its reduce kernel) in us, fitted to whole calls of up to 16 rows; `factor`: time
 // of a round against the table.
 double tc_gemm_estimate_us(int64_t size_m, int64_t size_n, int64_t size_k, double factor) {
   const tc::TcPlan pl = tc::plan_tiles(size_m, size_n, size_k, device_sm_count(), int64_t(1) << 40);
