@@ -138,7 +138,5 @@ def test_weights_of_prompts_are_fetched_behind_the_wait():
     exception for a layer's constants, the producer waits before its first copy."""
     code = _code()
     producer = code[code.index("warp == kProducerWarp) {"):code.index("warp == kTokenWarp) {")]
-    wait = re.search(r'if \(!p\.weights_ahead\) asm volatile\("griddepcontrol\.wait;', producer)
-    assert wait and wait.start() < producer.index("tma_load")
-    with open(os.path.join(os.path.dirname(SRC), "gemm_tc.cu")) as f:
-        assert re.findall(r"weights_ahead = ([^;]*);", f.read()) == ["size_m <= 128"]
+    wait = re.search(r'if \(p\.m > kAheadRows\) asm volatile\("griddepcontrol\.wait;', producer)
+    assert wait and wait.start() < producer.index("tma_load") and "constexpr int kAheadRows = 128;" in code

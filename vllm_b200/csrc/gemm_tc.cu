@@ -289,13 +289,8 @@ int launch_tc_gemm(const void* a, int64_t lda, const uint32_t* b, const void* sc
   p.sk_tiles = plan.sk_tiles;
   p.chan_factor = fmt != tc::kF8 ? 1.f : a_dtype == B200Q_F16 ? Fp8Cvt<half>::kRebiasInv : Fp8Cvt<__nv_bfloat16>::kRebiasInv;
   p.partials = static_cast<float*>(scratch);
-  // Fetched before the kernels in front are through up to 128 rows only, as include/b200q.h says: what such a kernel
-  // writes is visible after the wait alone.  Captured, us, fetched ahead / behind the wait / no early launch: 200 x 2048 x
-  // 2048 8.4 / 10.3 / 11.8, 256 x 4096 x 4096 16.3 / 17.0 / 19.0, 1000 x 4096 x 6144 41.9 / 42.0 / 43.1.  (Asked for in
-  // L2 before the wait: 17.3, 340 x 4096 x 14336 38.5 instead of 37.9.)
-  p.weights_ahead = size_m <= 128;
   // early launch, but not of many rows behind their act-order gather: the waiting CTAs would take the SMs from it
-  const bool pdl = pdl_enabled() && (size_m <= 128 || !gathered);
+  const bool pdl = pdl_enabled() && (size_m <= tc::kAheadRows || !gathered);
   rc = a_dtype == B200Q_F16 ? tc::launch_type<half>(maps, p, fmt, plan.cg, sums, pdl, stream)
                             : tc::launch_type<__nv_bfloat16>(maps, p, fmt, plan.cg, sums, pdl, stream);
   if (rc != B200Q_OK || plan.sk_tiles == 0) return rc;

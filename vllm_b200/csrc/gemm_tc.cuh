@@ -77,6 +77,11 @@ constexpr int kBN = 128;           // weight columns per CTA
 // epilogue warps: TMEM lane quadrant = warp % 4; with group scales on the sums two share a quadrant
 constexpr int epi_warps(bool sums) { return sums ? 8 : 4; }
 constexpr uint32_t kSpinLimit = 1u << 24;
+// Rows up to which a call fetches packed weights, scales and zero-points before the kernels in front are through, as
+// include/b200q.h says: what such a kernel writes is visible after the wait alone.  Captured, us, fetched ahead / behind the
+// wait / no early launch: 200 x 2048 x 2048 8.4 / 10.3 / 11.8, 256 x 4096 x 4096 16.3 / 17.0 / 19.0, 1000 x 4096 x 6144
+// 41.9 / 42.0 / 43.1.  (Asked for in L2 before the wait: 17.3, 340 x 4096 x 14336 38.5 instead of 37.9.)
+constexpr int kAheadRows = 128;
 
 struct TcParams {
   int* error;                // device word: 0 = ok; else (role << 8) | barrier id of the first wait that timed out
@@ -94,7 +99,6 @@ struct TcParams {
   int tok_tiles;             // token tiles
   int workers;               // CTAs, or CTA pairs, of the grid
   int sk_tiles;              // the first tiles are shared out by k-range among all workers
-  int weights_ahead;         // packed weights, scales and zero-points may be fetched before the kernel in front is through
   float chan_factor;         // of the channel-wise scales (fp8: takes the exponent re-bias out)
   float* partials;           // [worker][2][CG][tn][128] fp32
   // mixture of experts: tiles come from a list in device memory {expert, first row, rows}; the rows of A
@@ -665,8 +669,9 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
     if constexpr (Cfg::kSplitRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(Cfg::kOtherRegs));
     if (warp == kProducerWarp) {
       // ================= producer =========================================================
-      // Weights run ahead of the kernel in front where callers know that (include/b200q.h), else they wait as all else does.
-      if (!p.weights_ahead) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+      // Packed weights run ahead of the kernel in front, up to kAheadRows rows.  (The line itself costs calls below that 0 to
+      // 0.1 us, wherever it stands and whether as a branch or a predicate: 48 x 14336 x 4096 17.6 -> 17.7.)
+      if (p.m > kAheadRows) asm volatile("griddepcontrol.wait;\n" ::: "memory");
       Ring<WD> wr;
       bool ok = true;
       const int kt_all = p.k / 16;
