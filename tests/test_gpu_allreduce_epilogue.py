@@ -25,6 +25,8 @@ WORLD = 2
     (4, 256, 19456, "uint4b8", 64, False, "bfloat16"),    # more slices than SMs
     (12, 2048, 1024, "uint4b8", 32, True, "bfloat16"),    # 8-row blocks shared out
     (32, 1024, 256, "uint4b8", 32, False, "float16"),
+    (16, 1024, 1024, "uint4b8", 128, False, "bfloat16"),  # the shard that the two-GPU test compares with GEMM + all-reduce
+    (32, 1024, 1024, "uint4b8", 128, False, "bfloat16"),
 ])
 def test_epilogue_sums_what_the_other_rank_sent(M, K, N, qtype, group, act, dtype, rank):
     import torch

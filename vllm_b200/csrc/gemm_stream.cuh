@@ -187,7 +187,7 @@ struct StreamCfg {
 // weights, output rows are the ids themselves.
 // GATHER: act-order, up to eight rows: every CTA gathers its k-range of A through p.perm into shared memory, an item of
 // eight k of a row a thread; the gather kernel in front costs a launch and a hand-over (captured, us: 1 x 4096 x 6144 7.8 ->
-// 7.2, 1 x 4096 x 4096 6.2 -> 5.6, 2 x 2048 x 9472 7.45 -> 5.9; called 9.1 -> 7.6).
+// 7.1, 1 x 4096 x 4096 6.2 -> 5.5, 2 x 2048 x 9472 7.5 -> 5.8; called one by one 1 x 4096 x 4096 9.6 -> 7.2).
 template <typename T, int BITS, bool HAS_ZP, int GM, int MT, int NTW, int MINB, bool MOE = false, bool GATHER = false>
 __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const StreamParams p) {
   using Cfg = StreamCfg<BITS, HAS_ZP, GM, MT, NTW>;
@@ -670,7 +670,8 @@ __global__ void __launch_bounds__(kStreamThreads, MINB) gemm_stream_kernel(const
     // Up to eight rows, experts apart (kShared): the tile's columns are shared out among the CTAs; every CTA sends each of the others the
     // sums of that one's columns, and after one cluster barrier adds what it was sent in rank order (bitwise
     // reproducible).  (Rank 0 fetching all of them and a second barrier that kept the others from leaving took 3300 of
-    // 9100 cycles of 4 x 4096 x 4096: 5.9 -> 5.3 us, 1 x 4096 x 6144 with its gather 7.4 -> 6.5, 1024 x 1024 3.3 -> 2.7.)
+    // 9100 cycles of 4 x 4096 x 4096: 5.8 -> 5.3 us, 1 x 4096 x 6144 7.4 -> 6.5, behind a gather kernel 8.4 -> 7.8, 1024 x
+    // 1024 3.3 -> 2.7.)
     // More rows: every CTA publishes its tile in its own shared memory; after a cluster barrier the 8-row blocks are
     // shared out (block % ksplit), and each CTA adds the ranks' copies in rank order.  (By columns 12 x 4096 x 6144 took
     // 8.9 instead of 9.0 us, but 16 x 14336 x 4096 14.1 instead of 13.9 and 24 x 4096 x 6144 16.9 instead of 16.0.)

@@ -175,9 +175,11 @@ struct TcPlan {
 };
 
 // Microseconds of a round (128 deep in k) of one tile: the table that plans are compared by, measured on B200 for 4-bit
-// weights while all operands went through shared memory.  Now (690 to 1020 cycles, gemm_tc.cuh) single CTAs take 0.37,
-// pairs 0.41 at 160 tokens, 0.44 at 192 and 0.54 at 256, more at the clocks of long runs: about a common factor, which
-// leaves the choice as it is except where sharing is weighed, see below.
+// weights while all operands went through shared memory.  It is too high for the kernel as it is, and not by one factor.
+// Table / now, 4-bit at 1965 MHz: single CTAs of 48 tokens 0.45 / 0.36, of 128 0.58 / 0.35, pairs of 160 0.57 / 0.40, of 192
+// 0.64 / 0.43, of 256 0.78 / 0.52; 8-bit per column 160 0.36, 8-bit groups of 128 256 0.73.  So whole waves look longer
+// against shared ones than they are (fp8 24 x 4096 x 28672: 28.8 against 28.4 by the table, 21.6 against 22.8 by the time of
+// a round now), wide single CTAs longer against pairs, and 8 bits are planned as if they were 4.
 static double round_us(int cg, int tn) {
   if (cg == 1) return tn <= 64 ? 0.45 : 0.46 + 0.00096 * tn;
   const double t = 0.22 + 0.00217 * tn;

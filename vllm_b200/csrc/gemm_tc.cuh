@@ -13,9 +13,9 @@
 // Converted weights go to TMEM, where tcgen05.mma takes its 128-lane operand from as well: a thread converts one
 // column, which is a lane there, and shared memory carries neither the store nor the MMAs' reads of them.  Only tiles
 // of more than 192 tokens, whose accumulators fill TMEM, keep them in shared memory.  A round (below), cycles, with the
-// operand in shared memory / in TMEM: single CTAs 4-bit 48 tokens 822 / 687, 128 tokens 821 / 681, 8-bit 48 tokens 835 /
-// 612 (then HBM), fp8 24 tokens 882 / 662; pairs 4-bit 160 tokens 860 / 779, 192 tokens 865 / 827, 8-bit 160 tokens 1046 /
-// 679, 192 tokens 1035 / 798.  What bounds it now: instruction issue (60 to 66 % with one or two warps of a kind on a
+// operand in shared memory / in TMEM: single CTAs 4-bit 48 tokens 822 / 709, 128 tokens 811 / 696, 8-bit 48 tokens 835 /
+// 620 (then HBM), fp8 24 tokens 870 / 662; pairs 4-bit 160 tokens 869 / 781, 192 tokens 872 / 839, 8-bit 160 tokens 1039 /
+// 699, 192 tokens 1032 / 795.  What bounds it now: instruction issue (60 to 66 % with one or two warps of a kind on a
 // scheduler), of which eight instructions a packed word are the conversion; pairs in long runs the power limit.
 //
 // Roles, hand-offs through mbarriers; a step is 64 deep in k, two steps make a round:
@@ -390,7 +390,11 @@ struct TcCfg {
   // With few places in TMEM (pairs) a dequant warp holds the whole round in registers before it asks for one: with
   // half of the conversion done on the place, it went round in 2500 cycles (160 tokens, three places).
   static constexpr bool kHoldRound = kInTmem && !SUMS && kARing < 4;
-  // registers a thread of the roles (SUMS: the epilogue holds up to 80 sums); what the launch has is an upper limit
+  // Registers a thread of the roles (SUMS: the epilogue holds up to 80 sums); what the launch has is an upper limit.  The
+  // forms with a split spill 52 to 224 bytes, outside the rounds: warp-level loads and stores of local memory are 22200 and
+  // 18500 a launch at 160 tokens, 7400 and 7104 at 192, 15984 and 12284 for SUMS in single CTAs, at K = 4096 as at 16384;
+  // 0.2 % of the instructions of a layer of eight experts at 500 tokens.  (56 registers instead of 40 for the other roles
+  // leave them as they are.)
   static constexpr bool kSplitRegs = SUMS || kHoldRound;
   static constexpr int kDequantRegs = kHoldRound ? 88 : CG == 1 ? 64 : 56, kOtherRegs = kHoldRound ? 48 : 40,
                        kEpiRegs = kHoldRound ? 80 : CG == 1 ? 96 : 120;
@@ -476,7 +480,8 @@ struct Schedule {
     }
     return false;
   }
-  // tokens of the MMA for this segment (333 rows, tiles of 192: 192 and 160 instead of twice 192, 88.2 -> 86.1 us)
+  // tokens of the MMA for this segment: a narrow last tile leaves MMAs out (by itself worth up to 1 %: captured, 340 x 14336 x
+  // 4096 39.2 -> 38.9 us, 8-bit 333 x 3584 x 37888 76.25 -> 76.2)
   template <int CG>
   __device__ __forceinline__ int mma_n(const Segment& s) const {
     constexpr int g = 16 * CG;
@@ -580,8 +585,8 @@ __device__ __forceinline__ uint32_t fp4_scale(uint32_t b) {
 // 0.13 % over 2048 .. 8192 deep layers of every integer type (decode kernel 0.8 to 6 %, scaled weights rounded to 16 bits
 // 39 %).
 // What bounds it: the hand-overs, and instruction issue (58 to 64 %) with the conversion beside it.  Cycles a round, with
-// the operand in shared memory and the running sums of pairs in TMEM / now: single CTAs 4-bit 32 rows 1090 / 905, 8-bit 16
-// rows 1059 / 948; pairs at 125 rows (eight experts, 4096 / 14336, 500 tokens) 1320 / 1190.  Two terms per weight, the
+// the operand in shared memory and the running sums of pairs in TMEM / now: single CTAs 4-bit 32 rows 1084 / 890, 8-bit 16
+// rows 1056 / 959; pairs at 125 rows (eight experts, 4096 / 14336, 500 tokens) 1320 / 1190.  Two terms per weight, the
 // rounded product and the rest, are as exact but take the MMAs twice; with four epilogue warps, or a wait for every
 // buffer, a round took 0.78 us.
 template <typename T, int F, int CG, int TOK, bool SUMS>

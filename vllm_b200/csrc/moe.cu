@@ -238,6 +238,11 @@ struct Plan {
 //                        rows 384 / 449, 16 rows 569 / 447), with zero-points or 8 bits from 14 (8-bit 14 rows 581 / 448;
 //                        2048 / 1408 58.0 / 56.7, 12 rows 52.2 / 56.0)
 //   other groups         never: the group sums come in whole steps
+// The lines hold on other layers: groups of 64, 4-bit, decode kernel / tensor cores at 14 and at 15 rows: 64 experts top-6 2048
+// / 1408 205 / 199 and 304 / 198, 128 top-8 2048 / 768 243 / 232 and 377 / 232, 16 top-4 4096 / 2048 135 / 156 and 185 / 156,
+// 32 top-4 2880 / 2880 242 / 258 and 365 / 258, 8 top-2 2048 / 1408 43 / 50 and 53 / 50.  Farthest off: 8-bit at 12 to 13
+// rows in groups of 64 (577 / 462), 8-bit groups of 128 at three rows of 8 top-2 2048 / 1408 (41 / 46), zero-points in groups of
+// 128 at 8 to 13 rows of 128 experts (254 / 213 at 13).
 static bool on_tensor_cores(int64_t rows, int64_t experts, int64_t k, int64_t n, int bits, bool zp, int64_t group) {
   if (!tc_gemm_supported(2 * n, k, kChannel) || !tc_gemm_supported(k, n, kChannel)) return false;
   const double avg = (double)rows / (double)experts;
