@@ -675,8 +675,10 @@ gemm_tc_kernel(const __grid_constant__ TcMaps maps, const TcParams p) {
     if (warp == kProducerWarp) {
       // ================= producer =========================================================
       // Packed weights run ahead of the kernel in front, up to kAheadRows rows.  (The line itself costs calls below that 0 to
-      // 0.1 us, wherever it stands and whether as a branch or a predicate: 48 x 14336 x 4096 17.6 -> 17.7.)
-      if (p.m > kAheadRows) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+      // 0.1 us, wherever it stands: 48 x 14336 x 4096 17.6 -> 17.7.  With the scales on the sums a call has few rows or has
+      // waited for its tile list: expert layers were 1 % slower with the line.)
+      if constexpr (!SUMS)
+        if (p.m > kAheadRows) asm volatile("griddepcontrol.wait;\n" ::: "memory");
       Ring<WD> wr;
       bool ok = true;
       const int kt_all = p.k / 16;
