@@ -160,10 +160,11 @@ bool gather_inside(int64_t m, int64_t n, int64_t k, int bits, int a_dtype, const
 // 17 to 32 rows, integer weights: whether the tensor-core kernel's estimated time is below the decode kernel's, us.  The
 // tensor-core kernel: its rounds, a reduce kernel where k is shared out, and a start that the kernel in front hides only as
 // far as SMs are free.  The decode kernel: the tiles of its busiest SM, the exchange between the CTAs of a slice, further
-// waves.  Fits to B200 times of 1287 captured calls (33 shapes from 1024 x 1024 to 12288 x 28672 and 4096 x 28672, 17 to 32
+// waves.  Fits to B200 times of 1287 captured calls (33 shapes from 1024 x 1024 to 12288 x 8896 and 4096 x 28672, 17 to 32
 // rows, thirteen formats, both kernels timed): 27 take the kernel that is slower by more than 3 %, at most 7.5 %; of 630
-// calls of other shapes ten, at most 7 %.  (us, decode / tensor cores: 4-bit g128 fp16 with zero-points at 17 rows 2048 x 6144 8.8 / 10.4, 14336 x 4096 25.8 / 20.8; 4-bit
-// per column at 32 rows 1024 x 4096 5.9 / 4.7, 2048 x 2048 6.6 / 6.0, 4096 x 2048 8.2 / 8.6.)
+// calls of other shapes ten, at most 7 %.  (us, decode / tensor cores: 4-bit g128 fp16 with zero-points at 17 rows 2048 x
+// 6144 8.8 / 10.4, 14336 x 4096 25.8 / 20.8; 4-bit per column fp16 at 32 rows 1024 x 4096 5.9 / 4.7, 2048 x 2048 6.6 / 6.0,
+// 4096 x 2048 8.2 / 8.6.)
 bool rows_17_to_32_on_tc(int64_t m, int64_t n, int64_t k, int bits, bool grouped, int group_blocks, bool has_zp, bool bf16,
                          const DecodeSplit& d) {
   const int64_t sms = device_sm_count();
